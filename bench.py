@@ -306,8 +306,9 @@ def run_gpu(args):
     peak, peak_kind = measured_peaks()
     bpu = bytes_per_site_rhs(prec, n, nrhs)
     achieved = bpu * units / (ms_local * 1e-3) / 1e9
-    tcs_rings = {4: (4, 3), 5: (6, 3), 6: (3, 2), 7: (8, 3), 8: (6, 4)}  # (TMA stages, B buffers) of variants 4-8
-    kernel = (("wilson_tcs_kernel<N=%d,stages=%d,bbufs=%d> (tcgen05, %s)"
+    tcs_rings = {4: (4, 3), 6: (5, 2), 7: (8, 2), 8: (6, 2)}  # (TMA stages, B buffers) of variants 4, 6-8
+    kernel = ("wilson_mma_kernel<%s,N=%d> (register-fragment mma.sync)" % (pname, n) if stages == -5 else
+              ("wilson_tcs_kernel<N=%d,stages=%d,bbufs=%d> (tcgen05, %s)"
                % ((n,) + tcs_rings[-stages] + ("site-major" if prec == 5 else "component-major",)))
               if stages <= -4 else
               ("wilson_tc_kernel<%s,N=%d> (tcgen05)" % (pname, n)) if stages < 0 else

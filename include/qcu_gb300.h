@@ -240,11 +240,12 @@ int qcuMeasureFmaRate(int precision, double *tflops);
  * (RHS per thread, register-cap variant, packed, stages, recon, linktma) are
  * available; the first max_shapes are written to shapes[6 * i .. 6 * i + 5].
  * stages > 0 is the TMA-staged kernel with that many ring buffers, stages < 0
- * a tensor-core (tcgen05) kernel, BF16 only: -1 projected half-spinor
- * operands with direct loads, -2 / -3 the same with a TMA ring of that depth,
- * -4 / -5 / -6 the neighbour spinor block as the MMA operand (warp-specialised,
+ * a tensor-core kernel: -1 projected half-spinor operands (tcgen05, BF16) with
+ * direct loads, -2 / -3 the same with a TMA ring of that depth, -4 / -6 the
+ * neighbour spinor block as the MMA operand (tcgen05, BF16; warp-specialised,
  * TMA and B rings of different depths; nrhs a multiple of 4), -7 / -8 the
- * same with deeper rings of half-size stages (tiles of at most 32 RHS);
+ * same with deeper rings of half-size stages (tiles of at most 32 RHS), -5 the
+ * link product on register-fragment MMAs (FP16 and BF16; nrhs a multiple of 4);
  * recon = 1 reads
  * SU(3) links as two rows and reconstructs the third (used only when the
  * loaded gauge is SU(3) to the precision's rounding); linktma = 1 is the

@@ -355,7 +355,8 @@ def blas_mrhs(op: int, n_elements: int, nrhs: int, x, x_precision: int, y=None, 
 def tune_dslash(nrhs: int, precision: int):
     """(R, block, reg_cap, packed, stages, recon, linktma) of the tuned
     kernel; stages > 0: the TMA-staged kernel, -v: tensor-core variant v (1-3
-    projected half-spinor operands, 4-6 the spinor block as the MMA operand);
+    projected half-spinor operands, 4 and 6-8 the spinor block as the MMA
+    operand, 5 register-fragment MMAs);
     recon: two-row SU(3) links; linktma: links staged by TMA per x-row."""
     R, B, M, K, T, C, X = (ctypes.c_int() for _ in range(7))
     _raise_if(lib().qcuTuneDslash(int(nrhs), int(precision), ctypes.byref(R), ctypes.byref(B), ctypes.byref(M),
@@ -374,7 +375,7 @@ def last_dslash_shape():
 def dslash_kernels(precision: int, n_colors: int = 3):
     """Compiled dslash kernel shapes [(R, reg_cap, packed, stages, recon,
     linktma), ...]; stages > 0: the TMA-staged kernel, -v: tensor-core variant
-    v (1-6); recon: two-row SU(3) links; linktma: links staged by TMA per
+    v (1-8); recon: two-row SU(3) links; linktma: links staged by TMA per
     x-row."""
     arr = (ctypes.c_int * (6 * 96))()
     cnt = ctypes.c_int()

@@ -101,6 +101,10 @@ bool tc_runs(const DslashArgs& A_in, int prec, int N, int variant) {
   if (!find_tc(prec, N, variant)) return false;
   DslashArgs A = A_in;
   A.site_major = prec_site_major(prec) ? 1 : 0;
+  if (variant == kMmaVariant) {
+    MmaDslashArgs T5;
+    return mma_plan(A, prec, N, 1, 1, &T5);
+  }
   if (variant >= 4) {
     TcsDslashArgs T4;
     CUtensorMap m;

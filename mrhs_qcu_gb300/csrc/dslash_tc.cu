@@ -82,6 +82,23 @@ bool tcs_plan(const DslashArgs& A, int N, TcsDslashArgs* T, CUtensorMap* map_in)
   return true;
 }
 
+bool mma_plan(const DslashArgs& A, int prec, int N, int S, int MT, MmaDslashArgs* T) {
+  const Geometry& geo = A.geo;
+  const int nrhs = A.nrhs;
+  if (!prec_is16(prec) || N < 3 || N > 8 || nrhs < 1 || nrhs % 4 || !A.gauge_rec) return false;
+  if (((uintptr_t)A.in | (uintptr_t)A.out | (uintptr_t)A.x | (uintptr_t)A.gauge_rec) % 16) return false;
+  if (prec_has_norm(prec) && ((uintptr_t)A.in_norm | (uintptr_t)A.x_norm) % 16) return false;
+  if ((int64_t)4 * N * geo.vh * nrhs >= (1ll << 32)) return false;  // 32-bit element offsets into the fields
+  const int64_t groups = ((int64_t)geo.vh + S - 1) / S, chunks = (nrhs + 16 * MT - 1) / (16 * MT);
+  if (groups * chunks >= (1ll << 31)) return false;
+  T->A = A;
+  T->div_chunks = FastDiv((uint32_t)chunks);
+  T->warps = (uint32_t)(groups * chunks);
+  T->cstr = (uint32_t)(A.site_major ? nrhs : geo.vh * nrhs);
+  T->sstr = (uint32_t)(A.site_major ? 4 * N * nrhs : nrhs);
+  return true;
+}
+
 // CTAs per SM from the kernel's registers and shared memory (the runtime's
 // occupancy query reports 1 for kernels that allocate tensor memory), capped
 // by the 512 tensor-memory columns.

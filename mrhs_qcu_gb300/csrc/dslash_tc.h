@@ -3,8 +3,11 @@
 #pragma once
 
 #include <cstring>
+#include <mutex>
+#include <type_traits>
 
 #include "dslash.h"
+#include "dslash_mma.cuh"
 #include "dslash_tc.cuh"
 #include "dslash_tcs.cuh"
 #include "dslash_tma.h"
@@ -26,17 +29,16 @@ int tc_grid(const void* kernel, int ntiles, size_t smem, int tmem_cols = 32, int
 // offsets, and a field map the driver accepts).
 bool tcs_plan(const DslashArgs& A, int N, TcsDslashArgs* T, CUtensorMap* map_in);
 
-// ring depths of the spinor-operand variants 4-8: (TMA stages, B buffers, A
+// ring depths of the spinor-operand variants 4, 6, 7, 8: (TMA stages, B buffers, A
 // halves of 32 RHS per stage).  Variants 7 and 8 hold one half per stage, so
 // their deeper rings fit the same shared memory; they take tiles of at most
 // 32 RHS (nrhs <= 32, or RHS counts that split into such tiles).
-constexpr int tcs_stages(int variant) { return variant == 5 ? 6 : variant == 6 ? 5 : variant == 7 ? 8 : variant == 8 ? 6 : 4; }
+constexpr int tcs_stages(int variant) { return variant == 6 ? 5 : variant == 7 ? 8 : variant == 8 ? 6 : 4; }
 constexpr int tcs_bbufs(int variant) { return (variant == 6 || variant == 7 || variant == 8) ? 2 : 3; }
 constexpr int tcs_halves(int variant) { return variant >= 7 ? 1 : 2; }
 
-// Variants 4 and 6-8 are sized so that 4 CTAs share an SM (228 KB of shared
-// memory, 1 KB reserved per CTA; tensor memory 4 x 128 columns); variant 5
-// trades the fourth CTA for six stages.
+// They are sized so that 4 CTAs share an SM (228 KB of shared memory, 1 KB
+// reserved per CTA; tensor memory 4 x 128 columns).
 constexpr bool tcs_fits_4_ctas(int v) {
   return 4 * (tcs::smem_bytes(tcs_stages(v), tcs_bbufs(v), tcs_halves(v)) + 1024) <= 228 * 1024;
 }
@@ -64,6 +66,55 @@ void launch_wilson_tcs(const DslashArgs& A, cudaStream_t st) {
   tma_note_launch();
 }
 
+// Plan of the register-fragment MMA kernel for S sites x 16 MT RHS per warp;
+// false when it cannot run these arguments (FP16 or BF16 storage, N = 3..8,
+// nrhs a multiple of 4, the link records present, 32-bit element offsets,
+// 16-byte aligned fields and scales).
+bool mma_plan(const DslashArgs& A, int prec, int N, int S, int MT, MmaDslashArgs* T);
+
+template <int P, int N, int S, int MT, int NST, bool L1>
+void launch_wilson_mma_shape(const DslashArgs& A, cudaStream_t st) {
+  MmaDslashArgs T;
+  QCU_REQUIRE(mma_plan(A, P, N, S, MT, &T), QCU_ERR_UNSUPPORTED,
+              "tensor-core dslash: arguments outside the kernel's limits");
+  plan_site_order(T.A, P, N);
+  const size_t smem = (size_t)mma::kWarps * 4 * mma::warp_words(P, N, S, MT, NST);
+  auto* const k = &wilson_mma_kernel<P, N, S, MT, NST, L1>;
+  static std::once_flag smem_set;  // the size is the instance's own
+  if (smem > 48 * 1024)
+    std::call_once(smem_set, [&] {
+      QCU_CHECK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    });
+  k<<<(T.warps + mma::kWarps - 1) / mma::kWarps, 32 * mma::kWarps, smem, st>>>(T);
+}
+
+// Sites and RHS per warp, and ring depth, by colours and RHS count (us a hop,
+// 16^3x32 unless stated; two sites / one site per 16 RHS, then one site x 32):
+//   N <= 4, nrhs <= 16   two sites x 16 RHS, 2 stages (SU(4) nrhs 16: 52 / 58)
+//           nrhs > 16    one site x 32 RHS, 3 stages (SU(4) nrhs 64: 203, 224 with two sites x 16)
+//   N <= 6, nrhs <= 16   two sites x 16 RHS, 3 stages (SU(6) nrhs 16: 106 / 114)
+//   N >= 7, nrhs <= 16   one site x 16 RHS, 2 stages (SU(8) nrhs 16: 143 / 118, registers)
+//   N > 4,  nrhs > 16    one site x 32 RHS, 2 stages (SU(8) nrhs 64: 418, 455 with 3 stages, 489 x 16)
+// Copies through L1 where the RHS rows are not whole sectors (nrhs % 8): SU(3)
+// 24^3x48 nrhs 12 264 against 329 us past it, SU(4) nrhs 16 63 against 52.
+template <int P, int N>
+void launch_wilson_mma(const DslashArgs& A, cudaStream_t st) {
+  constexpr bool few = N <= 4;
+  auto go = [&](auto l1) {
+    constexpr bool L1 = decltype(l1)::value;
+    if (A.nrhs > 16)
+      launch_wilson_mma_shape<P, N, 1, 2, few ? 3 : 2, L1>(A, st);
+    else if constexpr (N >= 7)
+      launch_wilson_mma_shape<P, N, 1, 1, 2, L1>(A, st);
+    else
+      launch_wilson_mma_shape<P, N, 2, 1, few ? 2 : 3, L1>(A, st);
+  };
+  if (A.nrhs % 8)
+    go(std::true_type{});
+  else
+    go(std::false_type{});
+}
+
 template <int N, int NST>
 void launch_wilson_tc(const DslashArgs& A, cudaStream_t st) {
   TcDslashArgs T;
@@ -89,10 +140,12 @@ void launch_wilson_tc(const DslashArgs& A, cudaStream_t st) {
 }
 
 // variant: 1 = direct loads, 2 / 3 = TMA ring of 2 / 3 stages (projected
-// half-spinor operands, dslash_tc.cuh); 4 / 5 / 6 = the spinor-operand kernel
-// (dslash_tcs.cuh) with (TMA stages, B buffers) = (4, 3) / (6, 3) / (5, 2);
-// 7 / 8 = the same with one 32-RHS half per stage, (8, 2) / (6, 2)
+// half-spinor operands, dslash_tc.cuh); 4 / 6 = the spinor-operand kernel
+// (dslash_tcs.cuh) with (TMA stages, B buffers) = (4, 3) / (5, 2); 7 / 8 = the
+// same with one 32-RHS half per stage, (8, 2) / (6, 2); 5 = the
+// register-fragment MMA kernel (dslash_mma.cuh; FP16 and BF16 of either layout)
 constexpr int kTcVariants = 8;  // <= 15 (registry keys)
+constexpr int kMmaVariant = 5;
 using TcLauncher = void (*)(const DslashArgs&, cudaStream_t);
 void register_tc(int prec, int N, int variant, TcLauncher fn);
 TcLauncher find_tc(int prec, int N, int variant = 1);

@@ -517,6 +517,43 @@ void gauge_tc_records_bf16(int N, const void* src_fp64, void* dst, const Geometr
   QCU_CHECK_CUDA(cudaGetLastError());
 }
 
+namespace {
+// one thread per link of a record, sites fastest: the component reads are
+// contiguous over the warp, each thread writes its N * N elements in one run
+template <int P>
+__global__ void gauge_site_records_kernel(const double2* __restrict__ src, void* dst, Geometry geo, int N) {
+  using S = Store<P>;
+  using E = typename S::elem;
+  const int64_t vh = geo.vh, n = 16 * vh;
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
+    const uint32_t site = (uint32_t)(i % vh), pd = (uint32_t)(i / vh);
+    const uint32_t p = pd >> 3, d = pd & 7u;
+    const bool back = d & 1u;
+    const uint32_t lsite = back ? EoSite(geo, site).nb(geo, p, (int)d) : site;
+    const int64_t blk = (int64_t)(d & ~1u) + (back ? 1u - p : p);  // 2 mu + the link's parity
+    const double2* s = src + blk * N * N * vh + lsite;
+    E* o = static_cast<E*>(dst) + (((int64_t)p * vh + site) * 8 + d) * N * N;
+    for (int a = 0; a < N; a++)
+      for (int b = 0; b < N; b++) {
+        const double2 u = s[(int64_t)(back ? b * N + a : a * N + b) * vh];
+        o[a * N + b] = S::from_c(make_float2((float)u.x, (float)(back ? -u.y : u.y)));
+      }
+  }
+}
+}  // namespace
+
+void gauge_site_records(int prec, int N, const void* src_fp64, void* dst, const Geometry& geo, cudaStream_t st) {
+  const int block = 256;
+  const int grid = (int)std::min<int64_t>((16 * (int64_t)geo.vh + block - 1) / block, 152 * 32);
+  const double2* s = static_cast<const double2*>(src_fp64);
+  if (prec == PREC_HALF)
+    gauge_site_records_kernel<PREC_HALF><<<grid, block, 0, st>>>(s, dst, geo, N);
+  else
+    gauge_site_records_kernel<PREC_BF16><<<grid, block, 0, st>>>(s, dst, geo, N);
+  QCU_CHECK_CUDA(cudaGetLastError());
+}
+
 double su3_row_deviation(const void* src_fp64, int64_t vh, unsigned* scratch, cudaStream_t st) {
   QCU_CHECK_CUDA(cudaMemsetAsync(scratch, 0, sizeof(unsigned), st));
   const int block = 256;

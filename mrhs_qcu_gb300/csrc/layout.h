@@ -56,6 +56,13 @@ constexpr int kTcLinkBytes = 256;
 constexpr int kTcRecordBytes = 8 * kTcLinkBytes;
 inline size_t tc_links_bytes(int64_t vh) { return (size_t)2 * vh * kTcRecordBytes; }
 void gauge_tc_records_bf16(int N, const void* src_fp64, void* dst, const Geometry& geo, cudaStream_t st);
+// 16-bit links for the register-fragment MMA dslash (dslash_mma.cuh), one
+// record per output site and parity: [parity 2][Vh][hop 8][N][N] complex in
+// `prec` (FP16 or BF16), the matrix W that the hop multiplies by: U_mu(x) for
+// hop 2 mu (forward), U_mu(x - mu)^dag for hop 2 mu + 1 (backward).  Built
+// from the FP64 master [8][N*N][Vh].
+inline size_t site_records_bytes(int64_t vh, int N) { return (size_t)2 * vh * 8 * N * N * 4; }
+void gauge_site_records(int prec, int N, const void* src_fp64, void* dst, const Geometry& geo, cudaStream_t st);
 // per-RHS coalesced arrays (the reference's internal layout, one [ncomp][vh]
 // complex array per RHS, include/basic_data/qcu_point.cuh:80-88 of the
 // reference) <-> one MRHS field [ncomp][vh][nrhs], FP32 or FP64 (no

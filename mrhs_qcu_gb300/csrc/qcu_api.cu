@@ -674,7 +674,6 @@ int qcuTuneDslash(int nrhs, int precision, int* rhs_per_thread, int* block, int*
     qcu::DslashArgs A;
     A.gauge = s.gauge(precision);
     A.gauge12 = s.gauge12(precision);
-    if (qcu::prec_bf16(precision) && nrhs % 4 == 0) A.gauge_tc = s.gauge_tc();
     A.in = fi.data;
     A.in_norm = fi.norm;
     A.out = fo.data;
@@ -694,7 +693,10 @@ int qcuTuneDslash(int nrhs, int precision, int* rhs_per_thread, int* block, int*
     // the shape the dslash uses: the pinned or cached choice, else tuned now
     bool found = false;
     qcu::DslashConfig c = s.tuner.lookup(precision, s.N, nrhs, s.geo.vh, &found);
-    if (!found) c = s.tuner.tune(A, precision, s.N, s.stream());
+    if (!found) {
+      s.tensor_links(A, precision, -1);
+      c = s.tuner.tune(A, precision, s.N, s.stream());
+    }
     if (rhs_per_thread) *rhs_per_thread = c.R;
     if (block) *block = c.block;
     if (min_blocks) *min_blocks = c.minb;

@@ -233,12 +233,12 @@ DslashConfig Autotuner::tune(const DslashArgs& A, int prec, int N, cudaStream_t 
       best = c;
     }
   }
-  // the tensor-core kernel, where these arguments fit it; at N <= 4 the
-  // CUDA-core kernels were faster at every RHS count measured (16^3x32, nrhs
-  // 16-64), so component-major fields do not time them there
+  // the tensor-core kernels, where these arguments fit them; at N <= 4 the
+  // CUDA-core kernels were faster than the tcgen05 ones at every RHS count
+  // measured (16^3x32, nrhs 16-64), so component-major fields do not time those there
   for (int variant = 1; variant <= kTcVariants; variant++) {
     if (!tc_runs(A, prec, N, variant)) continue;
-    if (N <= 4 && !prec_site_major(prec)) continue;
+    if (N <= 4 && !prec_site_major(prec) && variant != kMmaVariant) continue;
     DslashConfig c;
     c.tc = variant;
     launch_dslash(A, prec, N, c, st);  // warm-up
@@ -308,7 +308,7 @@ void Session::load_gauge(const void* caller_gauge, int lex) {
   void* d = gauge_[PREC_DOUBLE].ensure(bytes);
   pack_gauge(PREC_DOUBLE, N, caller_gauge, lex, d, geo, stream());
   for (int p = 0; p < 5; p++) gauge_valid_[p] = gauge12_valid_[p] = false;
-  gauge_tc_valid_ = false;
+  gauge_tc_valid_ = gauge_rec_valid_[0] = gauge_rec_valid_[1] = false;
   gauge_valid_[PREC_DOUBLE] = true;
   su3_dev_ = -1.0;
   gauge_loaded_ = true;
@@ -357,6 +357,17 @@ const void* Session::gauge_tc() {
     gauge_tc_valid_ = true;
   }
   return gauge_tc_.get();
+}
+
+const void* Session::gauge_rec(int prec) {
+  QCU_REQUIRE(gauge_loaded_, QCU_ERR_NO_GAUGE, "localGauge_ is nullptr, not loaded.\n");
+  const int i = prec == PREC_HALF ? 0 : 1;
+  if (!gauge_rec_valid_[i]) {
+    void* d = gauge_rec_[i].ensure(site_records_bytes(geo.vh, N));
+    gauge_site_records(prec == PREC_HALF ? PREC_HALF : PREC_BF16, N, gauge_[PREC_DOUBLE].get(), d, geo, stream());
+    gauge_rec_valid_[i] = true;
+  }
+  return gauge_rec_[i].get();
 }
 
 void Session::load_clover(const void* caller_clover) {
@@ -476,8 +487,6 @@ void Session::hop(FieldView out, FieldView in, FieldView x, int parity, int dagg
   DslashArgs A;
   A.gauge = gauge(in.prec);
   A.gauge12 = gauge12(in.prec);
-  // BF16 RHS counts the spinor-operand tensor-core kernel takes
-  if (prec_bf16(in.prec) && in.nrhs % 4 == 0) A.gauge_tc = gauge_tc();
   A.in = in.data;
   A.in_norm = in.norm;
   A.out = out.data;
@@ -498,8 +507,16 @@ void Session::hop(FieldView out, FieldView in, FieldView x, int parity, int dagg
   DslashConfig c = tuner.lookup(in.prec, N, in.nrhs, geo.vh, &found);
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   QCU_CHECK_CUDA(cudaStreamIsCapturing(stream(), &cs));
-  if (!found && tuner.enabled() && cs == cudaStreamCaptureStatusNone) c = tuner.tune(A, in.prec, N, stream());
+  const bool tunes = !found && tuner.enabled() && cs == cudaStreamCaptureStatusNone;
+  tensor_links(A, in.prec, tunes ? -1 : c.tc);
+  if (tunes) c = tuner.tune(A, in.prec, N, stream());
   launch_dslash(A, in.prec, N, c, stream());
+}
+
+void Session::tensor_links(DslashArgs& A, int prec, int tc) {
+  if (!prec_is16(prec) || A.nrhs % 4) return;  // the RHS counts that these kernels take
+  if (tc < 0 || tc == kMmaVariant) A.gauge_rec = gauge_rec(prec);
+  if (prec_bf16(prec) && (tc < 0 || (tc >= 4 && tc != kMmaVariant))) A.gauge_tc = gauge_tc();
 }
 
 Blas& Session::blas() {

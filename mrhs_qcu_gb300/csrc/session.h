@@ -165,6 +165,12 @@ class Session {
   // gauge_tc_records_bf16), for the spinor-operand tensor-core dslash; built
   // on first use
   const void* gauge_tc();
+  // the links in FP16 or BF16 as per-site records of the hops' matrices
+  // (layout.h gauge_site_records), for the register-fragment MMA dslash;
+  // built on first use
+  const void* gauge_rec(int prec);
+  // sets in A the link forms that tensor-core variant tc reads (0: none; -1: any, for tuning)
+  void tensor_links(DslashArgs& A, int prec, int tc);
 
   // ---- clover term (clover.h) ---------------------------------------------
   // caller field [2][Vh][2][2N][2N] complex double, Hermitian blocks; packed
@@ -207,6 +213,8 @@ class Session {
   bool gauge12_valid_[5] = {false, false, false, false, false};
   DeviceBuffer gauge_tc_;
   bool gauge_tc_valid_ = false;
+  DeviceBuffer gauge_rec_[2];  // FP16, BF16
+  bool gauge_rec_valid_[2] = {false, false};
   double su3_dev_ = -1.0;  // max |row 2 - conj(row 0 x row 1)|, < 0: not measured
   DeviceBuffer su3_scratch_;
   bool clover_loaded_ = false;
