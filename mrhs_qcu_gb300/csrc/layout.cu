@@ -16,8 +16,8 @@
 // per-(site, RHS) scale for 16-bit storage), and the source may be
 // lexicographic: the lexicographic -> even-odd map is applied on the fly.
 #include <algorithm>
-
 #include <cstring>
+#include <type_traits>
 
 #include "layout.h"
 
@@ -37,100 +37,209 @@ __device__ __forceinline__ int64_t src_site(int mode, int64_t i, int p, const Ge
   return (((int64_t)t * g.L[2] + z) * g.L[1] + y) * g.L[0] + X;
 }
 
+// Both fermion transforms go through a shared-memory tile of ts sites x tr RHS
+// x 4N components, so that either side of memory is walked in its own
+// contiguous order: the caller fields site by site (all components of a site,
+// 64 N bytes, lie together), the MRHS field by (site, RHS) runs of one
+// component (site-major layout: by (component, RHS) runs of one site).  One
+// thread per (site, RHS) instead touches a cache line per lane on the caller
+// side.  The tile rows (one per component) are an odd number of elements
+// apart, which keeps both sides free of bank conflicts.
+// Bound by HBM.  32-bit fields, 24^3x48 SU(3) nrhs 12, lexicographic caller
+// fields, both parities packed and unpacked (4.6 GB): 2044 us with one thread
+// per (site, RHS), 991 us here.
+struct FermionTile {
+  int ts_log2, tr;  // sites (a power of two) and RHS per tile
+  FastDiv div_tr, div_chunks;
+  int pitch;        // elements between the tile's component rows
+};
+
+// the tile element: FP16 needs the FP64 values until the site's scale is known
+template <int P>
+struct TileElem {
+  using t = std::conditional_t<Store<P>::has_norm, double2, typename Store<P>::elem>;
+};
+
+constexpr int kTileThreads = 256;
+
+// the caller pointer of each tile RHS (a lane-indexed read of the parameter
+// itself is served one address at a time) and the caller site, in complexes,
+// of each tile site
+__device__ __forceinline__ void tile_tables(const void** ptr, int64_t* caller, const PtrArray& p, int r0, int rhs,
+                                            int nc, int64_t site0, int nsites, int mode, int parity,
+                                            const Geometry& g) {
+  for (int s = threadIdx.x; s < nsites; s += kTileThreads) caller[s] = src_site(mode, site0 + s, parity, g) * nc;
+  for (int r = threadIdx.x; r < rhs; r += kTileThreads) ptr[r] = p.p[r0 + r];
+}
+
 template <int P, int N>
-__global__ void pack_fermions_kernel(PtrArray src, int mode, int parity, void* dst, float* dst_norm, Geometry g,
-                                     int nrhs, FastDiv div_nrhs) {
+__global__ void __launch_bounds__(kTileThreads)
+    pack_fermions_kernel(const __grid_constant__ PtrArray src, int mode, int parity, void* dst, float* dst_norm,
+                         Geometry g, int nrhs, FermionTile T) {
   using S = Store<P>;
   using E = typename S::elem;
-  const uint32_t gid = blockIdx.x * blockDim.x + threadIdx.x;
-  uint32_t site, r;
-  div_nrhs.divmod(gid, site, r);
-  if ((int)site >= g.vh || src.p[r] == nullptr) return;  // a null pointer leaves RHS r untouched
-  const double2* s = static_cast<const double2*>(src.p[r]) + src_site(mode, site, parity, g) * (4 * N);
-  double2 v[4 * N];
+  using TE = typename TileElem<P>::t;
+  constexpr int NC = 4 * N;
+  extern __shared__ __align__(16) unsigned char tile_smem[];
+  const int ts = 1 << T.ts_log2;
+  TE* const tile = reinterpret_cast<TE*>(tile_smem);  // [NC][pitch], element s * tr + r
+  int64_t* const caller = reinterpret_cast<int64_t*>(tile_smem + (((size_t)NC * T.pitch * sizeof(TE) + 7) & ~(size_t)7));
+  const void** const ptr = reinterpret_cast<const void**>(caller + ts);
+  double* const inv = reinterpret_cast<double*>(ptr + T.tr);  // FP16: [ts * tr]
+  uint32_t tile_no, chunk;  // the RHS chunks of a tile of sites run together: their rows share pages
+  T.div_chunks.divmod(blockIdx.x, tile_no, chunk);
+  const int64_t site0 = (int64_t)tile_no << T.ts_log2;
+  const int nsites = (int)min((int64_t)ts, g.vh - site0);
+  const int r0 = (int)chunk * T.tr, rhs = min(T.tr, nrhs - r0);
+  tile_tables(ptr, caller, src, r0, rhs, NC, site0, nsites, mode, parity, g);
+  __syncthreads();
+  const int n = NC * rhs << T.ts_log2;
+  constexpr int U = 4;  // loads in flight per thread
+  for (int k0 = threadIdx.x; k0 < n; k0 += U * kTileThreads) {  // component fastest, then site, then RHS
+    double2 v[U];
+    int at[U];
 #pragma unroll
-  for (int c = 0; c < 4 * N; c++) v[c] = __ldg(s + c);
-  // component c at site * ss + c * cs + r (component- or site-major, by P)
-  const int64_t cs = field_comp_stride(P, g.vh, 4 * N, nrhs), ss = field_site_stride(P, g.vh, 4 * N, nrhs);
-  E* d = static_cast<E*>(dst) + (int64_t)site * ss + r;
-  if constexpr (S::has_norm) {
-    double m = 0.0;
+    for (int i = 0; i < U; i++) {
+      const int k = k0 + i * kTileThreads, q = k / NC, c = k - q * NC, s = q & (ts - 1), r = q >> T.ts_log2;
+      const double2* f = k < n ? static_cast<const double2*>(ptr[r]) : nullptr;
+      at[i] = -1;
+      if (s >= nsites || f == nullptr) continue;  // a null pointer leaves RHS r untouched
+      at[i] = c * T.pitch + s * T.tr + r;
+      v[i] = __ldcs(f + (caller[s] + c));
+    }
 #pragma unroll
-    for (int c = 0; c < 4 * N; c++) m = fmax(m, fmax(fabs(v[c].x), fabs(v[c].y)));
-    const float mf = (float)m;
-    const double inv = m > 0.0 ? 1.0 / (double)mf : 0.0;
-    dst_norm[(int64_t)site * nrhs + r] = mf;
-#pragma unroll
-    for (int c = 0; c < 4 * N; c++) d[c * cs] = S::from_c(make_float2((float)(v[c].x * inv), (float)(v[c].y * inv)));
-  } else {
-#pragma unroll
-    for (int c = 0; c < 4 * N; c++) {
-      E e;
-      e.x = v[c].x;
-      e.y = v[c].y;
-      d[c * cs] = e;
+    for (int i = 0; i < U; i++) {
+      if (at[i] < 0) continue;
+      if constexpr (S::has_norm)
+        tile[at[i]] = v[i];
+      else
+        tile[at[i]] = S::from_z(v[i]);
     }
   }
-}
-
-template <int P, int N>
-__global__ void unpack_fermions_kernel(PtrArray dstp, int mode, int parity, const void* src, const float* src_norm,
-                                       Geometry g, int nrhs, FastDiv div_nrhs) {
-  using S = Store<P>;
-  using E = typename S::elem;
-  const uint32_t gid = blockIdx.x * blockDim.x + threadIdx.x;
-  uint32_t site, r;
-  div_nrhs.divmod(gid, site, r);
-  if ((int)site >= g.vh || dstp.p[r] == nullptr) return;  // a null pointer skips RHS r
-  const int64_t cs = field_comp_stride(P, g.vh, 4 * N, nrhs), ss = field_site_stride(P, g.vh, 4 * N, nrhs);
-  const E* s = static_cast<const E*>(src) + (int64_t)site * ss + r;
-  double2* d = static_cast<double2*>(const_cast<void*>(dstp.p[r])) + src_site(mode, site, parity, g) * (4 * N);
-  double scale = 1.0;
-  if constexpr (S::has_norm) scale = (double)src_norm[(int64_t)site * nrhs + r];
+  __syncthreads();
+  if constexpr (S::has_norm) {
+    for (int k = threadIdx.x; k < T.tr << T.ts_log2; k += kTileThreads) {
+      uint32_t s, r;
+      T.div_tr.divmod((uint32_t)k, s, r);
+      if ((int)s >= nsites || (int)r >= rhs || ptr[r] == nullptr) continue;
+      double m = 0.0;
 #pragma unroll
-  for (int c = 0; c < 4 * N; c++) {
-    auto v = S::to_c(s[c * cs]);
-    d[c] = make_double2((double)v.x * scale, (double)v.y * scale);
+      for (int c = 0; c < NC; c++) m = fmax(m, fmax(fabs(tile[c * T.pitch + k].x), fabs(tile[c * T.pitch + k].y)));
+      const float mf = (float)m;
+      inv[k] = m > 0.0 ? 1.0 / (double)mf : 0.0;
+      dst_norm[(site0 + s) * nrhs + r0 + r] = mf;
+    }
+    __syncthreads();
   }
+  // a warp per component row (site-major: per site), RHS fastest
+  constexpr bool kSiteMajor = prec_site_major(P);
+  const int64_t cs = field_comp_stride(P, g.vh, NC, nrhs), ss = field_site_stride(P, g.vh, NC, nrhs);
+  E* const out = static_cast<E*>(dst) + site0 * ss + r0;
+  const int outer = kSiteMajor ? nsites : NC, inner = T.tr * (kSiteMajor ? NC : nsites);
+  for (int o = threadIdx.x >> 5; o < outer; o += kTileThreads / 32)
+#pragma unroll 4
+    for (int k = threadIdx.x & 31; k < inner; k += 32) {
+      uint32_t q, r;
+      T.div_tr.divmod((uint32_t)k, q, r);
+      const int c = kSiteMajor ? (int)q : o, s = kSiteMajor ? o : (int)q;
+      if ((int)r >= rhs || ptr[r] == nullptr) continue;
+      const TE v = tile[c * T.pitch + s * T.tr + (int)r];
+      E e;
+      if constexpr (S::has_norm) {
+        const double w = inv[s * T.tr + (int)r];
+        e = S::from_z(make_double2(v.x * w, v.y * w));
+      } else {
+        e = v;
+      }
+      out[s * ss + c * cs + r] = e;
+    }
 }
 
-// Unpack through a shared-memory tile (caller layouts whose sites are
-// contiguous: one parity or both parities in eo order).  A block stages ts
-// sites x tr RHS of the MRHS field as FP64 complex: the reads walk the
-// field's contiguous (site, RHS) runs of each component, the writes each
-// RHS's contiguous run of ts sites x 4N caller components.  (One thread per
-// (site, RHS) scatters every warp's writes over up to 32 RHS arrays.)
 template <int P, int N>
-__global__ void unpack_fermions_tiled_kernel(PtrArray dstp, int mode, int parity, const void* src,
-                                             const float* src_norm, Geometry g, int nrhs, int ts, int tr) {
+__global__ void __launch_bounds__(kTileThreads)
+    unpack_fermions_kernel(const __grid_constant__ PtrArray dstp, int mode, int parity, const void* src,
+                           const float* src_norm, Geometry g, int nrhs, FermionTile T) {
   using S = Store<P>;
   using E = typename S::elem;
   constexpr int NC = 4 * N;
-  extern __shared__ double2 tile[];  // [tr][ts][NC]
-  const int64_t site0 = (int64_t)blockIdx.x * ts;
-  const int r0 = blockIdx.y * tr;
+  extern __shared__ __align__(16) unsigned char tile_smem[];
+  const int ts = 1 << T.ts_log2;
+  E* const tile = reinterpret_cast<E*>(tile_smem);
+  int64_t* const caller = reinterpret_cast<int64_t*>(tile_smem + (((size_t)NC * T.pitch * sizeof(E) + 7) & ~(size_t)7));
+  const void** const ptr = reinterpret_cast<const void**>(caller + ts);
+  float* const scale = reinterpret_cast<float*>(ptr + T.tr);  // FP16: [ts * tr]
+  uint32_t tile_no, chunk;  // the RHS chunks of a tile of sites run together: their rows share pages
+  T.div_chunks.divmod(blockIdx.x, tile_no, chunk);
+  const int64_t site0 = (int64_t)tile_no << T.ts_log2;
+  const int nsites = (int)min((int64_t)ts, g.vh - site0);
+  const int r0 = (int)chunk * T.tr, rhs = min(T.tr, nrhs - r0);
+  tile_tables(ptr, caller, dstp, r0, rhs, NC, site0, nsites, mode, parity, g);
+  constexpr bool kSiteMajor = prec_site_major(P);
   const int64_t cs = field_comp_stride(P, g.vh, NC, nrhs), ss = field_site_stride(P, g.vh, NC, nrhs);
-  const E* in = static_cast<const E*>(src);
-  const int n = NC * ts * tr;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    const int r = i % tr, s = (i / tr) % ts, c = i / (tr * ts);
-    const int64_t site = site0 + s;
-    const int rhs = r0 + r;
-    if (site >= g.vh || rhs >= nrhs) continue;
-    const auto v = S::to_c(in[site * ss + c * cs + rhs]);
-    double scale = 1.0;
-    if constexpr (S::has_norm) scale = (double)src_norm[site * nrhs + rhs];
-    tile[((int64_t)r * ts + s) * NC + c] = make_double2((double)v.x * scale, (double)v.y * scale);
+  const E* const in = static_cast<const E*>(src) + site0 * ss + r0;
+  const int outer = kSiteMajor ? nsites : NC, inner = T.tr * (kSiteMajor ? NC : nsites);
+  constexpr int U = 4;  // loads in flight per thread
+  for (int o = threadIdx.x >> 5; o < outer; o += kTileThreads / 32)
+    for (int k0 = threadIdx.x & 31; k0 < inner; k0 += 32 * U) {
+      E v[U];
+      int at[U];
+#pragma unroll
+      for (int i = 0; i < U; i++) {
+        const int k = k0 + 32 * i;
+        uint32_t q, r;
+        T.div_tr.divmod((uint32_t)k, q, r);
+        const int c = kSiteMajor ? (int)q : o, s = kSiteMajor ? o : (int)q;
+        at[i] = -1;
+        if (k >= inner || (int)r >= rhs) continue;
+        at[i] = c * T.pitch + s * T.tr + (int)r;
+        v[i] = in[s * ss + c * cs + r];
+      }
+#pragma unroll
+      for (int i = 0; i < U; i++)
+        if (at[i] >= 0) tile[at[i]] = v[i];
+    }
+  if constexpr (S::has_norm) {
+    for (int k = threadIdx.x; k < T.tr << T.ts_log2; k += kTileThreads) {
+      uint32_t s, r;
+      T.div_tr.divmod((uint32_t)k, s, r);
+      if ((int)s < nsites && (int)r < rhs) scale[k] = src_norm[(site0 + s) * nrhs + r0 + r];
+    }
   }
   __syncthreads();
-  const int64_t base = (mode == SRC_EO_FULL ? (int64_t)parity * g.vh : 0) + site0;  // caller site of site0
-  const int nsites = (int)min((int64_t)ts, g.vh - site0);
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    const int r = i / (ts * NC), rem = i - r * ts * NC;
-    const int rhs = r0 + r;
-    if (rem >= nsites * NC || rhs >= nrhs || dstp.p[rhs] == nullptr) continue;  // a null pointer skips RHS r
-    static_cast<double2*>(const_cast<void*>(dstp.p[rhs]))[base * NC + rem] = tile[(int64_t)r * ts * NC + rem];
+  const int n = NC * rhs << T.ts_log2;
+#pragma unroll 4
+  for (int k = threadIdx.x; k < n; k += kTileThreads) {
+    const int q = k / NC, c = k - q * NC, s = q & (ts - 1), r = q >> T.ts_log2;
+    double2* f = static_cast<double2*>(const_cast<void*>(ptr[r]));
+    if (s >= nsites || f == nullptr) continue;  // a null pointer skips RHS r
+    double2 v = S::to_z(tile[c * T.pitch + s * T.tr + r]);
+    if constexpr (S::has_norm) {
+      const double w = to_f64(scale[s * T.tr + r]);
+      v.x *= w;
+      v.y *= w;
+    }
+    f[caller[s] + c] = v;
   }
+}
+
+// Tile of at most 24 KB: up to 32 RHS, then as many sites as fit (at most 64).
+// 12 and 8 KB tiles take 1.1x and 1.3-1.5x the time (24^3x48 SU(3) nrhs 12), 46
+// KB ones the same.  Small fields take fewer sites per tile, down to 4, until
+// every SM has four tiles: there the latency of one tile is the cost.
+template <typename TE>
+FermionTile fermion_tile(int nc, int nrhs, int64_t vh, size_t extra_per_unit, size_t* smem) {
+  FermionTile T;
+  T.tr = std::min(nrhs, 32);
+  const int chunks = (nrhs + T.tr - 1) / T.tr;
+  T.ts_log2 = 0;
+  while (T.ts_log2 < 6 && ((size_t)nc * T.tr * sizeof(TE) << (T.ts_log2 + 1)) <= 24 * 1024) T.ts_log2++;
+  while (T.ts_log2 > 2 && (vh >> T.ts_log2) * chunks < 4 * 152) T.ts_log2--;
+  T.div_tr = FastDiv((uint32_t)T.tr);
+  T.div_chunks = FastDiv((uint32_t)chunks);
+  const int units = T.tr << T.ts_log2;
+  T.pitch = units | 1;
+  *smem = (((size_t)nc * T.pitch * sizeof(TE) + 7) & ~(size_t)7) + ((size_t)8 << T.ts_log2) + 8 * T.tr + extra_per_unit * units;
+  return T;
 }
 
 // gauge: caller (eo or lexicographic) complex double -> [4][2][N*N][Vh] P
@@ -299,54 +408,47 @@ __global__ void transpose_c64_kernel(const double2* __restrict__ src, double2* _
   }
 }
 
+template <int P, int N>
+void pack_pn(const PtrArray& src, int mode, int parity, void* dst, float* dst_norm, const Geometry& g, int nrhs,
+             cudaStream_t st) {
+  size_t smem = 0;
+  const FermionTile T =
+      fermion_tile<typename TileElem<P>::t>(4 * N, nrhs, g.vh, Store<P>::has_norm ? sizeof(double) : 0, &smem);
+  const unsigned grid = (unsigned)((g.vh + (1 << T.ts_log2) - 1) >> T.ts_log2) * T.div_chunks.d;
+  pack_fermions_kernel<P, N><<<grid, kTileThreads, smem, st>>>(src, mode, parity, dst, dst_norm, g, nrhs, T);
+}
+
+template <int P, int N>
+void unpack_pn(const PtrArray& dst, int mode, int parity, const void* src, const float* src_norm, const Geometry& g,
+               int nrhs, cudaStream_t st) {
+  size_t smem = 0;
+  const FermionTile T =
+      fermion_tile<typename Store<P>::elem>(4 * N, nrhs, g.vh, Store<P>::has_norm ? sizeof(float) : 0, &smem);
+  const unsigned grid = (unsigned)((g.vh + (1 << T.ts_log2) - 1) >> T.ts_log2) * T.div_chunks.d;
+  unpack_fermions_kernel<P, N><<<grid, kTileThreads, smem, st>>>(dst, mode, parity, src, src_norm, g, nrhs, T);
+}
+
 template <int N>
 void pack_n(int prec, const PtrArray& src, int mode, int parity, void* dst, float* dst_norm, const Geometry& g,
             int nrhs, cudaStream_t st) {
-  const int64_t threads = (int64_t)g.vh * nrhs;
-  const int block = 128;
-  const int grid = (int)((threads + block - 1) / block);
-  FastDiv dn((uint32_t)nrhs);
   switch (prec) {
-    case PREC_DOUBLE: pack_fermions_kernel<PREC_DOUBLE, N><<<grid, block, 0, st>>>(src, mode, parity, dst, dst_norm, g, nrhs, dn); break;
-    case PREC_SINGLE: pack_fermions_kernel<PREC_SINGLE, N><<<grid, block, 0, st>>>(src, mode, parity, dst, dst_norm, g, nrhs, dn); break;
-    case PREC_HALF: pack_fermions_kernel<PREC_HALF, N><<<grid, block, 0, st>>>(src, mode, parity, dst, dst_norm, g, nrhs, dn); break;
-    case PREC_BF16: pack_fermions_kernel<PREC_BF16, N><<<grid, block, 0, st>>>(src, mode, parity, dst, dst_norm, g, nrhs, dn); break;
-    case PREC_BF16S: pack_fermions_kernel<PREC_BF16S, N><<<grid, block, 0, st>>>(src, mode, parity, dst, dst_norm, g, nrhs, dn); break;
+    case PREC_DOUBLE: pack_pn<PREC_DOUBLE, N>(src, mode, parity, dst, dst_norm, g, nrhs, st); break;
+    case PREC_SINGLE: pack_pn<PREC_SINGLE, N>(src, mode, parity, dst, dst_norm, g, nrhs, st); break;
+    case PREC_HALF: pack_pn<PREC_HALF, N>(src, mode, parity, dst, dst_norm, g, nrhs, st); break;
+    case PREC_BF16: pack_pn<PREC_BF16, N>(src, mode, parity, dst, dst_norm, g, nrhs, st); break;
+    case PREC_BF16S: pack_pn<PREC_BF16S, N>(src, mode, parity, dst, dst_norm, g, nrhs, st); break;
   }
 }
 
 template <int N>
 void unpack_n(int prec, const PtrArray& dst, int mode, int parity, const void* src, const float* src_norm,
               const Geometry& g, int nrhs, cudaStream_t st) {
-  if (mode != SRC_LEX) {
-    // tiles of ts sites x tr RHS, 24 KB of FP64 complex in shared memory (32^3x64, FP32,
-    // nrhs 12: 0.83 ms, against 1.15 ms with 48 KB tiles and 0.89 ms with 12 KB)
-    const int tr = std::min(nrhs, 16);
-    const int ts = std::max(1, std::min(32, 1536 / (tr * 4 * N)));
-    const dim3 grid((unsigned)((g.vh + ts - 1) / ts), (unsigned)((nrhs + tr - 1) / tr));
-    const size_t smem = (size_t)ts * tr * 4 * N * sizeof(double2);
-#define QCU_UNPACK_TILED(PR)                                                                                      \
-  unpack_fermions_tiled_kernel<PR, N><<<grid, 256, smem, st>>>(dst, mode, parity, src, src_norm, g, nrhs, ts, tr); \
-  return;
-    switch (prec) {
-      case PREC_DOUBLE: QCU_UNPACK_TILED(PREC_DOUBLE)
-      case PREC_SINGLE: QCU_UNPACK_TILED(PREC_SINGLE)
-      case PREC_HALF: QCU_UNPACK_TILED(PREC_HALF)
-      case PREC_BF16: QCU_UNPACK_TILED(PREC_BF16)
-      case PREC_BF16S: QCU_UNPACK_TILED(PREC_BF16S)
-    }
-#undef QCU_UNPACK_TILED
-  }
-  const int64_t threads = (int64_t)g.vh * nrhs;
-  const int block = 128;
-  const int grid = (int)((threads + block - 1) / block);
-  FastDiv dn((uint32_t)nrhs);
   switch (prec) {
-    case PREC_DOUBLE: unpack_fermions_kernel<PREC_DOUBLE, N><<<grid, block, 0, st>>>(dst, mode, parity, src, src_norm, g, nrhs, dn); break;
-    case PREC_SINGLE: unpack_fermions_kernel<PREC_SINGLE, N><<<grid, block, 0, st>>>(dst, mode, parity, src, src_norm, g, nrhs, dn); break;
-    case PREC_HALF: unpack_fermions_kernel<PREC_HALF, N><<<grid, block, 0, st>>>(dst, mode, parity, src, src_norm, g, nrhs, dn); break;
-    case PREC_BF16: unpack_fermions_kernel<PREC_BF16, N><<<grid, block, 0, st>>>(dst, mode, parity, src, src_norm, g, nrhs, dn); break;
-    case PREC_BF16S: unpack_fermions_kernel<PREC_BF16S, N><<<grid, block, 0, st>>>(dst, mode, parity, src, src_norm, g, nrhs, dn); break;
+    case PREC_DOUBLE: unpack_pn<PREC_DOUBLE, N>(dst, mode, parity, src, src_norm, g, nrhs, st); break;
+    case PREC_SINGLE: unpack_pn<PREC_SINGLE, N>(dst, mode, parity, src, src_norm, g, nrhs, st); break;
+    case PREC_HALF: unpack_pn<PREC_HALF, N>(dst, mode, parity, src, src_norm, g, nrhs, st); break;
+    case PREC_BF16: unpack_pn<PREC_BF16, N>(dst, mode, parity, src, src_norm, g, nrhs, st); break;
+    case PREC_BF16S: unpack_pn<PREC_BF16S, N>(dst, mode, parity, src, src_norm, g, nrhs, st); break;
   }
 }
 

@@ -186,6 +186,44 @@ struct EoSite {
 };
 
 // ---------------------------------------------------------------------------
+// FP64 <-> 32- and 16-bit conversions on the integer pipe.  The conversion
+// instructions issue on the FP64 pipe (2 lanes a cycle and SM here, 1/64 of
+// the FP32 rate): a layout transform of FP32 fields kept it 76% busy and ran
+// at 58% of HBM.  Same rounding (to nearest even) and results as the
+// instructions, which the values outside the normal range still take.
+__device__ __forceinline__ float to_f32(double v) {
+#ifdef __CUDA_ARCH__
+  const uint64_t u = (uint64_t)__double_as_longlong(v), a = u & 0x7fffffffffffffffull;
+  const uint32_t sign = (uint32_t)(u >> 32) & 0x80000000u;
+  if (a - 0x3810000000000000ull < 0x47f0000000000000ull - 0x3810000000000000ull)  // 2^-126 <= |v| < 2^128
+    return __uint_as_float(sign | (uint32_t)((a - 0x3800000000000000ull + 0x0fffffffull + ((a >> 29) & 1u)) >> 29));
+  if (a == 0) return __uint_as_float(sign);
+#endif
+  return (float)v;
+}
+__device__ __forceinline__ double to_f64(float v) {
+#ifdef __CUDA_ARCH__
+  const uint32_t u = __float_as_uint(v), a = u & 0x7fffffffu;
+  const uint64_t sign = (uint64_t)(u & 0x80000000u) << 32;
+  if (a - 0x00800000u < 0x7f800000u - 0x00800000u)  // normal
+    return __longlong_as_double((long long)(sign | (((uint64_t)a << 29) + 0x3800000000000000ull)));
+  if (a == 0) return __longlong_as_double((long long)sign);
+#endif
+  return (double)v;
+}
+__device__ __forceinline__ __nv_bfloat16 to_bf16(double v) {
+#ifdef __CUDA_ARCH__
+  const uint64_t u = (uint64_t)__double_as_longlong(v), a = u & 0x7fffffffffffffffull;
+  const uint32_t sign = (uint32_t)(u >> 48) & 0x8000u;
+  if (a - 0x3810000000000000ull < 0x47f0000000000000ull - 0x3810000000000000ull)
+    return __ushort_as_bfloat16((unsigned short)(
+        sign | (uint32_t)((a - 0x3800000000000000ull + 0xfffffffffffull + ((a >> 45) & 1u)) >> 45)));
+  if (a == 0) return __ushort_as_bfloat16((unsigned short)sign);
+#endif
+  return __double2bfloat16(v);
+}
+
+// ---------------------------------------------------------------------------
 // storage traits: how a complex number of precision P sits in memory and how
 // it converts to the compute type (double for FP64, float otherwise)
 template <int P> struct Store;
@@ -196,6 +234,8 @@ template <> struct Store<PREC_DOUBLE> {
   static constexpr bool has_norm = false;
   __device__ __forceinline__ static double2 to_c(double2 v) { return v; }
   __device__ __forceinline__ static double2 from_c(double2 v) { return v; }
+  __device__ __forceinline__ static double2 from_z(double2 v) { return v; }
+  __device__ __forceinline__ static double2 to_z(double2 v) { return v; }
 };
 template <> struct Store<PREC_SINGLE> {
   using elem = float2;
@@ -203,6 +243,8 @@ template <> struct Store<PREC_SINGLE> {
   static constexpr bool has_norm = false;
   __device__ __forceinline__ static float2 to_c(float2 v) { return v; }
   __device__ __forceinline__ static float2 from_c(float2 v) { return v; }
+  __device__ __forceinline__ static float2 from_z(double2 v) { return make_float2(to_f32(v.x), to_f32(v.y)); }
+  __device__ __forceinline__ static double2 to_z(float2 v) { return make_double2(to_f64(v.x), to_f64(v.y)); }
 };
 template <> struct Store<PREC_HALF> {
   using elem = __half2;
@@ -210,6 +252,11 @@ template <> struct Store<PREC_HALF> {
   static constexpr bool has_norm = true;
   __device__ __forceinline__ static float2 to_c(__half2 v) { return __half22float2(v); }
   __device__ __forceinline__ static __half2 from_c(float2 v) { return __float22half2_rn(v); }
+  __device__ __forceinline__ static __half2 from_z(double2 v) { return from_c(make_float2(to_f32(v.x), to_f32(v.y))); }
+  __device__ __forceinline__ static double2 to_z(__half2 v) {
+    const float2 f = to_c(v);
+    return make_double2(to_f64(f.x), to_f64(f.y));
+  }
 };
 template <> struct Store<PREC_BF16> {
   using elem = __nv_bfloat162;
@@ -217,6 +264,17 @@ template <> struct Store<PREC_BF16> {
   static constexpr bool has_norm = false;
   __device__ __forceinline__ static float2 to_c(__nv_bfloat162 v) { return __bfloat1622float2(v); }
   __device__ __forceinline__ static __nv_bfloat162 from_c(float2 v) { return __float22bfloat162_rn(v); }
+  // (rounded once)
+  __device__ __forceinline__ static __nv_bfloat162 from_z(double2 v) {
+    __nv_bfloat162 e;
+    e.x = to_bf16(v.x);
+    e.y = to_bf16(v.y);
+    return e;
+  }
+  __device__ __forceinline__ static double2 to_z(__nv_bfloat162 v) {
+    const float2 f = to_c(v);
+    return make_double2(to_f64(f.x), to_f64(f.y));
+  }
 };
 // site-major BF16: the same element, another layout
 template <> struct Store<PREC_BF16S> : Store<PREC_BF16> {};
