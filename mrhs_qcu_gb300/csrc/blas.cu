@@ -10,19 +10,13 @@
 #include <algorithm>
 
 #include "blas.h"
-
-// arithmetic helper for the complex reduction value type
-__device__ __forceinline__ double2 operator+(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
+#include "layout.h"  // QCU_MAX_RHS
 
 namespace qcu {
 namespace {
 
-__device__ __forceinline__ double shfl_xor(double v, int off) { return __shfl_xor_sync(0xffffffffu, v, off); }
-__device__ __forceinline__ double2 shfl_xor(double2 v, int off) {
-  return make_double2(__shfl_xor_sync(0xffffffffu, v.x, off), __shfl_xor_sync(0xffffffffu, v.y, off));
-}
-
 constexpr int kMaxBlocks = 1024;
+constexpr int kMaxThreads = 1024;  // block_size: a multiple of 32 and of the RHS groups (31 groups: 992)
 
 template <typename T> struct V2;
 template <> struct V2<double> { using t = double2; };
@@ -47,18 +41,121 @@ __device__ __forceinline__ float2 cmulf(float2 a, float2 b) {
 }
 __device__ __forceinline__ float2 tof(double2 a) { return make_float2((float)a.x, (float)a.y); }
 
-template <typename E>
-__device__ __forceinline__ double2 ld(const E* p) {
-  E v = *p;
-  return make_double2((double)v.x, (double)v.y);
+// FP64 values of a complex element, and back (integer-pipe conversions, qcu_common.cuh)
+__device__ __forceinline__ double2 ld(const double2* p) { return *p; }
+__device__ __forceinline__ double2 ld(const float2* p) { return Store<PREC_SINGLE>::to_z(*p); }
+__device__ __forceinline__ void st(double2* p, double2 v) { *p = v; }
+__device__ __forceinline__ void st(float2* p, double2 v) { *p = Store<PREC_SINGLE>::from_z(v); }
+
+// FP64 sum of FP32 products in groups.  One conversion and FP64 addition per
+// product is bound by the FP64 pipe (2 lanes a cycle and SM, and the
+// conversion issues there too): the norm of 24^3x48 SU(3) nrhs 12 FP32 took
+// 195 us against 56 us of HBM time.  So a few products are added in FP32 with
+// their rounding errors kept (Knuth's TwoSum), and two values per group go to
+// FP64.  Products that would take the group out of FP32's range, or are not
+// finite, go to FP64 themselves.
+struct GroupSum {
+  float hi = 0.f, lo = 0.f;
+  __device__ __forceinline__ void add(double& acc, float p) {
+    const float s = __fadd_rn(hi, p), b = __fsub_rn(s, hi);
+    if (fabsf(s) <= 3.402823466e38f) {
+      lo = __fadd_rn(lo, __fadd_rn(__fsub_rn(hi, __fsub_rn(s, b)), __fsub_rn(p, b)));
+      hi = s;
+    } else {
+      acc += (double)p;
+    }
+  }
+  __device__ __forceinline__ void flush(double& acc) {
+    acc += to_f64(hi);
+    acc += to_f64(lo);
+    hi = lo = 0.f;
+  }
+};
+constexpr int kGroup = 4;  // products per group
+// FP64 products accumulate as they are formed
+__device__ __forceinline__ void add_square(double& acc, double2 v) {
+  acc = fma(v.x, v.x, acc);
+  acc = fma(v.y, v.y, acc);
 }
-template <typename E>
-__device__ __forceinline__ void st(E* p, double2 v) {
-  E e;
-  e.x = v.x;
-  e.y = v.y;
-  *p = e;
+__device__ __forceinline__ void add_conj(double2& acc, double2 u, double2 v) {  // conj(u) v
+  acc.x = fma(u.x, v.x, acc.x);
+  acc.x = fma(u.y, v.y, acc.x);
+  acc.y = fma(u.x, v.y, acc.y);
+  acc.y = fma(-u.y, v.x, acc.y);
 }
+// per-RHS sums of one thread: FP32 fields in groups, FP64 fields directly
+template <int P>
+struct NormSum {
+  double acc = 0.0;
+  GroupSum g;
+  __device__ __forceinline__ void add(float2 v) { g.add(acc, fmaf(v.x, v.x, v.y * v.y)); }
+  __device__ __forceinline__ void add(double2 v) { add_square(acc, v); }
+  __device__ __forceinline__ void flush() {
+    if constexpr (P == PREC_SINGLE) g.flush(acc);
+  }
+};
+template <int P>
+struct DotSum {  // conj(u) v
+  double2 acc = make_double2(0.0, 0.0);
+  GroupSum re, im;
+  __device__ __forceinline__ void add(float2 u, float2 v) {
+    re.add(acc.x, fmaf(u.x, v.x, u.y * v.y));
+    im.add(acc.y, fmaf(u.x, v.y, -u.y * v.x));
+  }
+  __device__ __forceinline__ void add(double2 u, double2 v) { add_conj(acc, u, v); }
+  __device__ __forceinline__ void flush() {
+    if constexpr (P == PREC_SINGLE) {
+      re.flush(acc.x);
+      im.flush(acc.y);
+    }
+  }
+};
+template <typename A, typename S, int R>
+__device__ __forceinline__ void totals(A (&out)[R], const S (&sums)[R]) {
+#pragma unroll
+  for (int i = 0; i < R; i++) out[i] = sums[i].acc;
+}
+
+// chunk c of a field: R complex elements, one 16-byte vector for FP32 R = 2 and FP64 R = 1
+template <int R>
+__device__ __forceinline__ void load_chunk(const float2* f, int64_t c, float2 (&v)[R]) {
+  if constexpr (R == 2) {
+    const float4 q = reinterpret_cast<const float4*>(f)[c];
+    v[0] = make_float2(q.x, q.y);
+    v[1] = make_float2(q.z, q.w);
+  } else {
+#pragma unroll
+    for (int i = 0; i < R; i++) v[i] = f[c * R + i];
+  }
+}
+template <int R>
+__device__ __forceinline__ void store_chunk(float2* f, int64_t c, const float2 (&v)[R]) {
+  if constexpr (R == 2) {
+    reinterpret_cast<float4*>(f)[c] = make_float4(v[0].x, v[0].y, v[1].x, v[1].y);
+  } else {
+#pragma unroll
+    for (int i = 0; i < R; i++) f[c * R + i] = v[i];
+  }
+}
+template <int R>
+__device__ __forceinline__ void load_chunk(const double2* f, int64_t c, double2 (&v)[R]) {
+#pragma unroll
+  for (int i = 0; i < R; i++) v[i] = f[c * R + i];
+}
+template <int R>
+__device__ __forceinline__ void store_chunk(double2* f, int64_t c, const double2 (&v)[R]) {
+#pragma unroll
+  for (int i = 0; i < R; i++) f[c * R + i] = v[i];
+}
+// y + a x in the fields' own arithmetic
+__device__ __forceinline__ float2 add_mul(float2 a, float2 x, float2 y) {
+  return make_float2(fmaf(a.x, x.x, fmaf(-a.y, x.y, y.x)), fmaf(a.x, x.y, fmaf(a.y, x.x, y.y)));
+}
+__device__ __forceinline__ double2 add_mul(double2 a, double2 x, double2 y) {
+  return make_double2(fma(a.x, x.x, fma(-a.y, x.y, y.x)), fma(a.x, x.y, fma(a.y, x.x, y.y)));
+}
+__device__ __forceinline__ void coeff(double2 a, float2& c) { c = tof(a); }
+__device__ __forceinline__ void coeff(double2 a, double2& c) { c = a; }
 
 // block-level per-RHS reduction of `vals` (R values per thread) into
 // out[blockIdx.x * nrhs + r]
@@ -86,7 +183,7 @@ __device__ void block_reduce(A* sm, const A* vals, int R, int G, int nrhs, A* ou
 
 // ---------------------------------------------------------------------------
 template <int PX, int PY, int R, bool NORM>
-__global__ void axpby_kernel(const double2* __restrict__ a, const void* __restrict__ xv, const double2* __restrict__ b,
+__global__ void __launch_bounds__(kMaxThreads, 1) axpby_kernel(const double2* __restrict__ a, const void* __restrict__ xv, const double2* __restrict__ b,
                              void* __restrict__ yv, Shape s, double* partials) {
   using EX = typename V2<typename BT<PX>::real>::t;
   using EY = typename V2<typename BT<PY>::real>::t;
@@ -111,35 +208,28 @@ __global__ void axpby_kernel(const double2* __restrict__ a, const void* __restri
       fa[i] = tof(ca[i]);
       fb[i] = tof(cb[i]);
     }
-    for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < s.nchunks; c += stride) {
-      float2 xs[R], ys[R];
-      if constexpr (R == 2) {  // one 16-byte vector per operand (chunks are 16-byte aligned)
-        const float4 xq = reinterpret_cast<const float4*>(x)[c], yq = reinterpret_cast<const float4*>(y)[c];
-        xs[0] = make_float2(xq.x, xq.y);
-        xs[1] = make_float2(xq.z, xq.w);
-        ys[0] = make_float2(yq.x, yq.y);
-        ys[1] = make_float2(yq.z, yq.w);
-      } else {
+    NormSum<PREC_SINGLE> sum[R];
+    for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < s.nchunks;) {
+#pragma unroll
+      for (int u = 0; u < (NORM ? kGroup : 1); u++, c += stride) {
+        if (c >= s.nchunks) break;
+        float2 xs[R], ys[R];
+        load_chunk<R>(x, c, xs);
+        load_chunk<R>(y, c, ys);
 #pragma unroll
         for (int i = 0; i < R; i++) {
-          xs[i] = x[c * R + i];
-          ys[i] = y[c * R + i];
+          const float2 v = cmulf(fa[i], xs[i]), w = cmulf(fb[i], ys[i]);
+          ys[i] = make_float2(v.x + w.x, v.y + w.y);
+          if (NORM) sum[i].add(ys[i]);
         }
+        store_chunk<R>(y, c, ys);
       }
-      float2 v[R];
+      if (NORM) {
 #pragma unroll
-      for (int i = 0; i < R; i++) {
-        const float2 u = cmulf(fa[i], xs[i]), w = cmulf(fb[i], ys[i]);
-        v[i] = make_float2(u.x + w.x, u.y + w.y);
-        if (NORM) acc[i] += (double)fmaf(v[i].x, v[i].x, v[i].y * v[i].y);
-      }
-      if constexpr (R == 2) {
-        reinterpret_cast<float4*>(y)[c] = make_float4(v[0].x, v[0].y, v[1].x, v[1].y);
-      } else {
-#pragma unroll
-        for (int i = 0; i < R; i++) y[c * R + i] = v[i];
+        for (int i = 0; i < R; i++) sum[i].flush();
       }
     }
+    totals(acc, sum);
   } else if (b == nullptr) {
     // b = 1: no multiply of y (FP64 arithmetic is bound by the FP64 pipe here)
     for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < s.nchunks; c += stride) {
@@ -148,7 +238,7 @@ __global__ void axpby_kernel(const double2* __restrict__ a, const void* __restri
         const int64_t e = c * R + i;
         const double2 v = cmul(ca[i], ld(x + e)) + ld(y + e);
         st(y + e, v);
-        if (NORM) acc[i] += v.x * v.x + v.y * v.y;
+        if (NORM) add_square(acc[i], v);
       }
     }
   } else {
@@ -158,7 +248,7 @@ __global__ void axpby_kernel(const double2* __restrict__ a, const void* __restri
         const int64_t e = c * R + i;
         const double2 v = cmul(ca[i], ld(x + e)) + cmul(cb[i], ld(y + e));
         st(y + e, v);
-        if (NORM) acc[i] += v.x * v.x + v.y * v.y;
+        if (NORM) add_square(acc[i], v);
       }
     }
   }
@@ -169,7 +259,7 @@ __global__ void axpby_kernel(const double2* __restrict__ a, const void* __restri
 }
 
 template <int P, int R>
-__global__ void axpbypcz_kernel(const double2* __restrict__ a, const void* __restrict__ xv,
+__global__ void __launch_bounds__(kMaxThreads, 1) axpbypcz_kernel(const double2* __restrict__ a, const void* __restrict__ xv,
                                 const double2* __restrict__ b, const void* __restrict__ yv,
                                 const double2* __restrict__ c, void* __restrict__ zv, Shape s) {
   using E = typename V2<typename BT<P>::real>::t;
@@ -239,52 +329,312 @@ __global__ void axpbypcz_kernel(const double2* __restrict__ a, const void* __res
 // MODE 0: |x|^2, 1: <x, y>.  FAST (FP32 fields): the products in FP32, summed
 // in FP64; otherwise every product is formed in FP64 (exact for FP32 inputs).
 template <int PX, int PY, int R, int MODE, bool FAST = false>
-__global__ void reduce_kernel(const void* __restrict__ xv, const void* __restrict__ yv, Shape s, void* partials) {
+__global__ void __launch_bounds__(kMaxThreads, 1) reduce_kernel(const void* __restrict__ xv, const void* __restrict__ yv, Shape s, void* partials) {
   using EX = typename V2<typename BT<PX>::real>::t;
   using EY = typename V2<typename BT<PY>::real>::t;
   const EX* x = static_cast<const EX*>(xv);
   const EY* y = static_cast<const EY*>(yv);
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  if (MODE == 0) {
-    double acc[R];
+  // FAST: FP32 products in groups; else the elements in FP64
+  constexpr int PS = FAST ? PREC_SINGLE : PREC_DOUBLE;
+  auto val = [](const EX& e) {
+    if constexpr (FAST)
+      return e;
+    else
+      return ld(&e);
+  };
+  if constexpr (MODE == 0) {
+    NormSum<PS> sum[R];
+    for (int64_t c0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c0 < s.nchunks; c0 += kGroup * stride) {
+      EX v[kGroup][R];
 #pragma unroll
-    for (int i = 0; i < R; i++) acc[i] = 0.0;
-    for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < s.nchunks; k += stride) {
+      for (int u = 0; u < kGroup; u++) {
+#pragma unroll
+        for (int i = 0; i < R; i++) v[u][i] = EX{};
+        if (c0 + u * stride < s.nchunks) load_chunk<R>(x, c0 + u * stride, v[u]);
+      }
 #pragma unroll
       for (int i = 0; i < R; i++) {
-        if constexpr (FAST) {
-          const float2 v = reinterpret_cast<const float2*>(x)[k * R + i];
-          acc[i] += (double)fmaf(v.x, v.x, v.y * v.y);
-        } else {
-          const double2 v = ld(x + k * R + i);
-          acc[i] += v.x * v.x + v.y * v.y;
-        }
+#pragma unroll
+        for (int u = 0; u < kGroup; u++) sum[i].add(val(v[u][i]));
+        sum[i].flush();
       }
     }
+    double acc[R];
+    totals(acc, sum);
     __shared__ double sm[1024 * 2];
     block_reduce<double>(sm, acc, R, s.G, s.nrhs, static_cast<double*>(partials));
   } else {
-    double2 acc[R];
+    static_assert(PX == PY, "one precision");
+    DotSum<PS> sum[R];
+    for (int64_t c0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c0 < s.nchunks; c0 += kGroup * stride) {
+      EX a[kGroup][R], b[kGroup][R];
 #pragma unroll
-    for (int i = 0; i < R; i++) acc[i] = make_double2(0.0, 0.0);
-    for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < s.nchunks; k += stride) {
+      for (int u = 0; u < kGroup; u++) {
+#pragma unroll
+        for (int i = 0; i < R; i++) a[u][i] = EX{}, b[u][i] = EX{};
+        if (c0 + u * stride >= s.nchunks) continue;
+        load_chunk<R>(x, c0 + u * stride, a[u]);
+        load_chunk<R>(y, c0 + u * stride, b[u]);
+      }
 #pragma unroll
       for (int i = 0; i < R; i++) {
-        if constexpr (FAST) {
-          const float2 u = reinterpret_cast<const float2*>(x)[k * R + i];
-          const float2 v = reinterpret_cast<const float2*>(y)[k * R + i];
-          acc[i].x += (double)fmaf(u.x, v.x, u.y * v.y);  // conj(u) v
-          acc[i].y += (double)fmaf(u.x, v.y, -u.y * v.x);
-        } else {
-          const double2 u = ld(x + k * R + i), v = ld(y + k * R + i);
-          acc[i].x += u.x * v.x + u.y * v.y;  // conj(u) v
-          acc[i].y += u.x * v.y - u.y * v.x;
-        }
+#pragma unroll
+        for (int u = 0; u < kGroup; u++) sum[i].add(val(a[u][i]), val(b[u][i]));
+        sum[i].flush();
       }
     }
+    double2 acc[R];
+    totals(acc, sum);
     __shared__ double2 sm2[1024 * 2];
     block_reduce<double2>(sm2, acc, R, s.G, s.nrhs, static_cast<double2*>(partials));
   }
+}
+
+// ---- fused kernels of the Krylov iterations (solver.cu) ----------------------
+// s -= a q, r -= a w; partial |s|^2 (part) and |r|^2 (part2)
+template <int P, int R>
+__global__ void __launch_bounds__(kMaxThreads, 1) cg_update_kernel(const double2* __restrict__ a, const void* __restrict__ qv, void* __restrict__ sv,
+                                 const void* __restrict__ wv, void* __restrict__ rv, Shape sh, double* part,
+                                 double* part2) {
+  using E = typename V2<typename BT<P>::real>::t;
+  const E *q = static_cast<const E*>(qv), *w = static_cast<const E*>(wv);
+  E *s = static_cast<E*>(sv), *r = static_cast<E*>(rv);
+  const int g = threadIdx.x % sh.G;
+  E na[R];
+#pragma unroll
+  for (int i = 0; i < R; i++) {
+    const double2 c = a[g * R + i];
+    coeff(make_double2(-c.x, -c.y), na[i]);
+  }
+  NormSum<P> sums[R], sumr[R];
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < sh.nchunks;) {
+#pragma unroll
+    for (int u = 0; u < kGroup; u++, c += stride) {
+      if (c >= sh.nchunks) break;
+      E qs[R], ss[R], ws[R], rs[R];
+      load_chunk<R>(q, c, qs);
+      load_chunk<R>(s, c, ss);
+      load_chunk<R>(w, c, ws);
+      load_chunk<R>(r, c, rs);
+#pragma unroll
+      for (int i = 0; i < R; i++) {
+        ss[i] = add_mul(na[i], qs[i], ss[i]);
+        rs[i] = add_mul(na[i], ws[i], rs[i]);
+        sums[i].add(ss[i]);
+        sumr[i].add(rs[i]);
+      }
+      store_chunk<R>(s, c, ss);
+      store_chunk<R>(r, c, rs);
+    }
+#pragma unroll
+    for (int i = 0; i < R; i++) {
+      sums[i].flush();
+      sumr[i].flush();
+    }
+  }
+  double accs[R], accr[R];
+  totals(accs, sums);
+  totals(accr, sumr);
+  __shared__ double sm[1024 * 2];
+  block_reduce<double>(sm, accs, R, sh.G, sh.nrhs, part);
+  __syncthreads();
+  block_reduce<double>(sm, accr, R, sh.G, sh.nrhs, part2);
+}
+
+// x += a p, p = r + b p (a and b real)
+template <int P, int R>
+__global__ void __launch_bounds__(kMaxThreads, 1) cg_direction_kernel(const double2* __restrict__ a, const double2* __restrict__ b,
+                                    const void* __restrict__ rv, void* __restrict__ pv, void* __restrict__ xv,
+                                    Shape sh) {
+  using E = typename V2<typename BT<P>::real>::t;
+  const E* r = static_cast<const E*>(rv);
+  E *p = static_cast<E*>(pv), *x = static_cast<E*>(xv);
+  const int g = threadIdx.x % sh.G;
+  E ca[R], cb[R];
+#pragma unroll
+  for (int i = 0; i < R; i++) {
+    coeff(a[g * R + i], ca[i]);
+    coeff(b[g * R + i], cb[i]);
+  }
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < sh.nchunks; c += stride) {
+    E rs[R], ps[R], xs[R];
+    load_chunk<R>(r, c, rs);
+    load_chunk<R>(p, c, ps);
+    load_chunk<R>(x, c, xs);
+#pragma unroll
+    for (int i = 0; i < R; i++) {
+      xs[i].x = fma(ca[i].x, ps[i].x, xs[i].x);
+      xs[i].y = fma(ca[i].x, ps[i].y, xs[i].y);
+      ps[i].x = fma(cb[i].x, ps[i].x, rs[i].x);
+      ps[i].y = fma(cb[i].x, ps[i].y, rs[i].y);
+    }
+    store_chunk<R>(x, c, xs);
+    store_chunk<R>(p, c, ps);
+  }
+}
+
+// partial <x, y> (part2) and |x|^2 (part)
+template <int P, int R>
+__global__ void __launch_bounds__(kMaxThreads, 1) dot_norm_kernel(const void* __restrict__ xv, const void* __restrict__ yv, Shape sh, double* part,
+                                double2* part2) {
+  using E = typename V2<typename BT<P>::real>::t;
+  const E *x = static_cast<const E*>(xv), *y = static_cast<const E*>(yv);
+  NormSum<P> nrm[R];
+  DotSum<P> dot[R];
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  constexpr int U = kGroup / 2;  // loads of two chunks at a time
+  for (int64_t c0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c0 < sh.nchunks; c0 += U * stride) {
+    E a[U][R], b[U][R];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+#pragma unroll
+      for (int i = 0; i < R; i++) a[u][i] = E{}, b[u][i] = E{};
+      if (c0 + u * stride >= sh.nchunks) continue;
+      load_chunk<R>(x, c0 + u * stride, a[u]);
+      load_chunk<R>(y, c0 + u * stride, b[u]);
+    }
+#pragma unroll
+    for (int i = 0; i < R; i++) {
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        dot[i].add(a[u][i], b[u][i]);
+        nrm[i].add(a[u][i]);
+      }
+      dot[i].flush();
+      nrm[i].flush();
+    }
+  }
+  double2 accd[R];
+  double accn[R];
+  totals(accd, dot);
+  totals(accn, nrm);
+  __shared__ double2 sm[1024 * 2];
+  block_reduce<double2>(sm, accd, R, sh.G, sh.nrhs, part2);
+  __syncthreads();
+  block_reduce<double>(reinterpret_cast<double*>(sm), accn, R, sh.G, sh.nrhs, part);
+}
+
+// x += a p + o s, s -= o t; partial |s|^2 (part) and <r0, s> (part2)
+template <int P, int R>
+__global__ void __launch_bounds__(kMaxThreads, 1) bicg_update_kernel(const double2* __restrict__ a, const double2* __restrict__ o,
+                                   const void* __restrict__ pv, void* __restrict__ sv, const void* __restrict__ tv,
+                                   const void* __restrict__ r0v, void* __restrict__ xv, Shape sh, double* part,
+                                   double2* part2) {
+  using E = typename V2<typename BT<P>::real>::t;
+  const E *p = static_cast<const E*>(pv), *t = static_cast<const E*>(tv), *r0 = static_cast<const E*>(r0v);
+  E *s = static_cast<E*>(sv), *x = static_cast<E*>(xv);
+  const int g = threadIdx.x % sh.G;
+  E ca[R], co[R];
+#pragma unroll
+  for (int i = 0; i < R; i++) {
+    coeff(a[g * R + i], ca[i]);
+    coeff(o[g * R + i], co[i]);
+  }
+  NormSum<P> nrm[R];
+  DotSum<P> dot[R];
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < sh.nchunks;) {
+#pragma unroll
+    for (int u = 0; u < kGroup; u++, c += stride) {
+      if (c >= sh.nchunks) break;
+      E ps[R], ss[R], ts[R], rs[R], xs[R];
+      load_chunk<R>(p, c, ps);
+      load_chunk<R>(s, c, ss);
+      load_chunk<R>(t, c, ts);
+      load_chunk<R>(r0, c, rs);
+      load_chunk<R>(x, c, xs);
+#pragma unroll
+      for (int i = 0; i < R; i++) {
+        E no;
+        no.x = -co[i].x;
+        no.y = -co[i].y;
+        xs[i] = add_mul(co[i], ss[i], add_mul(ca[i], ps[i], xs[i]));
+        ss[i] = add_mul(no, ts[i], ss[i]);
+        nrm[i].add(ss[i]);
+        dot[i].add(rs[i], ss[i]);
+      }
+      store_chunk<R>(x, c, xs);
+      store_chunk<R>(s, c, ss);
+    }
+#pragma unroll
+    for (int i = 0; i < R; i++) {
+      nrm[i].flush();
+      dot[i].flush();
+    }
+  }
+  double2 accd[R];
+  double accn[R];
+  totals(accd, dot);
+  totals(accn, nrm);
+  __shared__ double2 sm[1024 * 2];
+  block_reduce<double2>(sm, accd, R, sh.G, sh.nrhs, part2);
+  __syncthreads();
+  block_reduce<double>(reinterpret_cast<double*>(sm), accn, R, sh.G, sh.nrhs, part);
+}
+
+// ---- masked moves between fields of selected RHS (no arithmetic on the others) ----
+// xh += xl, xl = 0; d = be - xh where d is given (FP64 xh, be, d; xl in P)
+template <int P>
+__global__ void fold_kernel(const int* __restrict__ sel, void* __restrict__ xlv, double2* __restrict__ xh,
+                            const double2* __restrict__ be, double2* __restrict__ d, Shape sh) {
+  using E = typename V2<typename BT<P>::real>::t;
+  if (!sel[threadIdx.x % sh.G]) return;
+  E* xl = static_cast<E*>(xlv);
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < sh.nchunks; c += stride) {
+    const double2 v = ld(xl + c) + xh[c];
+    xh[c] = v;
+    xl[c] = E{};
+    if (d) {
+      const double2 b = be[c];
+      d[c] = make_double2(b.x - v.x, b.y - v.y);
+    }
+  }
+}
+
+// y = x (converted), z = x where z is given; x = nullptr: y = 0
+template <int PX, int PY>
+__global__ void select_copy_kernel(const int* __restrict__ sel, const void* __restrict__ xv, void* __restrict__ yv,
+                                   void* __restrict__ zv, Shape sh) {
+  using EX = typename V2<typename BT<PX>::real>::t;
+  using EY = typename V2<typename BT<PY>::real>::t;
+  if (!sel[threadIdx.x % sh.G]) return;
+  const EX* x = static_cast<const EX*>(xv);
+  EY *y = static_cast<EY*>(yv), *z = static_cast<EY*>(zv);
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < sh.nchunks; c += stride) {
+    EY e{};
+    if (x) {
+      if constexpr (PX == PY)
+        e = x[c];
+      else
+        st(&e, ld(x + c));
+    }
+    y[c] = e;
+    if (z) z[c] = e;
+  }
+}
+
+// partial |x|^2 of the FP64 field x over every RHS; selected RHS: y = x converted to P
+template <int P>
+__global__ void residual_kernel(const int* __restrict__ sel, const double2* __restrict__ x, void* __restrict__ yv,
+                                Shape sh, double* part) {
+  using E = typename V2<typename BT<P>::real>::t;
+  E* y = static_cast<E*>(yv);
+  const bool mine = sel[threadIdx.x % sh.G] != 0;
+  double acc[1] = {0.0};
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  if (mine)
+    for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < sh.nchunks; c += stride) {
+      const double2 v = x[c];
+      add_square(acc[0], v);
+      st(y + c, v);
+    }
+  __shared__ double sm[1024];
+  block_reduce<double>(sm, acc, 1, sh.G, sh.nrhs, part);
 }
 
 // one warp per RHS: lane l sums the block partials l, l + 32, ... in order,
@@ -293,10 +643,7 @@ template <typename A>
 __global__ void finalize_kernel(const A* __restrict__ partials, int nblocks, int nrhs, A* out) {
   const int r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (r >= nrhs) return;  // whole warps leave together
-  A s = A{};
-  for (int b = lane; b < nblocks; b += 32) s = s + partials[(int64_t)b * nrhs + r];
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) s = s + shfl_xor(s, off);
+  const A s = sum_partials(partials, nblocks, nrhs, r, lane);
   if (lane == 0) out[r] = s;
 }
 
@@ -450,12 +797,11 @@ void Blas::cdot(const FieldRef& x, const FieldRef& y, double2* out, cudaStream_t
   check_field(y);
   QCU_REQUIRE(x.n == y.n && x.nrhs == y.nrhs && x.prec == y.prec, QCU_ERR_INVALID_ARGUMENT,
               "cdot: shape/precision mismatch");
-  const int R = pick_r(x);
+  const int R = pick_r(x, y.data);
   Shape s = make_shape(x, R);
   const int B = block_size(s.G);
   QCU_REQUIRE(B <= 1024, QCU_ERR_UNSUPPORTED, "nrhs too large for BLAS block");
   const int grid = grid_for(s.nchunks, B);
-  QCU_REQUIRE(2 * grid <= max_blocks_ * 2, QCU_ERR_INVALID_ARGUMENT, "partials too small");
   double2* p2 = reinterpret_cast<double2*>(partials_);
   if (x.prec == PREC_DOUBLE)
     reduce_kernel<PREC_DOUBLE, PREC_DOUBLE, 1, 1><<<grid, B, 0, st>>>(x.data, y.data, s, p2);
@@ -465,6 +811,166 @@ void Blas::cdot(const FieldRef& x, const FieldRef& y, double2* out, cudaStream_t
     reduce_kernel<PREC_SINGLE, PREC_SINGLE, 1, 1, true><<<grid, B, 0, st>>>(x.data, y.data, s, p2);
   QCU_CHECK_CUDA(cudaGetLastError());
   finalize<double2>(p2, grid, x.nrhs, out, st);
+  QCU_CHECK_CUDA(cudaGetLastError());
+}
+
+double* Blas::norms(int k) const { return partials_ + (size_t)(2 + k) * max_blocks_ * QCU_MAX_RHS; }
+
+namespace {
+struct Launch {
+  Shape s;
+  int R, block, grid;
+};
+Launch plan(const FieldRef& f, int R) {
+  Launch l;
+  l.R = R;
+  l.s = make_shape(f, R);
+  l.block = block_size(l.s.G);
+  QCU_REQUIRE(l.block <= 1024, QCU_ERR_UNSUPPORTED, "nrhs too large for BLAS block");
+  l.grid = grid_for(l.s.nchunks, l.block);
+  return l;
+}
+void check_same(const FieldRef& a, const FieldRef& b, const char* what) {
+  check_field(a);
+  check_field(b);
+  QCU_REQUIRE(a.n == b.n && a.nrhs == b.nrhs && a.prec == b.prec, QCU_ERR_INVALID_ARGUMENT,
+              std::string(what) + ": shape/precision mismatch");
+}
+}  // namespace
+
+Partials Blas::norm2_partials(const FieldRef& x, cudaStream_t st) {
+  check_field(x);
+  const Launch l = plan(x, pick_r(x));
+  double* p = norms(0);
+  if (x.prec == PREC_DOUBLE)
+    reduce_kernel<PREC_DOUBLE, PREC_DOUBLE, 1, 0><<<l.grid, l.block, 0, st>>>(x.data, x.data, l.s, p);
+  else if (l.R == 2)
+    reduce_kernel<PREC_SINGLE, PREC_SINGLE, 2, 0, true><<<l.grid, l.block, 0, st>>>(x.data, x.data, l.s, p);
+  else
+    reduce_kernel<PREC_SINGLE, PREC_SINGLE, 1, 0, true><<<l.grid, l.block, 0, st>>>(x.data, x.data, l.s, p);
+  QCU_CHECK_CUDA(cudaGetLastError());
+  return Partials{p, nullptr, nullptr, l.grid};
+}
+
+Partials Blas::dot_partials(const FieldRef& x, const FieldRef& y, cudaStream_t st) {
+  check_same(x, y, "dot");
+  const Launch l = plan(x, pick_r(x, y.data));
+  if (x.prec == PREC_DOUBLE)
+    reduce_kernel<PREC_DOUBLE, PREC_DOUBLE, 1, 1><<<l.grid, l.block, 0, st>>>(x.data, y.data, l.s, dots());
+  else if (l.R == 2)
+    reduce_kernel<PREC_SINGLE, PREC_SINGLE, 2, 1, true><<<l.grid, l.block, 0, st>>>(x.data, y.data, l.s, dots());
+  else
+    reduce_kernel<PREC_SINGLE, PREC_SINGLE, 1, 1, true><<<l.grid, l.block, 0, st>>>(x.data, y.data, l.s, dots());
+  QCU_CHECK_CUDA(cudaGetLastError());
+  return Partials{nullptr, nullptr, dots(), l.grid};
+}
+
+Partials Blas::dot_norm(const FieldRef& x, const FieldRef& y, cudaStream_t st) {
+  check_same(x, y, "dot_norm");
+  const Launch l = plan(x, pick_r(x, y.data));
+  if (x.prec == PREC_DOUBLE)
+    dot_norm_kernel<PREC_DOUBLE, 1><<<l.grid, l.block, 0, st>>>(x.data, y.data, l.s, norms(0), dots());
+  else if (l.R == 2)
+    dot_norm_kernel<PREC_SINGLE, 2><<<l.grid, l.block, 0, st>>>(x.data, y.data, l.s, norms(0), dots());
+  else
+    dot_norm_kernel<PREC_SINGLE, 1><<<l.grid, l.block, 0, st>>>(x.data, y.data, l.s, norms(0), dots());
+  QCU_CHECK_CUDA(cudaGetLastError());
+  return Partials{norms(0), nullptr, dots(), l.grid};
+}
+
+Partials Blas::cg_update(const double2* a, const FieldRef& q, const FieldRef& s, const FieldRef& w, const FieldRef& r,
+                         cudaStream_t st) {
+  check_same(q, s, "cg_update");
+  check_same(w, r, "cg_update");
+  check_same(q, r, "cg_update");
+  const int R = std::min(pick_r(q, s.data), pick_r(w, r.data));
+  const Launch l = plan(q, R);
+  if (q.prec == PREC_DOUBLE)
+    cg_update_kernel<PREC_DOUBLE, 1><<<l.grid, l.block, 0, st>>>(a, q.data, s.data, w.data, r.data, l.s, norms(0), norms(1));
+  else if (R == 2)
+    cg_update_kernel<PREC_SINGLE, 2><<<l.grid, l.block, 0, st>>>(a, q.data, s.data, w.data, r.data, l.s, norms(0), norms(1));
+  else
+    cg_update_kernel<PREC_SINGLE, 1><<<l.grid, l.block, 0, st>>>(a, q.data, s.data, w.data, r.data, l.s, norms(0), norms(1));
+  QCU_CHECK_CUDA(cudaGetLastError());
+  return Partials{norms(0), norms(1), nullptr, l.grid};
+}
+
+void Blas::cg_direction(const double2* a, const double2* b, const FieldRef& r, const FieldRef& p, const FieldRef& x,
+                        cudaStream_t st) {
+  check_same(r, p, "cg_direction");
+  check_same(p, x, "cg_direction");
+  const Launch l = plan(r, pick_r(r, p.data, x.data));
+  if (r.prec == PREC_DOUBLE)
+    cg_direction_kernel<PREC_DOUBLE, 1><<<l.grid, l.block, 0, st>>>(a, b, r.data, p.data, x.data, l.s);
+  else if (l.R == 2)
+    cg_direction_kernel<PREC_SINGLE, 2><<<l.grid, l.block, 0, st>>>(a, b, r.data, p.data, x.data, l.s);
+  else
+    cg_direction_kernel<PREC_SINGLE, 1><<<l.grid, l.block, 0, st>>>(a, b, r.data, p.data, x.data, l.s);
+  QCU_CHECK_CUDA(cudaGetLastError());
+}
+
+Partials Blas::bicg_update(const double2* a, const double2* o, const FieldRef& p, const FieldRef& s,
+                           const FieldRef& t, const FieldRef& r0, const FieldRef& x, cudaStream_t st) {
+  check_same(p, s, "bicg_update");
+  check_same(t, r0, "bicg_update");
+  check_same(p, x, "bicg_update");
+  check_same(p, t, "bicg_update");
+  const int R = std::min(pick_r(p, s.data, t.data), pick_r(r0, x.data));
+  const Launch l = plan(p, R);
+  if (p.prec == PREC_DOUBLE)
+    bicg_update_kernel<PREC_DOUBLE, 1><<<l.grid, l.block, 0, st>>>(a, o, p.data, s.data, t.data, r0.data, x.data, l.s, norms(0), dots());
+  else if (R == 2)
+    bicg_update_kernel<PREC_SINGLE, 2><<<l.grid, l.block, 0, st>>>(a, o, p.data, s.data, t.data, r0.data, x.data, l.s, norms(0), dots());
+  else
+    bicg_update_kernel<PREC_SINGLE, 1><<<l.grid, l.block, 0, st>>>(a, o, p.data, s.data, t.data, r0.data, x.data, l.s, norms(0), dots());
+  QCU_CHECK_CUDA(cudaGetLastError());
+  return Partials{norms(0), nullptr, dots(), l.grid};
+}
+
+// the masked moves keep one RHS per thread (R = 1), so a thread is selected or leaves at once
+void Blas::fold(const int* sel, const FieldRef& xl, const FieldRef& xh, const FieldRef& be, const FieldRef& d,
+                cudaStream_t st) {
+  check_field(xl);
+  check_field(xh);
+  QCU_REQUIRE(xl.n == xh.n && xh.prec == PREC_DOUBLE, QCU_ERR_INVALID_ARGUMENT, "fold: shape/precision mismatch");
+  const Launch l = plan(xl, 1);
+  double2 *h = static_cast<double2*>(xh.data), *dd = static_cast<double2*>(d.data);
+  const double2* b = static_cast<const double2*>(be.data);
+  if (xl.prec == PREC_DOUBLE)
+    fold_kernel<PREC_DOUBLE><<<l.grid, l.block, 0, st>>>(sel, xl.data, h, b, dd, l.s);
+  else
+    fold_kernel<PREC_SINGLE><<<l.grid, l.block, 0, st>>>(sel, xl.data, h, b, dd, l.s);
+  QCU_CHECK_CUDA(cudaGetLastError());
+}
+
+void Blas::select_copy(const int* sel, const FieldRef& x, const FieldRef& y, const FieldRef& z, cudaStream_t st) {
+  check_field(y);
+  QCU_REQUIRE(!x.data || x.n == y.n, QCU_ERR_INVALID_ARGUMENT, "select_copy: shape mismatch");
+  const Launch l = plan(y, 1);
+  const int px = x.data ? x.prec : y.prec;
+  if (px == PREC_DOUBLE && y.prec == PREC_DOUBLE)
+    select_copy_kernel<PREC_DOUBLE, PREC_DOUBLE><<<l.grid, l.block, 0, st>>>(sel, x.data, y.data, z.data, l.s);
+  else if (px == PREC_DOUBLE)
+    select_copy_kernel<PREC_DOUBLE, PREC_SINGLE><<<l.grid, l.block, 0, st>>>(sel, x.data, y.data, z.data, l.s);
+  else if (y.prec == PREC_DOUBLE)
+    select_copy_kernel<PREC_SINGLE, PREC_DOUBLE><<<l.grid, l.block, 0, st>>>(sel, x.data, y.data, z.data, l.s);
+  else
+    select_copy_kernel<PREC_SINGLE, PREC_SINGLE><<<l.grid, l.block, 0, st>>>(sel, x.data, y.data, z.data, l.s);
+  QCU_CHECK_CUDA(cudaGetLastError());
+}
+
+void Blas::residual(const int* sel, const FieldRef& x, const FieldRef& y, double* out, cudaStream_t st) {
+  check_field(x);
+  check_field(y);
+  QCU_REQUIRE(x.n == y.n && x.prec == PREC_DOUBLE, QCU_ERR_INVALID_ARGUMENT, "residual: shape/precision mismatch");
+  const Launch l = plan(x, 1);
+  const double2* xp = static_cast<const double2*>(x.data);
+  if (y.prec == PREC_DOUBLE)
+    residual_kernel<PREC_DOUBLE><<<l.grid, l.block, 0, st>>>(sel, xp, y.data, l.s, norms(0));
+  else
+    residual_kernel<PREC_SINGLE><<<l.grid, l.block, 0, st>>>(sel, xp, y.data, l.s, norms(0));
+  QCU_CHECK_CUDA(cudaGetLastError());
+  finalize<double>(norms(0), l.grid, x.nrhs, out, st);
   QCU_CHECK_CUDA(cudaGetLastError());
 }
 

@@ -298,29 +298,46 @@ __global__ void convert_field_kernel(const void* src, const float* src_norm, voi
   const int64_t csi = field_comp_stride(PI, vh, ncomp, nrhs), csd = field_comp_stride(PO, vh, ncomp, nrhs);
   const auto* s = static_cast<const typename SI::elem*>(src) + (int64_t)site * field_site_stride(PI, vh, ncomp, nrhs) + r;
   auto* d = static_cast<typename SO::elem*>(dst) + (int64_t)site * field_site_stride(PO, vh, ncomp, nrhs) + r;
-  double si = 1.0;
-  if constexpr (SI::has_norm) si = (double)src_norm[(int64_t)site * nrhs + r];
-  double m = 0.0;
-  if constexpr (SO::has_norm) {
+  // 32- and 16-bit conversions in FP32 arithmetic, exact or rounded once as
+  // FP64 arithmetic would leave them (the FP64 pipe has 1/64 of the FP32 rate)
+  if constexpr (PO != PREC_DOUBLE && PI != PREC_DOUBLE && !(SI::has_norm && SO::has_norm)) {
+    float si = 1.f;
+    if constexpr (SI::has_norm) si = src_norm[(int64_t)site * nrhs + r];
+    float m = 0.f;
+    if constexpr (SO::has_norm) {
+      for (int c = 0; c < ncomp; c++) {
+        const auto v = SI::to_c(s[c * csi]);
+        m = fmaxf(m, fmaxf(fabsf(v.x), fabsf(v.y)));
+      }
+      dst_norm[(int64_t)site * nrhs + r] = m;
+    }
     for (int c = 0; c < ncomp; c++) {
       auto v = SI::to_c(s[c * csi]);
-      m = fmax(m, fmax(fabs((double)v.x * si), fabs((double)v.y * si)));
+      if constexpr (SI::has_norm) v = make_float2(v.x * si, v.y * si);
+      if constexpr (SO::has_norm)
+        v = m > 0.f ? make_float2(__fdiv_rn(v.x, m), __fdiv_rn(v.y, m)) : make_float2(0.f, 0.f);
+      d[c * csd] = SO::from_c(v);
     }
-    dst_norm[(int64_t)site * nrhs + r] = (float)m;
-  }
-  const double inv = SO::has_norm ? (m > 0.0 ? 1.0 / (double)(float)m : 0.0) : 1.0;
-  for (int c = 0; c < ncomp; c++) {
-    auto v = SI::to_c(s[c * csi]);
-    const double re = (double)v.x * si * inv, im = (double)v.y * si * inv;
-    typename SO::elem e;
-    if constexpr (PO == PREC_DOUBLE) {
-      e = make_double2(re, im);
-    } else if constexpr (PO == PREC_SINGLE) {
-      e = make_float2((float)re, (float)im);
-    } else {
-      e = SO::from_c(make_float2((float)re, (float)im));
+  } else {
+    double si = 1.0;
+    if constexpr (SI::has_norm) si = to_f64(src_norm[(int64_t)site * nrhs + r]);
+    double m = 0.0;
+    if constexpr (SO::has_norm) {
+      for (int c = 0; c < ncomp; c++) {
+        const double2 v = SI::to_z(s[c * csi]);
+        m = fmax(m, fmax(fabs(v.x * si), fabs(v.y * si)));
+      }
+      dst_norm[(int64_t)site * nrhs + r] = (float)m;
     }
-    d[c * csd] = e;
+    const double inv = SO::has_norm ? (m > 0.0 ? 1.0 / (double)(float)m : 0.0) : 1.0;
+    for (int c = 0; c < ncomp; c++) {
+      double2 v = SI::to_z(s[c * csi]);
+      if constexpr (SI::has_norm || SO::has_norm) v = make_double2(v.x * si * inv, v.y * si * inv);
+      if constexpr (PO == PREC_BF16 || PO == PREC_BF16S)
+        d[c * csd] = SO::from_c(make_float2(to_f32(v.x), to_f32(v.y)));
+      else
+        d[c * csd] = SO::from_z(v);
+    }
   }
 }
 

@@ -522,7 +522,7 @@ void Session::tensor_links(DslashArgs& A, int prec, int tc) {
 Blas& Session::blas() {
   if (!blas_) {
     const int max_blocks = 1024;
-    double* p = static_cast<double*>(partials_.ensure((size_t)max_blocks * QCU_MAX_RHS * 2 * sizeof(double)));
+    double* p = static_cast<double*>(partials_.ensure((size_t)max_blocks * QCU_MAX_RHS * 4 * sizeof(double)));
     blas_.reset(new Blas(p, max_blocks));
   }
   return *blas_;

@@ -5,7 +5,7 @@
 //
 // Schur system on the even sites, per RHS r with its own kappa_r:
 //   Mhat_r = 1 - kappa_r^2 D_eo D_oe,   bhat_r = b_e + kappa_r D_eo b_o,
-//   x_o    = b_o + kappa_r D_oe x_e,
+//   x_o    = b_o + kappa_r D_oe x_e,    bhat_r - Mhat_r x_e = (b_e - x_e) + kappa_r D_eo x_o,
 // and Mhat^dag = 1 - kappa^2 D_eo^- D_oe^- (the dagger flag f = -1), because
 // D^dag = gamma5 D gamma5 is the hop with f = -1.  With x_o reconstructed
 // that way, |b - M x| over the full lattice equals |bhat - Mhat x_e|.
@@ -43,18 +43,26 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <type_traits>
 
 #include "solver.h"
 
 namespace qcu {
 namespace {
 
-__global__ void cg_alpha_kernel(SolverScalars S, int nrhs) {
-  const int r = threadIdx.x;
+// The per-RHS scalar kernels sum the block partials of the reduction before
+// them (one warp per RHS, 4 per block) and its lane 0 updates the slot.
+constexpr int kScalarThreads = 128;
+__device__ __forceinline__ int scalar_rhs() { return blockIdx.x * (kScalarThreads / 32) + (threadIdx.x >> 5); }
+
+// alpha = |r|^2 / |q|^2
+__global__ void cg_alpha_kernel(SolverScalars S, int nrhs, Partials P) {
+  const int r = scalar_rhs(), lane = threadIdx.x & 31;
   if (r >= nrhs) return;
+  const double q = sum_partials(P.norm, P.blocks, nrhs, r, lane);
+  if (lane) return;
   double a = 0.0;
   if (S.active[r]) {
-    const double q = S.qq[r];
     if (q > 0.0 && isfinite(q)) {
       a = S.rr[r] / q;
     } else {
@@ -63,40 +71,43 @@ __global__ void cg_alpha_kernel(SolverScalars S, int nrhs) {
     }
   }
   S.alpha[r] = make_double2(a, 0.0);
-  S.nalpha[r] = make_double2(-a, 0.0);
 }
 
-// beta, convergence and reliable-update test per slot; one block of >= nrhs threads
-__global__ void cg_beta_kernel(SolverScalars S, int nrhs, double delta2) {
-  const int r = threadIdx.x;
-  int act = 0;
-  if (r < nrhs) {
-    double b = 0.0;
-    if (S.active[r]) {
-      b = S.rr_new[r] / S.rr[r];
-      S.rr[r] = S.rr_new[r];
-      const double ss = S.ss[r];
-      if (!(ss > S.stop2[r])) {  // reached the tolerance (or NaN): verify in FP64
-        S.active[r] = 0;
-        S.upd[r] = 1;
-      } else if (ss < delta2 * S.maxss[r]) {
-        S.upd[r] = 1;
-      }
-      act = S.active[r];
-    }
-    S.beta[r] = make_double2(b, 0.0);
+// the slot's residual ss: tolerance reached (or NaN) -> verify in FP64; dropped by delta -> reliable update
+__device__ __forceinline__ void test_residual(const SolverScalars& S, int r, double ss, double delta2) {
+  if (!(ss > S.stop2[r])) {
+    S.active[r] = 0;
+    S.upd[r] = 1;
+  } else if (ss < delta2 * S.maxss[r]) {
+    S.upd[r] = 1;
   }
-  const int n_act = __syncthreads_count(act);
-  if (threadIdx.x == 0) S.status[0] = n_act;
+}
+
+// beta, convergence and reliable-update test per slot
+__global__ void cg_beta_kernel(SolverScalars S, int nrhs, Partials P, double delta2) {
+  const int r = scalar_rhs(), lane = threadIdx.x & 31;
+  if (r >= nrhs) return;
+  const double ss = sum_partials(P.norm, P.blocks, nrhs, r, lane);
+  const double rr = sum_partials(P.norm2, P.blocks, nrhs, r, lane);
+  if (lane) return;
+  double b = 0.0;
+  if (S.active[r]) {
+    b = rr / S.rr[r];
+    S.rr[r] = rr;
+    test_residual(S, r, ss, delta2);
+  }
+  S.beta[r] = make_double2(b, 0.0);
 }
 
 // BiCGStab: alpha = rho / <r0, v>
-__global__ void bicg_alpha_kernel(SolverScalars S, int nrhs) {
-  const int r = threadIdx.x;
+__global__ void bicg_alpha_kernel(SolverScalars S, int nrhs, Partials P) {
+  const int r = scalar_rhs(), lane = threadIdx.x & 31;
   if (r >= nrhs) return;
+  const double2 d = sum_partials(P.dot, P.blocks, nrhs, r, lane);
+  if (lane) return;
   double2 a = make_double2(0.0, 0.0);
   if (S.active[r]) {
-    const double2 d = S.tmp1[r], rho = S.rho[r];
+    const double2 rho = S.rho[r];
     const double den = d.x * d.x + d.y * d.y;
     if (den > 0.0 && isfinite(den)) {
       a = make_double2((rho.x * d.x + rho.y * d.y) / den, (rho.y * d.x - rho.x * d.y) / den);
@@ -109,102 +120,81 @@ __global__ void bicg_alpha_kernel(SolverScalars S, int nrhs) {
   S.nalpha[r] = make_double2(-a.x, -a.y);
 }
 
-// omega = <t, s> / <t, t>   (tmp1 = <t, s>, qq = |t|^2)
-__global__ void bicg_omega_kernel(SolverScalars S, int nrhs) {
-  const int r = threadIdx.x;
+// omega = <t, s> / <t, t>
+__global__ void bicg_omega_kernel(SolverScalars S, int nrhs, Partials P) {
+  const int r = scalar_rhs(), lane = threadIdx.x & 31;
   if (r >= nrhs) return;
+  const double2 ts = sum_partials(P.dot, P.blocks, nrhs, r, lane);
+  const double tt = sum_partials(P.norm, P.blocks, nrhs, r, lane);
+  if (lane) return;
   double2 w = make_double2(0.0, 0.0);
   if (S.active[r]) {
-    const double tt = S.qq[r];
     if (tt > 0.0 && isfinite(tt)) {
-      w = make_double2(S.tmp1[r].x / tt, S.tmp1[r].y / tt);
+      w = make_double2(ts.x / tt, ts.y / tt);
     } else {
       S.active[r] = 0;
       S.upd[r] = 1;
     }
   }
   S.omega[r] = w;
-  S.nomega[r] = make_double2(-w.x, -w.y);
 }
 
-// beta = (rho_new / rho) (alpha / omega); tmp2 = rho_new; test |r|
-__global__ void bicg_beta_kernel(SolverScalars S, int nrhs, double delta2) {
-  const int r = threadIdx.x;
-  int act = 0;
-  if (r < nrhs) {
-    double2 b = make_double2(0.0, 0.0), nbo = make_double2(0.0, 0.0);
-    if (S.active[r]) {
-      const double2 rn = S.tmp2[r], ro = S.rho[r], a = S.alpha[r], w = S.omega[r];
-      const double d1 = ro.x * ro.x + ro.y * ro.y, d2 = w.x * w.x + w.y * w.y;
-      if (d1 > 0.0 && d2 > 0.0 && isfinite(d1) && isfinite(d2)) {
-        const double2 q1 = make_double2((rn.x * ro.x + rn.y * ro.y) / d1, (rn.y * ro.x - rn.x * ro.y) / d1);
-        const double2 q2 = make_double2((a.x * w.x + a.y * w.y) / d2, (a.y * w.x - a.x * w.y) / d2);
-        b = make_double2(q1.x * q2.x - q1.y * q2.y, q1.x * q2.y + q1.y * q2.x);
-        nbo = make_double2(-(b.x * w.x - b.y * w.y), -(b.x * w.y + b.y * w.x));
-        S.rho[r] = rn;
-      } else {
-        S.active[r] = 0;
-        S.upd[r] = 1;
-      }
-      const double ss = S.ss[r];
-      if (S.active[r]) {
-        if (!(ss > S.stop2[r])) {
-          S.active[r] = 0;
-          S.upd[r] = 1;
-        } else if (ss < delta2 * S.maxss[r]) {
-          S.upd[r] = 1;
-        }
-      }
-      act = S.active[r];
-    }
-    S.beta[r] = b;
-    S.nbo[r] = nbo;
-  }
-  const int n_act = __syncthreads_count(act);
-  if (threadIdx.x == 0) S.status[0] = n_act;
-}
-
-// masked-operation coefficients from sel: cm = sel, ck = 1 - sel, cn = -sel
-__global__ void select_coeffs_kernel(SolverScalars S, int nrhs) {
-  const int r = threadIdx.x;
+// beta = (rho_new / rho) (alpha / omega), rho_new = <r0, r>; test |r|
+__global__ void bicg_beta_kernel(SolverScalars S, int nrhs, Partials P, double delta2) {
+  const int r = scalar_rhs(), lane = threadIdx.x & 31;
   if (r >= nrhs) return;
-  const double m = S.sel[r] ? 1.0 : 0.0;
-  S.cm[r] = make_double2(m, 0.0);
-  S.ck[r] = make_double2(1.0 - m, 0.0);
-  S.cn[r] = make_double2(-m, 0.0);
-  S.zero[r] = make_double2(0.0, 0.0);
-  S.one[r] = make_double2(1.0, 0.0);
+  const double2 rn = sum_partials(P.dot, P.blocks, nrhs, r, lane);
+  const double ss = sum_partials(P.norm, P.blocks, nrhs, r, lane);
+  if (lane) return;
+  double2 b = make_double2(0.0, 0.0), nbo = make_double2(0.0, 0.0);
+  if (S.active[r]) {
+    const double2 ro = S.rho[r], a = S.alpha[r], w = S.omega[r];
+    const double d1 = ro.x * ro.x + ro.y * ro.y, d2 = w.x * w.x + w.y * w.y;
+    if (d1 > 0.0 && d2 > 0.0 && isfinite(d1) && isfinite(d2)) {
+      const double2 q1 = make_double2((rn.x * ro.x + rn.y * ro.y) / d1, (rn.y * ro.x - rn.x * ro.y) / d1);
+      const double2 q2 = make_double2((a.x * w.x + a.y * w.y) / d2, (a.y * w.x - a.x * w.y) / d2);
+      b = make_double2(q1.x * q2.x - q1.y * q2.y, q1.x * q2.y + q1.y * q2.x);
+      nbo = make_double2(-(b.x * w.x - b.y * w.y), -(b.x * w.y + b.y * w.x));
+      S.rho[r] = rn;
+    } else {
+      S.active[r] = 0;
+      S.upd[r] = 1;
+    }
+    if (S.active[r]) test_residual(S, r, ss, delta2);
+  }
+  S.beta[r] = b;
+  S.nbo[r] = nbo;
 }
 
-// after a (re)start of the selected slots: rr, maxss and ss from the fresh
-// residuals; the CG invariant <r, p> = |r|^2 restored by p += c r with
+// after a (re)start of the selected slots: rr, maxss from the fresh residuals;
+// the CG invariant <r, p> = |r|^2 restored by p += c r with
 // c = 1 - <r, p> / |r|^2 (fresh slots have p = 0, so p becomes r).  The
 // update p += c r runs over every slot, so c = 0 for the slots not restarted.
-__global__ void restart_kernel(SolverScalars S, int nrhs) {
-  const int r = threadIdx.x;
+__global__ void restart_kernel(SolverScalars S, int nrhs, Partials P) {
+  const int r = scalar_rhs(), lane = threadIdx.x & 31;
   if (r >= nrhs) return;
-  if (!S.sel[r]) {
-    S.tmp2[r] = make_double2(0.0, 0.0);
-    return;
-  }
-  S.rr[r] = S.rr_new[r];
-  S.maxss[r] = S.ss_true[r];
-  S.ss[r] = S.ss_true[r];
-  S.upd[r] = 0;
-  const double rr = S.rr_new[r];
+  const double rr = sum_partials(P.norm, P.blocks, nrhs, r, lane);
+  const double2 rp = sum_partials(P.dot, P.blocks, nrhs, r, lane);
+  if (lane) return;
   double2 c = make_double2(0.0, 0.0);
-  if (rr > 0.0 && isfinite(rr)) c = make_double2(1.0 - S.tmp1[r].x / rr, -S.tmp1[r].y / rr);
+  if (S.sel[r]) {
+    S.rr[r] = rr;
+    S.maxss[r] = S.ss_true[r];
+    S.upd[r] = 0;
+    if (rr > 0.0 && isfinite(rr)) c = make_double2(1.0 - rp.x / rr, -rp.y / rr);
+  }
   S.tmp2[r] = c;
 }
 
-// BiCGStab restart of the selected slots: rho = <r0, r> (tmp1)
-__global__ void bicg_restart_kernel(SolverScalars S, int nrhs) {
-  const int r = threadIdx.x;
-  if (r >= nrhs || !S.sel[r]) return;
+// BiCGStab restart of the selected slots: r0 = r, so rho = <r0, r> = |r|^2
+__global__ void bicg_restart_kernel(SolverScalars S, int nrhs, Partials P) {
+  const int r = scalar_rhs(), lane = threadIdx.x & 31;
+  if (r >= nrhs) return;
+  const double rr = sum_partials(P.norm, P.blocks, nrhs, r, lane);
+  if (lane || !S.sel[r]) return;
   S.maxss[r] = S.ss_true[r];
-  S.ss[r] = S.ss_true[r];
   S.upd[r] = 0;
-  S.rho[r] = S.tmp1[r];
+  S.rho[r] = make_double2(rr, 0.0);
 }
 
 }  // namespace
@@ -218,6 +208,7 @@ FieldRef SlotEngine::ref(const FieldView& f) const {
   return r;
 }
 
+// (an upper bound by two FP64 fields; admission keeps it, so a budget admits what it always did)
 size_t SlotEngine::bytes_needed(const Session& s, int capacity, int inner_prec) {
   const int kp = inner_prec == PREC_DOUBLE ? PREC_DOUBLE : PREC_SINGLE;
   size_t b = 8 * s.field_bytes(PREC_DOUBLE, capacity) + 7 * s.field_bytes(kp, capacity);
@@ -245,19 +236,17 @@ SlotEngine::SlotEngine(Session& s, int capacity, const SolveRequest& q, const st
   const std::string t = tag + ".";
   be_ = s.alloc_field(t + "be", PREC_DOUBLE, n_);
   bo_ = s.alloc_field(t + "bo", PREC_DOUBLE, n_);
-  bh_ = s.alloc_field(t + "bh", PREC_DOUBLE, n_);
   xh_ = s.alloc_field(t + "xh", PREC_DOUBLE, n_);
   xo_ = s.alloc_field(t + "xo", PREC_DOUBLE, n_);
   sh_ = s.alloc_field(t + "sh", PREC_DOUBLE, n_);
-  th_ = s.alloc_field(t + "th", PREC_DOUBLE, n_);
-  tmp64_ = s.alloc_field(t + "tmp64", PREC_DOUBLE, n_);
+  dh_ = s.alloc_field(t + "dh", PREC_DOUBLE, n_);
   xl_ = s.alloc_field(t + "xl", kp_, n_);
   sl_ = s.alloc_field(t + "sl", kp_, n_);
   rl_ = s.alloc_field(t + "rl", kp_, n_);
   pl_ = s.alloc_field(t + "pl", kp_, n_);
   ql_ = s.alloc_field(t + "ql", kp_, n_);
   wl_ = s.alloc_field(t + "wl", kp_, n_);
-  r0l_ = s.alloc_field(t + "r0l", kp_, n_);
+  if (q.solver == 1) r0l_ = s.alloc_field(t + "r0l", kp_, n_);
   if (op_ != kp_) {
     pop_ = s.alloc_field(t + "pop", op_, n_);
     qop_ = s.alloc_field(t + "qop", op_, n_);
@@ -278,50 +267,25 @@ SlotEngine::SlotEngine(Session& s, int capacity, const SolveRequest& q, const st
   }
   // per-slot device scalars
   const int R = QCU_MAX_RHS;
-  char* d = static_cast<char*>(s.ws.get(t + "scalars", (size_t)R * 64 * sizeof(double) + 4096));
-  double* dd = reinterpret_cast<double*>(d);
-  S_.rr = dd;
-  S_.rr_new = dd + R;
-  S_.qq = dd + 2 * R;
-  S_.ss = dd + 3 * R;
-  S_.ss_true = dd + 4 * R;
-  S_.maxss = dd + 5 * R;
-  S_.stop2 = dd + 6 * R;
-  S_.bb = dd + 7 * R;
-  S_.bo2 = dd + 8 * R;
-  S_.kap_d = dd + 9 * R;
-  S_.nk2_d = dd + 10 * R;
-  double2* c = reinterpret_cast<double2*>(dd + 11 * R);
-  S_.alpha = c;
-  S_.nalpha = c + R;
-  S_.beta = c + 2 * R;
-  S_.omega = c + 3 * R;
-  S_.nomega = c + 4 * R;
-  S_.rho = c + 5 * R;
-  S_.tmp1 = c + 6 * R;
-  S_.tmp2 = c + 7 * R;
-  S_.nbo = c + 8 * R;
-  S_.cm = c + 9 * R;
-  S_.ck = c + 10 * R;
-  S_.cn = c + 11 * R;
-  S_.zero = c + 12 * R;
-  S_.one = c + 13 * R;
-  float* ff = reinterpret_cast<float*>(c + 14 * R);  // at dd + 39R
-  S_.nk2_f = ff;
-  int* ip = reinterpret_cast<int*>(ff + R);
-  S_.active = ip;
-  S_.upd = ip + R;
-  S_.sel = ip + 2 * R;
-  S_.status = ip + 3 * R;
+  const size_t scalar_bytes = (size_t)R * (8 * sizeof(double) + 8 * sizeof(double2) + sizeof(float) + 3 * sizeof(int));
+  char* d = static_cast<char*>(s.ws.get(t + "scalars", scalar_bytes));
+  auto take = [&](auto*& p) {
+    p = reinterpret_cast<std::remove_reference_t<decltype(p)>>(d);
+    d += R * sizeof(*p);
+  };
+  char* const base = d;
+  for (double2** p : {&S_.alpha, &S_.nalpha, &S_.beta, &S_.omega, &S_.rho, &S_.tmp2, &S_.nbo, &S_.one}) take(*p);
+  for (double** p : {&S_.rr, &S_.ss_true, &S_.maxss, &S_.stop2, &S_.bb, &S_.bo2, &S_.kap_d, &S_.nk2_d}) take(*p);
+  take(S_.nk2_f);
+  for (int** p : {&S_.active, &S_.upd, &S_.sel}) take(*p);
   host_.assign(n_, SlotState{});
-  QCU_CHECK_CUDA(cudaMemsetAsync(d, 0, (size_t)R * 64 * sizeof(double) + 4096, st_));
-  // every field starts at zero: masked slots never meet uninitialised memory
-  for (FieldView* f : {&be_, &bo_, &bh_, &xh_, &xo_, &sh_, &th_, &tmp64_, &xl_, &sl_, &rl_, &pl_, &ql_, &wl_, &r0l_,
-                       &pop_, &qop_, &wop_, &tmpop_, &tmp64b_, &tmpopb_}) {
-    if (!f->data) continue;
-    QCU_CHECK_CUDA(cudaMemsetAsync(f->data, 0, s.field_bytes(f->prec, n_), st_));
-    if (f->norm) QCU_CHECK_CUDA(cudaMemsetAsync(f->norm, 0, s.norm_bytes(f->prec, n_), st_));
-  }
+  // The fields stay as they are: a slot's fields are written (moves, never
+  // products with a zero coefficient) when it is admitted, and no operation
+  // mixes slots.
+  QCU_CHECK_CUDA(cudaMemsetAsync(base, 0, scalar_bytes, st_));
+  std::vector<double> one(2 * n_, 0.0);
+  for (int r = 0; r < n_; r++) one[2 * r] = 1.0;
+  QCU_CHECK_CUDA(cudaMemcpyAsync(S_.one, one.data(), sizeof(double2) * n_, cudaMemcpyHostToDevice, st_));
   s.blas();  // BLAS scratch, before any graph capture
   QCU_CHECK_CUDA(cudaStreamSynchronize(st_));
 }
@@ -347,8 +311,6 @@ void SlotEngine::upload_sel(const std::vector<int>& slots) {
   std::vector<int> m(n_, 0);
   for (int r : slots) m[r] = 1;
   QCU_CHECK_CUDA(cudaMemcpyAsync(S_.sel, m.data(), sizeof(int) * n_, cudaMemcpyHostToDevice, st_));
-  select_coeffs_kernel<<<1, QCU_MAX_RHS, 0, st_>>>(S_, n_);
-  QCU_CHECK_CUDA(cudaGetLastError());
   // the upload reads host memory asynchronously: keep it alive until done
   QCU_CHECK_CUDA(cudaStreamSynchronize(st_));
 }
@@ -408,34 +370,30 @@ void SlotEngine::cg_iteration() {
     convert_field(op_, qop_.data, qop_.norm, kp_, ql_.data, nullptr, s_.geo.vh, 4 * s_.N, n_, st_, S_.active);
     convert_field(op_, wop_.data, wop_.norm, kp_, wl_.data, nullptr, s_.geo.vh, 4 * s_.N, n_, st_, S_.active);
   }
-  B.norm2(ref(ql_), S_.qq, st_, false);
-  cg_alpha_kernel<<<1, QCU_MAX_RHS, 0, st_>>>(S_, n_);
-  B.axpby(S_.alpha, ref(pl_), nullptr, ref(xl_), st_);                  // x += a p
-  B.axpby_norm(S_.nalpha, ref(ql_), nullptr, ref(sl_), S_.ss, st_);      // s -= a q
-  B.axpby_norm(S_.nalpha, ref(wl_), nullptr, ref(rl_), S_.rr_new, st_);  // r -= a w
-  cg_beta_kernel<<<1, QCU_MAX_RHS, 0, st_>>>(S_, n_, delta2_);
-  B.axpby(nullptr, ref(rl_), S_.beta, ref(pl_), st_);  // p = r + b p
+  const Partials qq = B.norm2_partials(ref(ql_), st_);
+  cg_alpha_kernel<<<scalar_blocks(), kScalarThreads, 0, st_>>>(S_, n_, qq);
+  // s -= a q, r -= a w with their norms; then x += a p, p = r + b p in one pass over p
+  const Partials sr = B.cg_update(S_.alpha, ref(ql_), ref(sl_), ref(wl_), ref(rl_), st_);
+  cg_beta_kernel<<<scalar_blocks(), kScalarThreads, 0, st_>>>(S_, n_, sr, delta2_);
+  B.cg_direction(S_.alpha, S_.beta, ref(rl_), ref(pl_), ref(xl_), st_);
 }
 
 void SlotEngine::bicg_iteration() {
   Blas& B = s_.blas();
   op_apply(ql_, pl_, 0, S_.active);  // v = Mhat p
-  B.cdot(ref(r0l_), ref(ql_), S_.tmp1, st_);
-  bicg_alpha_kernel<<<1, QCU_MAX_RHS, 0, st_>>>(S_, n_);
+  const Partials rv = B.dot_partials(ref(r0l_), ref(ql_), st_);
+  bicg_alpha_kernel<<<scalar_blocks(), kScalarThreads, 0, st_>>>(S_, n_, rv);
   B.axpby(S_.nalpha, ref(ql_), nullptr, ref(sl_), st_);  // s = r - alpha v (sl holds r)
   op_apply(wl_, sl_, 0, S_.active);                       // t = Mhat s
-  B.cdot(ref(wl_), ref(sl_), S_.tmp1, st_);
-  B.norm2(ref(wl_), S_.qq, st_, false);
-  bicg_omega_kernel<<<1, QCU_MAX_RHS, 0, st_>>>(S_, n_);
-  B.axpbypcz(S_.alpha, ref(pl_), S_.omega, ref(sl_), nullptr, ref(xl_), st_);  // x += alpha p + omega s
-  B.axpby_norm(S_.nomega, ref(wl_), nullptr, ref(sl_), S_.ss, st_);            // r = s - omega t
-  B.cdot(ref(r0l_), ref(sl_), S_.tmp2, st_);
-  bicg_beta_kernel<<<1, QCU_MAX_RHS, 0, st_>>>(S_, n_, delta2_);
+  const Partials ts = B.dot_norm(ref(wl_), ref(sl_), st_);
+  bicg_omega_kernel<<<scalar_blocks(), kScalarThreads, 0, st_>>>(S_, n_, ts);
+  // x += alpha p + omega s, r = s - omega t, with |r|^2 and <r0, r>
+  const Partials rr = B.bicg_update(S_.alpha, S_.omega, ref(pl_), ref(sl_), ref(wl_), ref(r0l_), ref(xl_), st_);
+  bicg_beta_kernel<<<scalar_blocks(), kScalarThreads, 0, st_>>>(S_, n_, rr, delta2_);
   B.axpbypcz(S_.one, ref(sl_), S_.nbo, ref(ql_), S_.beta, ref(pl_), st_);  // p = r + beta p - beta omega v
 }
 
 void SlotEngine::run_chunk(int k) {
-  QCU_CHECK_CUDA(cudaMemsetAsync(S_.status, 0, sizeof(int) * 4, st_));
   if (q_.use_graph && k == chunk_) {
     if (!graph_exec_) {
       // kernel shapes are tuned in the first (eager) chunk; later chunks replay a graph
@@ -464,29 +422,43 @@ void SlotEngine::run_chunk(int k) {
   }
 }
 
+// out = M_oo^-1 (b_o + kappa D_oe x_e): x_o of the slots in sel
+void SlotEngine::odd_solution() {
+  if (cl_) {
+    s_.hop(tmp64b_, xh_, bo_, 1, 0, 0.0, 1.0, S_.sel, nullptr, S_.kap_d);
+    s_.clover_apply(xo_, tmp64b_, FieldView{}, 1, true, 1.0, 0.0, S_.sel);
+  } else {
+    s_.hop(xo_, xh_, bo_, 1, 0, 0.0, 1.0, S_.sel, nullptr, S_.kap_d);
+  }
+}
+
 // (Re)start the slots in `slots`: fold x_lo into x, recompute the true
-// residual s = bhat - Mhat x in FP64, decide convergence, and restart the
-// Krylov recurrence of the slots that go on.  `fresh` slots start from x = 0
-// with p = r.
+// residual in FP64, decide convergence, and restart the Krylov recurrence of
+// the slots that go on.  With x_o = b_o + kappa D_oe x_e the residual is
+//   s = bhat - Mhat x_e = (b_e - x_e) + kappa D_eo x_o
+// (clover: x_o = A_oo^-1 (..), s = (b_e - A_ee x_e) + kappa D_eo x_o), so a
+// reliable update also leaves the odd half of the solution, and bhat itself
+// is never formed.  `fresh` slots start from x = 0 with p = r.
 void SlotEngine::restart(const std::vector<int>& slots, bool fresh) {
   if (slots.empty()) return;
   Blas& B = s_.blas();
   upload_sel(slots);
-  if (!fresh) B.axpby(S_.cm, ref(xl_), nullptr, ref(xh_), st_);  // x += x_lo
-  B.axpby(S_.zero, ref(xl_), S_.ck, ref(xl_), st_);              // x_lo = 0
   if (fresh) {
-    B.axpby(S_.zero, ref(xh_), S_.ck, ref(xh_), st_);  // x = 0
-    B.axpby(S_.zero, ref(pl_), S_.ck, ref(pl_), st_);  // p = 0
-  }
-  // s = bhat - Mhat x  (only the selected slots are computed); fresh slots
-  // start from x = 0, so their true residual is bhat itself
-  B.axpby(S_.cm, ref(bh_), S_.ck, ref(sh_), st_);
-  if (fresh) {
-    B.norm2(ref(sh_), S_.ss_true, st_);
+    // s = b_e + kappa D_eo b_o (clover: b_e + kappa D_eo A_oo^-1 b_o)
+    for (const FieldView* f : {&xl_, &xh_, &pl_}) B.select_copy(S_.sel, FieldRef{}, ref(*f), FieldRef{}, st_);
+    FieldView odd = bo_;
+    if (cl_) {
+      s_.clover_apply(tmp64b_, bo_, FieldView{}, 1, true, 1.0, 0.0, S_.sel);
+      odd = tmp64b_;
+    }
+    s_.hop(sh_, odd, be_, 0, 0, 0.0, 1.0, S_.sel, nullptr, S_.kap_d);
   } else {
-    apply_mhat(th_, xh_, tmp64_, tmp64b_, 0, S_.sel);
-    B.axpby_norm(S_.cn, ref(th_), nullptr, ref(sh_), S_.ss_true, st_);
+    B.fold(S_.sel, ref(xl_), ref(xh_), ref(be_), cl_ ? FieldRef{} : ref(dh_), st_);
+    odd_solution();
+    if (cl_) s_.clover_apply(dh_, xh_, be_, 0, false, -1.0, 1.0, S_.sel);
+    s_.hop(sh_, xo_, dh_, 0, 0, 0.0, 1.0, S_.sel, nullptr, S_.kap_d);
   }
+  B.residual(S_.sel, ref(sh_), ref(sl_), S_.ss_true, st_);  // |s|^2, and s_lo = s
   std::vector<double> ss(n_);
   QCU_CHECK_CUDA(cudaMemcpyAsync(ss.data(), S_.ss_true, sizeof(double) * n_, cudaMemcpyDeviceToHost, st_));
   std::vector<int> act(n_);
@@ -519,19 +491,16 @@ void SlotEngine::restart(const std::vector<int>& slots, bool fresh) {
     QCU_CHECK_CUDA(cudaStreamSynchronize(st_));
     return;
   }
-  upload_sel(go_on);
-  B.axpby(S_.cm, ref(sh_), S_.ck, ref(sl_), st_);  // s_lo = s
+  if (go_on.size() != slots.size()) upload_sel(go_on);
   if (q_.solver == 0) {
     op_apply(rl_, sl_, 1, S_.sel);  // r = Mhat^dag s
-    B.norm2(ref(rl_), S_.rr_new, st_, false);
-    B.cdot(ref(rl_), ref(pl_), S_.tmp1, st_);
-    restart_kernel<<<1, QCU_MAX_RHS, 0, st_>>>(S_, n_);
+    const Partials rp = B.dot_norm(ref(rl_), ref(pl_), st_);
+    restart_kernel<<<scalar_blocks(), kScalarThreads, 0, st_>>>(S_, n_, rp);
     B.axpby(S_.tmp2, ref(rl_), nullptr, ref(pl_), st_);  // p += c r
   } else {
-    B.axpby(S_.cm, ref(sl_), S_.ck, ref(r0l_), st_);  // shadow residual r0 = r
-    B.axpby(S_.cm, ref(sl_), S_.ck, ref(pl_), st_);   // p = r
-    B.cdot(ref(r0l_), ref(sl_), S_.tmp1, st_);
-    bicg_restart_kernel<<<1, QCU_MAX_RHS, 0, st_>>>(S_, n_);
+    B.select_copy(S_.sel, ref(sl_), ref(r0l_), ref(pl_), st_);  // shadow residual r0 = r, p = r
+    const Partials rr = B.norm2_partials(ref(sl_), st_);
+    bicg_restart_kernel<<<scalar_blocks(), kScalarThreads, 0, st_>>>(S_, n_, rr);
   }
   QCU_CHECK_CUDA(cudaGetLastError());
   QCU_CHECK_CUDA(cudaStreamSynchronize(st_));
@@ -576,14 +545,6 @@ void SlotEngine::admit(const std::vector<int>& slots, void* const* b, const doub
     stop2[r] = h.stop2;
   }
   QCU_CHECK_CUDA(cudaMemcpyAsync(S_.stop2, stop2.data(), sizeof(double) * n_, cudaMemcpyHostToDevice, st_));
-  // bhat = b_e + kappa_r D_eo b_o (clover: b_e + kappa_r D_eo A_oo^-1 b_o) for the new slots
-  upload_sel(slots);
-  if (cl_) {
-    s_.clover_apply(tmp64b_, bo_, FieldView{}, 1, true, 1.0, 0.0, S_.sel);
-    s_.hop(bh_, tmp64b_, be_, 0, 0, 0.0, 1.0, S_.sel, nullptr, S_.kap_d);
-  } else {
-    s_.hop(bh_, bo_, be_, 0, 0, 0.0, 1.0, S_.sel, nullptr, S_.kap_d);
-  }
   restart(slots, true);
 }
 
@@ -625,13 +586,13 @@ void SlotEngine::retire(const std::vector<int>& slots, void* const* x, int src_m
                 "retire: slot has not finished");
     px.p[r] = x[i];
   }
-  upload_sel(slots);
-  // x_o = b_o + kappa_r D_oe x_e (clover: A_oo^-1 of it)
-  if (cl_) {
-    s_.hop(tmp64b_, xh_, bo_, 1, 0, 0.0, 1.0, S_.sel, nullptr, S_.kap_d);
-    s_.clover_apply(xo_, tmp64b_, FieldView{}, 1, true, 1.0, 0.0, S_.sel);
-  } else {
-    s_.hop(xo_, xh_, bo_, 1, 0, 0.0, 1.0, S_.sel, nullptr, S_.kap_d);
+  // x_o is the last reliable update's; a slot that finished without one has x = 0, so x_o is still to be formed
+  std::vector<int> untouched;
+  for (int r : slots)
+    if (host_[r].updates == 0) untouched.push_back(r);
+  if (!untouched.empty()) {
+    upload_sel(untouched);
+    odd_solution();
   }
   unpack_fermions(PREC_DOUBLE, s_.N, px, src_mode, 0, xh_.data, nullptr, s_.geo, n_, st_);
   unpack_fermions(PREC_DOUBLE, s_.N, px, src_mode, 1, xo_.data, nullptr, s_.geo, n_, st_);

@@ -12,14 +12,13 @@ namespace qcu {
 
 // per-slot device scalars (arrays of QCU_MAX_RHS entries)
 struct SolverScalars {
-  double *rr, *rr_new, *qq, *ss, *ss_true, *maxss, *stop2, *bb, *bo2, *kap_d, *nk2_d;
-  double2 *alpha, *nalpha, *beta, *omega, *nomega, *rho, *tmp1, *tmp2, *nbo;
-  double2 *cm, *ck, *cn, *zero, *one;  // masked-operation coefficients from sel
-  float* nk2_f;                        // -kappa^2 for FP32 arithmetic
-  int* active;                         // slot iterates
-  int* upd;                            // slot asks for a reliable update
-  int* sel;                            // slots selected for a masked operation
-  int* status;                         // [0] active count of the last chunk
+  double *rr, *ss_true, *maxss, *stop2, *bb, *bo2, *kap_d, *nk2_d;
+  double2 *alpha, *nalpha, *beta, *omega, *rho, *tmp2, *nbo;
+  double2* one;
+  float* nk2_f;  // -kappa^2 for FP32 arithmetic
+  int* active;   // slot iterates
+  int* upd;      // slot asks for a reliable update
+  int* sel;      // slots selected for a masked operation
 };
 
 struct SlotState {
@@ -68,6 +67,8 @@ class SlotEngine {
   void bicg_iteration();
   void run_chunk(int k);
   void restart(const std::vector<int>& slots, bool fresh);
+  void odd_solution();
+  int scalar_blocks() const { return (n_ + 3) / 4; }  // one warp per RHS, four per block
 
   Session& s_;
   int n_;
@@ -75,7 +76,7 @@ class SlotEngine {
   int kp_, op_;
   double delta2_;
   cudaStream_t st_;
-  FieldView be_, bo_, bh_, xh_, xo_, sh_, th_, tmp64_;
+  FieldView be_, bo_, xh_, xo_, sh_, dh_;  // dh: b_e - x_e (clover: b_e - A_ee x_e)
   FieldView xl_, sl_, rl_, pl_, ql_, wl_, r0l_;
   FieldView pop_, qop_, wop_, tmpop_;
   FieldView tmp64b_, tmpopb_;  // second temporaries of the clover operator
