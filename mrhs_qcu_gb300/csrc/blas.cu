@@ -47,31 +47,39 @@ __device__ __forceinline__ double2 ld(const float2* p) { return Store<PREC_SINGL
 __device__ __forceinline__ void st(double2* p, double2 v) { *p = v; }
 __device__ __forceinline__ void st(float2* p, double2 v) { *p = Store<PREC_SINGLE>::from_z(v); }
 
-// FP64 sum of FP32 products in groups.  One conversion and FP64 addition per
-// product is bound by the FP64 pipe (2 lanes a cycle and SM, and the
-// conversion issues there too): the norm of 24^3x48 SU(3) nrhs 12 FP32 took
-// 195 us against 56 us of HBM time.  So a few products are added in FP32 with
-// their rounding errors kept (Knuth's TwoSum), and two values per group go to
-// FP64.  Products that would take the group out of FP32's range, or are not
-// finite, go to FP64 themselves.
+// FP64 sum of FP32 products in groups of four.  One conversion and FP64
+// addition per product is bound by the FP64 pipe (2 lanes a cycle and SM, and
+// the conversion issues there too): the norm of 24^3x48 SU(3) nrhs 12 FP32
+// took 195 us against 56 us of HBM time.  So the products of a group are added in
+// FP32 with their rounding errors kept (Knuth's TwoSum), and two values go to
+// FP64.  A group that leaves FP32's range, or is not finite, is added product
+// by product (a call: as predicated instructions it would hold the FP64 pipe).
+constexpr int kGroup = 4;
+static __device__ __noinline__ double add_plainly(double acc, float a, float b, float c, float d) {
+  acc += (double)a;
+  acc += (double)b;
+  acc += (double)c;
+  return acc + (double)d;
+}
 struct GroupSum {
-  float hi = 0.f, lo = 0.f;
-  __device__ __forceinline__ void add(double& acc, float p) {
-    const float s = __fadd_rn(hi, p), b = __fsub_rn(s, hi);
-    if (fabsf(s) <= 3.402823466e38f) {
-      lo = __fadd_rn(lo, __fadd_rn(__fsub_rn(hi, __fsub_rn(s, b)), __fsub_rn(p, b)));
+  float p[kGroup];
+  __device__ __forceinline__ void set(int u, float v) { p[u] = v; }  // u: a constant once the loops are unrolled
+  __device__ __forceinline__ void flush(double& acc) {
+    float hi = p[0], lo = 0.f;
+#pragma unroll
+    for (int u = 1; u < kGroup; u++) {
+      const float s = __fadd_rn(hi, p[u]), b = __fsub_rn(s, hi);
+      lo = __fadd_rn(lo, __fadd_rn(__fsub_rn(hi, __fsub_rn(s, b)), __fsub_rn(p[u], b)));
       hi = s;
+    }
+    if (fabsf(hi) <= 3.402823466e38f) {
+      acc += to_f64(hi);
+      acc += to_f64(lo);
     } else {
-      acc += (double)p;
+      acc = add_plainly(acc, p[0], p[1], p[2], p[3]);
     }
   }
-  __device__ __forceinline__ void flush(double& acc) {
-    acc += to_f64(hi);
-    acc += to_f64(lo);
-    hi = lo = 0.f;
-  }
 };
-constexpr int kGroup = 4;  // products per group
 // FP64 products accumulate as they are formed
 __device__ __forceinline__ void add_square(double& acc, double2 v) {
   acc = fma(v.x, v.x, acc);
@@ -88,8 +96,8 @@ template <int P>
 struct NormSum {
   double acc = 0.0;
   GroupSum g;
-  __device__ __forceinline__ void add(float2 v) { g.add(acc, fmaf(v.x, v.x, v.y * v.y)); }
-  __device__ __forceinline__ void add(double2 v) { add_square(acc, v); }
+  __device__ __forceinline__ void add(int u, float2 v) { g.set(u, fmaf(v.x, v.x, v.y * v.y)); }
+  __device__ __forceinline__ void add(int, double2 v) { add_square(acc, v); }
   __device__ __forceinline__ void flush() {
     if constexpr (P == PREC_SINGLE) g.flush(acc);
   }
@@ -98,11 +106,11 @@ template <int P>
 struct DotSum {  // conj(u) v
   double2 acc = make_double2(0.0, 0.0);
   GroupSum re, im;
-  __device__ __forceinline__ void add(float2 u, float2 v) {
-    re.add(acc.x, fmaf(u.x, v.x, u.y * v.y));
-    im.add(acc.y, fmaf(u.x, v.y, -u.y * v.x));
+  __device__ __forceinline__ void add(int k, float2 u, float2 v) {
+    re.set(k, fmaf(u.x, v.x, u.y * v.y));
+    im.set(k, fmaf(u.x, v.y, -u.y * v.x));
   }
-  __device__ __forceinline__ void add(double2 u, double2 v) { add_conj(acc, u, v); }
+  __device__ __forceinline__ void add(int, double2 u, double2 v) { add_conj(acc, u, v); }
   __device__ __forceinline__ void flush() {
     if constexpr (P == PREC_SINGLE) {
       re.flush(acc.x);
@@ -208,21 +216,28 @@ __global__ void __launch_bounds__(kMaxThreads, 1) axpby_kernel(const double2* __
       fa[i] = tof(ca[i]);
       fb[i] = tof(cb[i]);
     }
+    // U chunks loaded ahead of the stores (which the loads may not pass)
+    constexpr int U = NORM ? kGroup : 1;
     NormSum<PREC_SINGLE> sum[R];
-    for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < s.nchunks;) {
+    for (int64_t c0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c0 < s.nchunks; c0 += U * stride) {
+      float2 xs[U][R], ys[U][R];
 #pragma unroll
-      for (int u = 0; u < (NORM ? kGroup : 1); u++, c += stride) {
-        if (c >= s.nchunks) break;
-        float2 xs[R], ys[R];
-        load_chunk<R>(x, c, xs);
-        load_chunk<R>(y, c, ys);
+      for (int u = 0; u < U; u++) {
+#pragma unroll
+        for (int i = 0; i < R; i++) xs[u][i] = ys[u][i] = make_float2(0.f, 0.f);
+        if (c0 + u * stride >= s.nchunks) continue;
+        load_chunk<R>(x, c0 + u * stride, xs[u]);
+        load_chunk<R>(y, c0 + u * stride, ys[u]);
+      }
+#pragma unroll
+      for (int u = 0; u < U; u++) {
 #pragma unroll
         for (int i = 0; i < R; i++) {
-          const float2 v = cmulf(fa[i], xs[i]), w = cmulf(fb[i], ys[i]);
-          ys[i] = make_float2(v.x + w.x, v.y + w.y);
-          if (NORM) sum[i].add(ys[i]);
+          const float2 v = cmulf(fa[i], xs[u][i]), w = cmulf(fb[i], ys[u][i]);
+          ys[u][i] = make_float2(v.x + w.x, v.y + w.y);
+          if (NORM) sum[i].add(u, ys[u][i]);
         }
-        store_chunk<R>(y, c, ys);
+        if (c0 + u * stride < s.nchunks) store_chunk<R>(y, c0 + u * stride, ys[u]);
       }
       if (NORM) {
 #pragma unroll
@@ -356,7 +371,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1) reduce_kernel(const void* __re
 #pragma unroll
       for (int i = 0; i < R; i++) {
 #pragma unroll
-        for (int u = 0; u < kGroup; u++) sum[i].add(val(v[u][i]));
+        for (int u = 0; u < kGroup; u++) sum[i].add(u, val(v[u][i]));
         sum[i].flush();
       }
     }
@@ -380,7 +395,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1) reduce_kernel(const void* __re
 #pragma unroll
       for (int i = 0; i < R; i++) {
 #pragma unroll
-        for (int u = 0; u < kGroup; u++) sum[i].add(val(a[u][i]), val(b[u][i]));
+        for (int u = 0; u < kGroup; u++) sum[i].add(u, val(a[u][i]), val(b[u][i]));
         sum[i].flush();
       }
     }
@@ -409,24 +424,34 @@ __global__ void __launch_bounds__(kMaxThreads, 1) cg_update_kernel(const double2
   }
   NormSum<P> sums[R], sumr[R];
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  constexpr int U = 2;  // chunks loaded ahead of the stores
   for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < sh.nchunks;) {
 #pragma unroll
-    for (int u = 0; u < kGroup; u++, c += stride) {
-      if (c >= sh.nchunks) break;
-      E qs[R], ss[R], ws[R], rs[R];
-      load_chunk<R>(q, c, qs);
-      load_chunk<R>(s, c, ss);
-      load_chunk<R>(w, c, ws);
-      load_chunk<R>(r, c, rs);
+    for (int k = 0; k < kGroup; k += U, c += U * stride) {
+      E qs[U][R], ss[U][R], ws[U][R], rs[U][R];
 #pragma unroll
-      for (int i = 0; i < R; i++) {
-        ss[i] = add_mul(na[i], qs[i], ss[i]);
-        rs[i] = add_mul(na[i], ws[i], rs[i]);
-        sums[i].add(ss[i]);
-        sumr[i].add(rs[i]);
+      for (int u = 0; u < U; u++) {
+#pragma unroll
+        for (int i = 0; i < R; i++) qs[u][i] = ss[u][i] = ws[u][i] = rs[u][i] = E{};
+        if (c + u * stride >= sh.nchunks) continue;
+        load_chunk<R>(q, c + u * stride, qs[u]);
+        load_chunk<R>(s, c + u * stride, ss[u]);
+        load_chunk<R>(w, c + u * stride, ws[u]);
+        load_chunk<R>(r, c + u * stride, rs[u]);
       }
-      store_chunk<R>(s, c, ss);
-      store_chunk<R>(r, c, rs);
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+#pragma unroll
+        for (int i = 0; i < R; i++) {
+          ss[u][i] = add_mul(na[i], qs[u][i], ss[u][i]);
+          rs[u][i] = add_mul(na[i], ws[u][i], rs[u][i]);
+          sums[i].add(k + u, ss[u][i]);
+          sumr[i].add(k + u, rs[u][i]);
+        }
+        if (c + u * stride >= sh.nchunks) continue;
+        store_chunk<R>(s, c + u * stride, ss[u]);
+        store_chunk<R>(r, c + u * stride, rs[u]);
+      }
     }
 #pragma unroll
     for (int i = 0; i < R; i++) {
@@ -485,7 +510,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1) dot_norm_kernel(const void* __
   NormSum<P> nrm[R];
   DotSum<P> dot[R];
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  constexpr int U = kGroup / 2;  // loads of two chunks at a time
+  constexpr int U = kGroup;
   for (int64_t c0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c0 < sh.nchunks; c0 += U * stride) {
     E a[U][R], b[U][R];
 #pragma unroll
@@ -500,8 +525,8 @@ __global__ void __launch_bounds__(kMaxThreads, 1) dot_norm_kernel(const void* __
     for (int i = 0; i < R; i++) {
 #pragma unroll
       for (int u = 0; u < U; u++) {
-        dot[i].add(a[u][i], b[u][i]);
-        nrm[i].add(a[u][i]);
+        dot[i].add(u, a[u][i], b[u][i]);
+        nrm[i].add(u, a[u][i]);
       }
       dot[i].flush();
       nrm[i].flush();
@@ -539,13 +564,15 @@ __global__ void __launch_bounds__(kMaxThreads, 1) bicg_update_kernel(const doubl
   for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < sh.nchunks;) {
 #pragma unroll
     for (int u = 0; u < kGroup; u++, c += stride) {
-      if (c >= sh.nchunks) break;
-      E ps[R], ss[R], ts[R], rs[R], xs[R];
-      load_chunk<R>(p, c, ps);
-      load_chunk<R>(s, c, ss);
-      load_chunk<R>(t, c, ts);
-      load_chunk<R>(r0, c, rs);
-      load_chunk<R>(x, c, xs);
+      E ps[R] = {}, ss[R] = {}, ts[R] = {}, rs[R] = {}, xs[R] = {};
+      const bool in = c < sh.nchunks;
+      if (in) {
+        load_chunk<R>(p, c, ps);
+        load_chunk<R>(s, c, ss);
+        load_chunk<R>(t, c, ts);
+        load_chunk<R>(r0, c, rs);
+        load_chunk<R>(x, c, xs);
+      }
 #pragma unroll
       for (int i = 0; i < R; i++) {
         E no;
@@ -553,11 +580,13 @@ __global__ void __launch_bounds__(kMaxThreads, 1) bicg_update_kernel(const doubl
         no.y = -co[i].y;
         xs[i] = add_mul(co[i], ss[i], add_mul(ca[i], ps[i], xs[i]));
         ss[i] = add_mul(no, ts[i], ss[i]);
-        nrm[i].add(ss[i]);
-        dot[i].add(rs[i], ss[i]);
+        nrm[i].add(u, ss[i]);
+        dot[i].add(u, rs[i], ss[i]);
       }
-      store_chunk<R>(x, c, xs);
-      store_chunk<R>(s, c, ss);
+      if (in) {
+        store_chunk<R>(x, c, xs);
+        store_chunk<R>(s, c, ss);
+      }
     }
 #pragma unroll
     for (int i = 0; i < R; i++) {
@@ -627,11 +656,17 @@ __global__ void residual_kernel(const int* __restrict__ sel, const double2* __re
   const bool mine = sel[threadIdx.x % sh.G] != 0;
   double acc[1] = {0.0};
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  constexpr int U = 4;  // elements loaded ahead of the stores
   if (mine)
-    for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < sh.nchunks; c += stride) {
-      const double2 v = x[c];
-      add_square(acc[0], v);
-      st(y + c, v);
+    for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < sh.nchunks; c += U * stride) {
+      double2 v[U];
+#pragma unroll
+      for (int u = 0; u < U; u++) v[u] = c + u * stride < sh.nchunks ? x[c + u * stride] : make_double2(0.0, 0.0);
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        add_square(acc[0], v[u]);
+        if (c + u * stride < sh.nchunks) st(y + c + u * stride, v[u]);
+      }
     }
   __shared__ double sm[1024];
   block_reduce<double>(sm, acc, 1, sh.G, sh.nrhs, part);

@@ -162,6 +162,9 @@ inline Geometry make_geometry(const int L[4]) {
 // previous one or the same (backward).
 struct EoSite {
   uint32_t site, xh, y, z, t, eo;
+  __host__ __device__ __forceinline__ EoSite(uint32_t s, uint32_t xh_, uint32_t y_, uint32_t z_, uint32_t t_,
+                                             uint32_t eo_)
+      : site(s), xh(xh_), y(y_), z(z_), t(t_), eo(eo_) {}
   __host__ __device__ __forceinline__ EoSite(const Geometry& g, uint32_t s) : site(s) {
     uint32_t rest, rest2;
     g.div_hx.divmod(s, rest, xh);
@@ -190,16 +193,24 @@ struct EoSite {
 // instructions issue on the FP64 pipe (2 lanes a cycle and SM here, 1/64 of
 // the FP32 rate): a layout transform of FP32 fields kept it 76% busy and ran
 // at 58% of HBM.  Same rounding (to nearest even) and results as the
-// instructions, which the values outside the normal range still take.
+// instructions, which the values outside the normal range still take: in
+// functions of their own, so that they are branches and not predicated
+// instructions (which occupy the FP64 pipe whether or not a lane needs them).
+namespace cvt {
+static __device__ __noinline__ float f32(double v) { return (float)v; }
+static __device__ __noinline__ double f64(float v) { return (double)v; }
+static __device__ __noinline__ __nv_bfloat16 bf16(double v) { return __double2bfloat16(v); }
+}  // namespace cvt
 __device__ __forceinline__ float to_f32(double v) {
 #ifdef __CUDA_ARCH__
   const uint64_t u = (uint64_t)__double_as_longlong(v), a = u & 0x7fffffffffffffffull;
   const uint32_t sign = (uint32_t)(u >> 32) & 0x80000000u;
   if (a - 0x3810000000000000ull < 0x47f0000000000000ull - 0x3810000000000000ull)  // 2^-126 <= |v| < 2^128
     return __uint_as_float(sign | (uint32_t)((a - 0x3800000000000000ull + 0x0fffffffull + ((a >> 29) & 1u)) >> 29));
-  if (a == 0) return __uint_as_float(sign);
-#endif
+  return a == 0 ? __uint_as_float(sign) : cvt::f32(v);
+#else
   return (float)v;
+#endif
 }
 __device__ __forceinline__ double to_f64(float v) {
 #ifdef __CUDA_ARCH__
@@ -207,9 +218,10 @@ __device__ __forceinline__ double to_f64(float v) {
   const uint64_t sign = (uint64_t)(u & 0x80000000u) << 32;
   if (a - 0x00800000u < 0x7f800000u - 0x00800000u)  // normal
     return __longlong_as_double((long long)(sign | (((uint64_t)a << 29) + 0x3800000000000000ull)));
-  if (a == 0) return __longlong_as_double((long long)sign);
-#endif
+  return a == 0 ? __longlong_as_double((long long)sign) : cvt::f64(v);
+#else
   return (double)v;
+#endif
 }
 __device__ __forceinline__ __nv_bfloat16 to_bf16(double v) {
 #ifdef __CUDA_ARCH__
@@ -218,9 +230,10 @@ __device__ __forceinline__ __nv_bfloat16 to_bf16(double v) {
   if (a - 0x3810000000000000ull < 0x47f0000000000000ull - 0x3810000000000000ull)
     return __ushort_as_bfloat16((unsigned short)(
         sign | (uint32_t)((a - 0x3800000000000000ull + 0xfffffffffffull + ((a >> 45) & 1u)) >> 45)));
-  if (a == 0) return __ushort_as_bfloat16((unsigned short)sign);
-#endif
+  return a == 0 ? __ushort_as_bfloat16((unsigned short)sign) : cvt::bf16(v);
+#else
   return __double2bfloat16(v);
+#endif
 }
 
 // ---------------------------------------------------------------------------
