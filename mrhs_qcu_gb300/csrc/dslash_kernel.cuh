@@ -22,6 +22,8 @@
 // coefficients.
 #pragma once
 
+#include <type_traits>
+
 #include "qcu_common.cuh"
 
 namespace qcu {
@@ -224,13 +226,19 @@ __device__ __forceinline__ void load_su3_two_row(const char* lbase, uint32_t ls_
   }
 }
 
+__device__ __forceinline__ double flip_sign(double v, bool flip) {
+  const uint64_t u = (uint64_t)__double_as_longlong(v);
+  return __longlong_as_double((long long)(flip ? u ^ 0x8000000000000000ull : u));
+}
+
 // One hop (direction MU, forward or backward) accumulated into acc.
 //   s = -f (forward, projector 1 - f g) or +f (backward, 1 + f g)
 //   kup  = bc * scale_r        multiplies the two upper rows
 //   klo  = s * sign(lo) * bc * scale_r   the reconstructed lower rows
 // Offsets are 32-bit element indices into the field / gauge arrays (the host
 // checks that every array has fewer than 2^32 elements).
-template <int P, int N, int R, int MU, bool FWD, bool RC = false>
+// FIRST: the accumulator is empty, and bc = 1.
+template <int P, int N, int R, int MU, bool FWD, bool RC = false, bool FIRST = false>
 __device__ __forceinline__ void hop(C2<typename Store<P>::real> (&acc)[4][N][R], const DslashArgs& A,
                                    const typename Store<P>::elem* __restrict__ in,
                                    const typename Store<P>::elem* __restrict__ gauge, uint32_t link_off,
@@ -334,24 +342,42 @@ __device__ __forceinline__ void hop(C2<typename Store<P>::real> (&acc)[4][N][R],
           t[u][r].y = fma(ui, h[u][b][r].x, t[u][r].y);
         }
     }
+    if constexpr (FIRST) {
+      // no operation for the empty accumulator (FP64 arithmetic is bound by its pipe: 840
+      // operations per site and RHS at SU(3) instead of 864): the +-1 factors are sign flips
+      static_assert(P == PREC_DOUBLE, "unscaled");
 #pragma unroll
-    for (int r = 0; r < R; r++) {
-      const T ku = scale[r];
-      const T kl0 = klo0 * scale[r], kl1 = klo1 * scale[r];
-      acc[0][a][r].x = fma(ku, t[0][r].x, acc[0][a][r].x);
-      acc[0][a][r].y = fma(ku, t[0][r].y, acc[0][a][r].y);
-      acc[1][a][r].x = fma(ku, t[1][r].x, acc[1][a][r].x);
-      acc[1][a][r].y = fma(ku, t[1][r].y, acc[1][a][r].y);
-      if constexpr (im) {
-        acc[u0p][a][r].x = fma(-kl0, t[0][r].y, acc[u0p][a][r].x);
-        acc[u0p][a][r].y = fma(kl0, t[0][r].x, acc[u0p][a][r].y);
-        acc[u1p][a][r].x = fma(-kl1, t[1][r].y, acc[u1p][a][r].x);
-        acc[u1p][a][r].y = fma(kl1, t[1][r].x, acc[u1p][a][r].y);
-      } else {
-        acc[u0p][a][r].x = fma(kl0, t[0][r].x, acc[u0p][a][r].x);
-        acc[u0p][a][r].y = fma(kl0, t[0][r].y, acc[u0p][a][r].y);
-        acc[u1p][a][r].x = fma(kl1, t[1][r].x, acc[u1p][a][r].x);
-        acc[u1p][a][r].y = fma(kl1, t[1][r].y, acc[u1p][a][r].y);
+      for (int r = 0; r < R; r++) {
+        acc[0][a][r] = t[0][r];
+        acc[1][a][r] = t[1][r];
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+          C2<T>& lo = acc[u == 0 ? u0p : u1p][a][r];
+          const bool neg = (u == 0 ? klo0 : klo1) < (T)0;
+          lo.x = flip_sign(im ? t[u][r].y : t[u][r].x, neg != im);
+          lo.y = flip_sign(im ? t[u][r].x : t[u][r].y, neg);
+        }
+      }
+    } else {
+#pragma unroll
+      for (int r = 0; r < R; r++) {
+        const T ku = scale[r];
+        const T kl0 = klo0 * scale[r], kl1 = klo1 * scale[r];
+        acc[0][a][r].x = fma(ku, t[0][r].x, acc[0][a][r].x);
+        acc[0][a][r].y = fma(ku, t[0][r].y, acc[0][a][r].y);
+        acc[1][a][r].x = fma(ku, t[1][r].x, acc[1][a][r].x);
+        acc[1][a][r].y = fma(ku, t[1][r].y, acc[1][a][r].y);
+        if constexpr (im) {
+          acc[u0p][a][r].x = fma(-kl0, t[0][r].y, acc[u0p][a][r].x);
+          acc[u0p][a][r].y = fma(kl0, t[0][r].x, acc[u0p][a][r].y);
+          acc[u1p][a][r].x = fma(-kl1, t[1][r].y, acc[u1p][a][r].x);
+          acc[u1p][a][r].y = fma(kl1, t[1][r].x, acc[u1p][a][r].y);
+        } else {
+          acc[u0p][a][r].x = fma(kl0, t[0][r].x, acc[u0p][a][r].x);
+          acc[u0p][a][r].y = fma(kl0, t[0][r].y, acc[u0p][a][r].y);
+          acc[u1p][a][r].x = fma(kl1, t[1][r].x, acc[u1p][a][r].x);
+          acc[u1p][a][r].y = fma(kl1, t[1][r].y, acc[u1p][a][r].y);
+        }
       }
     }
   }
@@ -554,7 +580,9 @@ struct HopAcc<T, N, R, true> {
 // prefetch of the line holding p into L1: no register is held while it is in flight
 __device__ __forceinline__ void prefetch_l1(const void* p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
 
-template <int P, int N, int R, bool PK, int MU, bool FWD, bool RC>
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
+template <int P, int N, int R, bool PK, int MU, bool FWD, bool RC, bool FIRST = false>
 __device__ __forceinline__ void hop_any(HopAcc<typename Store<P>::real, N, R, PK>& acc, const DslashArgs& A,
                                        const typename Store<P>::elem* __restrict__ in,
                                        const typename Store<P>::elem* __restrict__ gauge, uint32_t link_off,
@@ -565,7 +593,7 @@ __device__ __forceinline__ void hop_any(HopAcc<typename Store<P>::real, N, R, PK
                                  (RC ? 32u : (uint32_t)A.geo.vh) * (uint32_t)sizeof(typename Store<P>::elem), nb,
                                  rhs0, bc, f);
   else
-    hop<P, N, R, MU, FWD, RC>(acc.c, A, in, gauge, link_off, nb, rhs0, bc, f);
+    hop<P, N, R, MU, FWD, RC, FIRST>(acc.c, A, in, gauge, link_off, nb, rhs0, bc, f);
 }
 
 }  // namespace detail
@@ -602,31 +630,57 @@ __device__ __forceinline__ void store_out(C2<typename Store<P>::real> (&acc)[4][
   const uint32_t o = site * nrhs + rhs0;
   // a plain D application (a = 1, no x): the accumulator is the result
   const bool plain = !xin && (sizeof(T) == 4 ? (!A.a_rhs_f && A.af == 1.f) : (!A.a_rhs_d && A.a == 1.0));
+  if (xin) {
+    // x in batches of up to 48 registers, each batch's loads issued together, from L2 (the site's
+    // lines were prefetched before the hops).  With a branch around every component the loads ran one
+    // after the other, a DRAM latency each: out = a D in + b x against D in alone, us, before / now,
+    // SU(3) nrhs 12 FP32 24^3x48 389 / 245 (plain 231), 32^3x64 1226 / 866 (656), SU(4) 16^3x32 nrhs 16
+    // 245 / 138 (125)
+    constexpr int B = R * (int)sizeof(E) >= 192 ? 1 : 192 / (R * (int)sizeof(E));
+    constexpr int NB = B < 4 * N ? B : 4 * N;
+    auto add_x = [&](auto unit) {  // unit: b = 1, one operation less per real component
 #pragma unroll
-  for (int sp = 0; sp < 4; sp++)
+      for (int k0 = 0; k0 < 4 * N; k0 += NB) {
+        VecBuf<E, R> xv[NB];
 #pragma unroll
-    for (int a = 0; a < N; a++) {
-      const uint32_t off = o + (uint32_t)(sp * N + a) * cs;
-      if (plain) continue;
-      if (xin) {
-        VecBuf<E, R> xv;
-        Vec<E, R>::load(xin + off, xv.v);
+        for (int k = 0; k < NB; k++)
+          if (k0 + k < 4 * N) Vec<E, R>::load(xin + (o + (uint32_t)(k0 + k) * cs), xv[k].v);
 #pragma unroll
-        for (int r = 0; r < R; r++) {
-          auto xc = S::to_c(xv.v[r]);
-          T sx = cbx;
-          if constexpr (S::has_norm) sx *= (T)xs[r];
-          acc[sp][a][r].x = fma(sx, (T)xc.x, ca[r] * acc[sp][a][r].x);
-          acc[sp][a][r].y = fma(sx, (T)xc.y, ca[r] * acc[sp][a][r].y);
+        for (int k = 0; k < NB; k++) {
+          if (k0 + k >= 4 * N) continue;
+#pragma unroll
+          for (int r = 0; r < R; r++) {
+            const auto xc = S::to_c(xv[k].v[r]);
+            C2<T>& v = acc[(k0 + k) / N][(k0 + k) % N][r];
+            if constexpr (decltype(unit)::value) {
+              v.x = fma(ca[r], v.x, (T)xc.x);
+              v.y = fma(ca[r], v.y, (T)xc.y);
+            } else {
+              T sx = cbx;
+              if constexpr (S::has_norm) sx *= (T)xs[r];
+              v.x = fma(sx, (T)xc.x, ca[r] * v.x);
+              v.y = fma(sx, (T)xc.y, ca[r] * v.y);
+            }
+          }
         }
-      } else {
+      }
+    };
+    // two bodies: as one with a select, both sides' FP64 operations would take the pipe
+    if (!S::has_norm && cbx == (T)1)
+      add_x(std::true_type{});
+    else
+      add_x(std::false_type{});
+  } else if (!plain) {
+#pragma unroll
+    for (int sp = 0; sp < 4; sp++)
+#pragma unroll
+      for (int a = 0; a < N; a++)
 #pragma unroll
         for (int r = 0; r < R; r++) {
           acc[sp][a][r].x *= ca[r];
           acc[sp][a][r].y *= ca[r];
         }
-      }
-    }
+  }
 
   E* __restrict__ out = static_cast<E*>(A.out);
   if constexpr (S::has_norm) {
@@ -736,6 +790,17 @@ __device__ __forceinline__ void wilson_site(const DslashArgs& A, uint32_t gid) {
   const E* __restrict__ gauge = static_cast<const E*>(RC ? A.gauge12 : A.gauge);
   constexpr uint32_t NN = RC ? (N - 1) * N : N * N;  // stored components per link
 
+  // the xpay field's lines into L2 while the hops run (each line by one of the lanes that share it)
+  if (A.x) {
+    constexpr uint32_t kLanes = 128u / (R * sizeof(E)) < 32u ? 128u / (R * sizeof(E)) : 32u;
+    const E* x = static_cast<const E*>(A.x) + (site * (uint32_t)A.nrhs + rhs0);
+#pragma unroll
+    for (uint32_t c = 0; c < 4u * N; c += kLanes) {
+      const uint32_t k = c + (threadIdx.x & (kLanes - 1u));
+      if (k < 4u * N) prefetch_l2(x + k * (vh * (uint32_t)A.nrhs));
+    }
+  }
+
   HopAcc<T, N, R, PK> hacc;
   hacc.zero();
 
@@ -793,7 +858,7 @@ __device__ __forceinline__ void wilson_site(const DslashArgs& A, uint32_t gid) {
     {  // X
       const uint32_t nf = (eo != p) ? (xh == hx - 1 ? site - (hx - 1) : site + 1) : site;
       const uint32_t nbk = (eo == p) ? (xh == 0 ? site + (hx - 1) : site - 1) : site;
-      hop_any<P, N, R, PK, 0, true, RC>(hacc, A, in, gauge, lf, nf, rhs0, (T)1, f);
+      hop_any<P, N, R, PK, 0, true, RC, P == PREC_DOUBLE>(hacc, A, in, gauge, lf, nf, rhs0, (T)1, f);
       hop_any<P, N, R, PK, 0, false, RC>(hacc, A, in, gauge, lb + lsite(nbk), nbk, rhs0, (T)1, f);
     }
     {  // Y
