@@ -15,6 +15,7 @@ from __future__ import annotations
 
 import ctypes
 import os
+import struct
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "libqcu.so")
@@ -86,6 +87,10 @@ class QcuHopSegment(ctypes.Structure):
                 ("in_", ctypes.c_void_p), ("out", ctypes.c_void_p), ("x", ctypes.c_void_p),
                 ("a", ctypes.c_double), ("b", ctypes.c_double), ("nrhs", ctypes.c_int), ("parity", ctypes.c_int),
                 ("dagger", ctypes.c_int), ("antiperiodic_t", ctypes.c_int)]
+
+
+_SEGMENT = struct.Struct("@4i5P2d4i")  # QcuHopSegment packed in one call
+assert _SEGMENT.size == ctypes.sizeof(QcuHopSegment)
 
 
 class QcuRequestInfo(ctypes.Structure):
@@ -302,15 +307,24 @@ def eo_to_lex(lex_out, eo_in, ncomp: int) -> None:
     _raise_if(lib().qcuEoToLex(_p(lex_out), _p(eo_in), int(ncomp)))
 
 
+def _a(x):
+    """A device address for a c_void_p argument, without a ctypes object of its own."""
+    return None if x is None else int(x)
+
+
 def dslash_mrhs(out, out_norm, inp, in_norm, nrhs: int, parity: int, dagger: int, precision: int) -> None:
-    _raise_if(lib().qcuDslashMRHS(_p(out), _p(out_norm), _p(inp), _p(in_norm), int(nrhs), int(parity), int(dagger),
-                                  int(precision)))
+    rc = (_lib or lib()).qcuDslashMRHS(_a(out), _a(out_norm), _a(inp), _a(in_norm), int(nrhs), int(parity),
+                                       int(dagger), int(precision))
+    if rc:
+        _raise_if(rc)
 
 
 def dslash_xpay_mrhs(out, out_norm, inp, in_norm, x, x_norm, nrhs: int, parity: int, dagger: int, precision: int,
                      a: float, b: float) -> None:
-    _raise_if(lib().qcuDslashXpayMRHS(_p(out), _p(out_norm), _p(inp), _p(in_norm), _p(x), _p(x_norm), int(nrhs),
-                                      int(parity), int(dagger), int(precision), float(a), float(b)))
+    rc = (_lib or lib()).qcuDslashXpayMRHS(_a(out), _a(out_norm), _a(inp), _a(in_norm), _a(x), _a(x_norm), int(nrhs),
+                                           int(parity), int(dagger), int(precision), float(a), float(b))
+    if rc:
+        _raise_if(rc)
 
 
 def dslash_segments(segments, n_colors: int, precision: int, stream=None) -> None:
@@ -318,16 +332,13 @@ def dslash_segments(segments, n_colors: int, precision: int, stream=None) -> Non
     (qcuDslashSegments).  `segments`: dicts with keys lattice, gauge,
     gauge_two_row (or None), in_, out, x (or None), a, b, nrhs, parity,
     dagger, antiperiodic_t; pointers are device addresses."""
-    arr = (QcuHopSegment * max(1, len(segments)))()
-    for i, d in enumerate(segments):
-        g = arr[i]
-        g.lattice = (ctypes.c_int * 4)(*d["lattice"])
-        g.gauge, g.gauge_two_row = d["gauge"], d.get("gauge_two_row")
-        g.in_, g.out, g.x = d["in_"], d["out"], d.get("x")
-        g.a, g.b = d.get("a", 1.0), d.get("b", 0.0)
-        g.nrhs, g.parity, g.dagger = d["nrhs"], d.get("parity", 0), d.get("dagger", 0)
-        g.antiperiodic_t = int(bool(d.get("antiperiodic_t", False)))
-    _raise_if(lib().qcuDslashSegments(arr, len(segments), int(n_colors), int(precision), _p(stream)))
+    data = b"".join(
+        _SEGMENT.pack(*d["lattice"], d["gauge"] or 0, d.get("gauge_two_row") or 0, d["in_"] or 0, d["out"] or 0,
+                      d.get("x") or 0, d.get("a", 1.0), d.get("b", 0.0), d["nrhs"], d.get("parity", 0), d.get("dagger", 0),
+                      bool(d.get("antiperiodic_t", False))) for d in segments)
+    n = len(segments)
+    arr = (QcuHopSegment * n).from_buffer_copy(data) if n else (QcuHopSegment * 1)()
+    _raise_if(lib().qcuDslashSegments(arr, n, int(n_colors), int(precision), _p(stream)))
 
 
 def check_wait_timeout(limit_seconds: float) -> int:

@@ -6,6 +6,7 @@
 // instead of terminating the process (the reference's errorQcu / CHECK_CUDA
 // call exit(1), include/qcu_macro.cuh:16-40); QCU_ABORT_ON_ERROR=1 restores
 // that behaviour.
+#include <atomic>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -13,6 +14,7 @@
 #include <memory>
 #include <mutex>
 #include <string>
+#include <thread>
 
 #pragma GCC visibility push(default)  // the public headers: exported
 #include "../../include/qcu.h"
@@ -107,7 +109,7 @@ void apply_settings(Session& s) {
 
 // run the hopping term on caller-layout fermions through the session
 void caller_dslash(Session& s, int prec, void* const* outs, void* const* ins, int n, int in_mode, int out_mode,
-                   int parity, int dagger) {
+                   int parity, int dagger, bool wait = true) {
   using namespace qcu;
   for (int base = 0; base < n; base += QCU_MAX_RHS) {
     const int m = std::min(QCU_MAX_RHS, n - base);
@@ -122,8 +124,58 @@ void caller_dslash(Session& s, int prec, void* const* outs, void* const* ins, in
     s.hop(fout, fin, FieldView{}, parity, dagger, 1.0, 0.0);
     unpack_fermions(prec, s.N, pout, out_mode, parity, fout.data, fout.norm, s.geo, m, s.stream());
   }
-  s.sync();
+  if (wait) s.sync();
 }
+
+// The session of the one-call operators (dslashQcu, fullDslashQcu).  Between
+// calls on one lattice and device it keeps its stream and buffers: setting
+// them up and freeing them took 0.4 of the 0.59 ms of a 12^3x24 call.  At most kKeepBytes stay
+// allocated; another lattice, initGridSize and an allocation that would fail
+// free them.  Used under the API lock; `busy` keeps an allocation of a solve
+// server's thread from freeing it during a call.
+class OneCall {
+ public:
+  static constexpr size_t kKeepBytes = (size_t)256 << 20;
+  template <typename F>
+  void run(const QcuParam& p, F&& f) {
+    while (busy_.exchange(true)) std::this_thread::yield();
+    struct Done {
+      OneCall& o;
+      bool ok = false;
+      ~Done() {
+        if (!ok || (o.s_ && o.s_->device_bytes() > kKeepBytes)) o.s_.reset();
+        o.busy_.store(false);
+      }
+    } done{*this};
+    int dev = 0;
+    QCU_CHECK_CUDA(cudaGetDevice(&dev));
+    bool same = s_ && dev == device_;
+    for (int i = 0; same && i < 4; i++) same = s_->latt.dim[i] == p.lattice_size[i];
+    if (!same) {
+      s_.reset();
+      const int g[4] = {1, 1, 1, 1};
+      s_.reset(new Session(p.lattice_size, g, 3));
+      device_ = dev;
+    }
+    apply_settings(*s_);
+    f(*s_);
+    done.ok = true;
+  }
+  bool release() {
+    if (busy_.exchange(true)) return false;
+    const bool had = s_ != nullptr;
+    s_.reset();
+    busy_.store(false);
+    return had;
+  }
+
+ private:
+  std::unique_ptr<Session> s_;
+  int device_ = 0;
+  std::atomic<bool> busy_{false};
+};
+OneCall g_one_call;
+const bool g_release_set = (qcu::release_idle_memory = [] { return g_one_call.release(); }, true);
 
 }  // namespace
 
@@ -147,6 +199,7 @@ void initGridSize(QcuGrid_t* grid, QcuParam* p_param, int nColors) {
       QCU_REQUIRE(g[i] == 1, QCU_ERR_UNSUPPORTED,
                   "process grids other than 1x1x1x1 are not supported (one GPU per process)");
     g_session.reset();
+    g_one_call.release();
     g_session.reset(new Session(p_param->lattice_size, g, nColors));
     apply_settings(*g_session);
   });
@@ -205,11 +258,10 @@ void dslashQcu(void* fermion_out, void* fermion_in, void* gauge, QcuParam* param
   guarded([&] {
     check_lattice(param);
     QCU_REQUIRE(fermion_out && fermion_in && gauge, QCU_ERR_INVALID_ARGUMENT, "null pointer");
-    int g[4] = {1, 1, 1, 1};
-    Session s(param->lattice_size, g, 3);
-    apply_settings(s);
-    s.load_gauge(gauge, 0);
-    caller_dslash(s, qcu::PREC_DOUBLE, &fermion_out, &fermion_in, 1, qcu::SRC_EO_HALF, qcu::SRC_EO_HALF, parity, 0);
+    g_one_call.run(*param, [&](Session& s) {
+      s.load_gauge(gauge, 0);
+      caller_dslash(s, qcu::PREC_DOUBLE, &fermion_out, &fermion_in, 1, qcu::SRC_EO_HALF, qcu::SRC_EO_HALF, parity, 0);
+    });
   });
 }
 
@@ -217,13 +269,12 @@ void fullDslashQcu(void* fermion_out, void* fermion_in, void* gauge, QcuParam* p
   guarded([&] {
     check_lattice(param);
     QCU_REQUIRE(fermion_out && fermion_in && gauge, QCU_ERR_INVALID_ARGUMENT, "null pointer");
-    int g[4] = {1, 1, 1, 1};
-    Session s(param->lattice_size, g, 3);
-    apply_settings(s);
-    s.load_gauge(gauge, 0);
-    for (int p = 0; p < 2; p++)
-      caller_dslash(s, qcu::PREC_DOUBLE, &fermion_out, &fermion_in, 1, qcu::SRC_EO_FULL, qcu::SRC_EO_FULL, p,
-                    dagger_flag);
+    g_one_call.run(*param, [&](Session& s) {
+      s.load_gauge(gauge, 0);
+      for (int p = 0; p < 2; p++)
+        caller_dslash(s, qcu::PREC_DOUBLE, &fermion_out, &fermion_in, 1, qcu::SRC_EO_FULL, qcu::SRC_EO_FULL, p,
+                      dagger_flag, p == 1);
+    });
   });
 }
 
@@ -581,35 +632,39 @@ int qcuDslashSegments(const QcuHopSegment* segments, int count, int nColors, int
     qcu::Autotuner& tuner = qcu::global_tuner();
     bool found = false;
     const qcu::DslashArgs& B = segs[big];
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    QCU_CHECK_CUDA(cudaStreamIsCapturing(st, &cs));
-    const bool may_tune = tuner.enabled() && cs == cudaStreamCaptureStatusNone;
+    auto may_tune = [&] {
+      cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+      QCU_CHECK_CUDA(cudaStreamIsCapturing(st, &cs));
+      return tuner.enabled() && cs == cudaStreamCaptureStatusNone;
+    };
     qcu::DslashConfig c;
     if (getenv("QCU_DSLASH_CONFIG")) c = tuner.lookup(precision, nColors, B.nrhs, B.geo.vh, &found);
     if (!found && count > 1) {  // one segment: the lattice's own tuned shape, as for qcuDslashMRHS
-      std::string key = std::to_string(precision) + ":" + std::to_string(nColors);
-      for (const qcu::DslashArgs& A : segs)
-        key += ":" + std::to_string(A.geo.vh) + "x" + std::to_string(A.nrhs) + (A.gauge12 ? "r" : "f");
-      static std::map<std::string, qcu::DslashConfig> tuned_lists;  // under the API lock
+      std::vector<int> key{precision, nColors};
+      for (const qcu::DslashArgs& A : segs) {
+        key.push_back(A.geo.vh);
+        key.push_back(2 * A.nrhs + (A.gauge12 ? 1 : 0));
+      }
+      static std::map<std::vector<int>, qcu::DslashConfig> tuned_lists;  // under the API lock
       auto it = tuned_lists.find(key);
       if (it != tuned_lists.end()) {
         c = it->second;
         found = true;
-      } else if (may_tune) {
+      } else if (may_tune()) {
         c = tune_work_list(segs, precision, nColors, st, &found);
         if (found) tuned_lists[key] = c;
       }
     }
     if (!found) {
       c = tuner.lookup(precision, nColors, B.nrhs, B.geo.vh, &found);
-      if (!found && may_tune) c = tuner.tune(B, precision, nColors, st);
+      if (!found && may_tune()) c = tuner.tune(B, precision, nColors, st);
     }
     std::vector<int> misfits;
     qcu::launch_dslash_segments(segs, precision, nColors, c, st, &misfits);
     for (int i : misfits) {  // an RHS count the shared shape cannot take: the segment's own shape
       const qcu::DslashArgs& A = segs[i];
       qcu::DslashConfig own = tuner.lookup(precision, nColors, A.nrhs, A.geo.vh, &found);
-      if (!found && may_tune) own = tuner.tune(A, precision, nColors, st);
+      if (!found && may_tune()) own = tuner.tune(A, precision, nColors, st);
       qcu::launch_dslash(A, precision, nColors, own, st);
     }
   });

@@ -15,11 +15,17 @@
 namespace qcu {
 
 // ---------------------------------------------------------------------------
+bool (*release_idle_memory)() = nullptr;
+
 void* DeviceBuffer::ensure(size_t bytes) {
   if (bytes == 0) bytes = 16;
   if (bytes > bytes_) {
     release();
-    const cudaError_t e = cudaMalloc(&p_, bytes);
+    cudaError_t e = cudaMalloc(&p_, bytes);
+    if (e == cudaErrorMemoryAllocation && release_idle_memory && release_idle_memory()) {
+      (void)cudaGetLastError();
+      e = cudaMalloc(&p_, bytes);
+    }
     if (e != cudaSuccess) {
       p_ = nullptr;
       // clear the runtime's last error, so the next launch check does not report this failure again
@@ -59,12 +65,6 @@ bool Autotuner::enabled() const {
   return !(e && e[0] == '0');
 }
 
-std::string Autotuner::key(int prec, int N, int nrhs, int vh) const {
-  std::ostringstream o;
-  o << prec << ":" << N << ":" << nrhs << ":" << vh;
-  return o.str();
-}
-
 void Autotuner::load_file() {
   file_loaded_ = true;
   const char* path = getenv("QCU_TUNE_CACHE");
@@ -80,7 +80,8 @@ void Autotuner::load_file() {
     if (!(ls >> c.tc)) c.tc = 0;
     if (!(ls >> c.rc)) c.rc = 0;
     if (!(ls >> c.lt)) c.lt = 0;
-    cache_[k] = c;
+    Key key;
+    if (sscanf(k.c_str(), "%d:%d:%d:%d", &key.prec, &key.N, &key.nrhs, &key.vh) == 4) cache_[key] = c;
   }
 }
 
@@ -89,7 +90,7 @@ void Autotuner::save_file() {
   if (!path) return;
   std::ofstream out(path);
   for (auto& kv : cache_)
-    out << kv.first << " " << kv.second.R << " " << kv.second.block << " " << kv.second.minb << " " << kv.second.pk
+    out << kv.first.prec << ":" << kv.first.N << ":" << kv.first.nrhs << ":" << kv.first.vh << " " << kv.second.R << " " << kv.second.block << " " << kv.second.minb << " " << kv.second.pk
         << " " << kv.second.tma << " " << kv.second.rcta << " " << kv.second.tc << " " << kv.second.rc << " "
         << kv.second.lt << "\n";
 }
@@ -121,27 +122,27 @@ DslashConfig Autotuner::lookup(int prec, int N, int nrhs, int vh, bool* found) {
     }
   }
   if (!file_loaded_) load_file();
-  auto it = cache_.find(key(prec, N, nrhs, vh));
+  auto it = cache_.find(Key{prec, N, nrhs, vh});
   *found = it != cache_.end();
   return *found ? it->second : heuristic(prec, N, nrhs);
 }
 
 void Autotuner::store(int prec, int N, int nrhs, int vh, const DslashConfig& c) {
   std::lock_guard<std::mutex> lk(m_);
-  cache_[key(prec, N, nrhs, vh)] = c;
+  cache_[Key{prec, N, nrhs, vh}] = c;
   save_file();
 }
 
 bool Autotuner::layout_site_major(int N, int nrhs, int vh, bool* known) {
   std::lock_guard<std::mutex> lk(m_);
-  auto it = layout_.find(key(PREC_BF16S, N, nrhs, vh));
+  auto it = layout_.find(Key{PREC_BF16S, N, nrhs, vh});
   *known = it != layout_.end();
   return *known && it->second;
 }
 
 void Autotuner::store_layout(int N, int nrhs, int vh, bool site_major) {
   std::lock_guard<std::mutex> lk(m_);
-  layout_[key(PREC_BF16S, N, nrhs, vh)] = site_major;
+  layout_[Key{PREC_BF16S, N, nrhs, vh}] = site_major;
 }
 
 DslashConfig Autotuner::heuristic(int prec, int N, int nrhs) {
@@ -170,46 +171,30 @@ DslashConfig Autotuner::tune(const DslashArgs& A, int prec, int N, cudaStream_t 
     DslashConfig c = lookup(prec, N, A.nrhs, A.geo.vh, &pinned);
     if (pinned) return c;
   }
+  std::vector<DslashConfig> cand;
   int opts[8];
   const int n = dslash_r_options(prec, N, opts, 8);
-  const int blocks[] = {32, 64, 128, 256};
-  cudaEvent_t e0, e1;
-  QCU_CHECK_CUDA(cudaEventCreate(&e0));
-  QCU_CHECK_CUDA(cudaEventCreate(&e1));
-  DslashConfig best = heuristic(prec, N, A.nrhs);
-  float best_ms = 1e30f;
   for (int i = 0; i < n; i++) {
     if (A.nrhs % opts[i]) continue;
     // scalar / packed FP32x2 arithmetic x full / two-row links x links from L1 / staged by TMA
     for (int v = 0; v < 8; v++) {
-    const int pk = v & 1, rc = (v >> 1) & 1, lt = v >> 2;
-    if (rc && !A.gauge12) continue;
-    if (lt && !tmalink_runs(A, opts[i], prec_complex_bytes(prec), rc ? (N - 1) * N : N * N)) continue;
-    int minbs[8];
-    const int nm = dslash_minb_options(prec, N, opts[i], pk, minbs, 8, rc, lt);
-    for (int j = 0; j < nm; j++)
-      for (int b : blocks) {
-        if (lt && b != blocks[0]) continue;  // the link-staged kernel's CTA is one x-row, whatever the block
-        DslashConfig c;
-        c.R = opts[i];
-        c.block = b;
-        c.minb = minbs[j];
-        c.pk = pk;
-        c.rc = rc;
-        c.lt = lt;
-        launch_dslash(A, prec, N, c, st);  // warm-up
-        QCU_CHECK_CUDA(cudaEventRecord(e0, st));
-        const int reps = 3;
-        for (int k = 0; k < reps; k++) launch_dslash(A, prec, N, c, st);
-        QCU_CHECK_CUDA(cudaEventRecord(e1, st));
-        QCU_CHECK_CUDA(cudaEventSynchronize(e1));
-        float ms = 0;
-        QCU_CHECK_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-        if (ms < best_ms) {
-          best_ms = ms;
-          best = c;
+      const int pk = v & 1, rc = (v >> 1) & 1, lt = v >> 2;
+      if (rc && !A.gauge12) continue;
+      if (lt && !tmalink_runs(A, opts[i], prec_complex_bytes(prec), rc ? (N - 1) * N : N * N)) continue;
+      int minbs[8];
+      const int nm = dslash_minb_options(prec, N, opts[i], pk, minbs, 8, rc, lt);
+      for (int j = 0; j < nm; j++)
+        for (int b : {32, 64, 128, 256}) {
+          if (lt && b != 32) continue;  // the link-staged kernel's CTA is one x-row, whatever the block
+          DslashConfig c;
+          c.R = opts[i];
+          c.block = b;
+          c.minb = minbs[j];
+          c.pk = pk;
+          c.rc = rc;
+          c.lt = lt;
+          cand.push_back(c);
         }
-      }
     }
   }
   // the TMA-staged kernel, where these arguments fit it
@@ -219,19 +204,7 @@ DslashConfig Autotuner::tune(const DslashArgs& A, int prec, int N, cudaStream_t 
     DslashConfig c;
     c.R = tr[i];
     c.tma = ts[i];
-    if (!tma_runs(A, prec, N, c)) continue;
-    launch_dslash(A, prec, N, c, st);  // warm-up
-    QCU_CHECK_CUDA(cudaEventRecord(e0, st));
-    const int reps = 3;
-    for (int k = 0; k < reps; k++) launch_dslash(A, prec, N, c, st);
-    QCU_CHECK_CUDA(cudaEventRecord(e1, st));
-    QCU_CHECK_CUDA(cudaEventSynchronize(e1));
-    float ms = 0;
-    QCU_CHECK_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-    if (ms < best_ms) {
-      best_ms = ms;
-      best = c;
-    }
+    if (tma_runs(A, prec, N, c)) cand.push_back(c);
   }
   // the tensor-core kernels, where these arguments fit them; at N <= 4 the
   // CUDA-core kernels were faster than the tcgen05 ones at every RHS count
@@ -241,19 +214,35 @@ DslashConfig Autotuner::tune(const DslashArgs& A, int prec, int N, cudaStream_t 
     if (N <= 4 && !prec_site_major(prec) && variant != kMmaVariant) continue;
     DslashConfig c;
     c.tc = variant;
-    launch_dslash(A, prec, N, c, st);  // warm-up
+    cand.push_back(c);
+  }
+  if (cand.empty()) return heuristic(prec, N, A.nrhs);
+
+  cudaEvent_t e0, e1;
+  QCU_CHECK_CUDA(cudaEventCreate(&e0));
+  QCU_CHECK_CUDA(cudaEventCreate(&e1));
+  auto time = [&](const DslashConfig& c, int reps) {  // ms a launch, after one untimed
+    launch_dslash(A, prec, N, c, st);
     QCU_CHECK_CUDA(cudaEventRecord(e0, st));
-    const int reps = 3;
     for (int k = 0; k < reps; k++) launch_dslash(A, prec, N, c, st);
     QCU_CHECK_CUDA(cudaEventRecord(e1, st));
     QCU_CHECK_CUDA(cudaEventSynchronize(e1));
     float ms = 0;
     QCU_CHECK_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-    if (ms < best_ms) {
-      best_ms = ms;
-      best = c;
-    }
-  }
+    return ms / reps;
+  };
+  // Every shape once, then the nearest few again, keeping each one's best: a
+  // single pass picked shapes 20% slower than the best where another stream's
+  // work or the clocks' ramp fell on the wrong one.
+  std::vector<std::pair<float, size_t>> t;
+  for (size_t i = 0; i < cand.size(); i++) t.emplace_back(time(cand[i], 2), i);
+  std::sort(t.begin(), t.end());
+  const float near = 1.3f * t[0].first;
+  while (t.size() > 8 || t.back().first > near) t.pop_back();
+  const int reps = std::max(3, std::min(20, (int)(0.2f / std::max(t[0].first, 1e-3f))));
+  for (int round = 0; round < 2; round++)
+    for (auto& k : t) k.first = std::min(k.first, time(cand[k.second], reps));
+  const DslashConfig best = cand[std::min_element(t.begin(), t.end())->second];
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   store(prec, N, A.nrhs, A.geo.vh, best);
@@ -486,7 +475,6 @@ void Session::hop(FieldView out, FieldView in, FieldView x, int parity, int dagg
               "dslash operands must share nrhs");
   DslashArgs A;
   A.gauge = gauge(in.prec);
-  A.gauge12 = gauge12(in.prec);
   A.in = in.data;
   A.in_norm = in.norm;
   A.out = out.data;
@@ -505,9 +493,13 @@ void Session::hop(FieldView out, FieldView in, FieldView x, int parity, int dagg
   A.antiperiodic_t = antiperiodic_t ? 1 : 0;
   bool found = false;
   DslashConfig c = tuner.lookup(in.prec, N, in.nrhs, geo.vh, &found);
-  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-  QCU_CHECK_CUDA(cudaStreamIsCapturing(stream(), &cs));
-  const bool tunes = !found && tuner.enabled() && cs == cudaStreamCaptureStatusNone;
+  bool tunes = false;
+  if (!found && tuner.enabled()) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    QCU_CHECK_CUDA(cudaStreamIsCapturing(stream(), &cs));
+    tunes = cs == cudaStreamCaptureStatusNone;
+  }
+  if (tunes || c.rc) A.gauge12 = gauge12(in.prec);  // measured and built on first use
   tensor_links(A, in.prec, tunes ? -1 : c.tc);
   if (tunes) c = tuner.tune(A, in.prec, N, stream());
   launch_dslash(A, in.prec, N, c, stream());
@@ -526,6 +518,13 @@ Blas& Session::blas() {
     blas_.reset(new Blas(p, max_blocks));
   }
   return *blas_;
+}
+
+size_t Session::device_bytes() const {
+  size_t b = ws.total_bytes() + gauge_tc_.bytes() + clover_flag_.bytes() + su3_scratch_.bytes() + partials_.bytes() +
+             scalars_.bytes() + gauge_rec_[0].bytes() + gauge_rec_[1].bytes();
+  for (int p = 0; p < 5; p++) b += gauge_[p].bytes() + gauge12_[p].bytes() + clover_[p].bytes() + cloverinv_[p].bytes();
+  return b;
 }
 
 double* Session::scalars(size_t count) { return static_cast<double*>(scalars_.ensure(count * sizeof(double))); }

@@ -18,6 +18,7 @@
 #include <memory>
 #include <mutex>
 #include <string>
+#include <tuple>
 #include <vector>
 
 #include "blas.h"
@@ -32,6 +33,10 @@ struct LattDesc {
 struct ProcDesc {
   int dim[4];
 };
+
+// Frees device memory that the library keeps only to reuse; true if it freed
+// any (set by qcu_api.cu; an allocation that fails tries once more after it).
+extern bool (*release_idle_memory)();
 
 class DeviceBuffer {
  public:
@@ -75,10 +80,15 @@ class Autotuner {
   void store_layout(int N, int nrhs, int vh, bool site_major);
 
  private:
+  struct Key {
+    int prec, N, nrhs, vh;
+    bool operator<(const Key& o) const {
+      return std::tie(prec, N, nrhs, vh) < std::tie(o.prec, o.N, o.nrhs, o.vh);
+    }
+  };
   std::mutex m_;
-  std::map<std::string, DslashConfig> cache_;
-  std::map<std::string, bool> layout_;
-  std::string key(int prec, int N, int nrhs, int vh) const;
+  std::map<Key, DslashConfig> cache_;
+  std::map<Key, bool> layout_;
   void load_file();
   void save_file();
   bool file_loaded_ = false;
@@ -200,6 +210,8 @@ class Session {
   void hop(FieldView out, FieldView in, FieldView x, int parity, int dagger, double a, double b,
            const int* mask = nullptr, const float* a_rhs_f = nullptr, const double* a_rhs_d = nullptr);
 
+  // device memory this session holds
+  size_t device_bytes() const;
   Blas& blas();
   double* scalars(size_t count);  // device scratch for per-RHS scalars
 
