@@ -1,0 +1,390 @@
+// FP64 Wilson hop of SU(3) and SU(4) with the colour multiply in block fixed point.
+//
+// The FP64 pipe of sm_103a takes 2 multiply-adds per clock and SM, and 840 of them a site and RHS kept
+// it 97% busy at SU(3).  32 x 32 -> 64-bit integer multiply-adds run at about 16 times that rate.  So
+// only the projection (12 operations a hop at SU(3)) is left on the FP64 pipe, and the colour multiply
+// and the sum over hops are done in integers:
+//
+//   projected spinor   the 4N real parts of a neighbour's two rows, 59 bits over their common exponent
+//   link               its 2N^2 real parts, 59 bits over theirs
+//   product            limbs of 28 and 31 bits, the three larger limb products summed exactly in two
+//                      64-bit accumulators a component; only low x low (2^-56 of the operands' largest
+//                      parts, at most) is left out
+//   sum over hops      64-bit integers over the largest hop's exponent
+//   result             rounded once to double (nearest even); the xpay epilogue stays FP64
+//
+// No sum can overflow (the bounds stand beside the constants), and none rounds before the last step
+// but by the right shifts to the accumulator's unit.  Relative L2 error against quad precision on random
+// fields: 0.84e-16, where the FP64 multiply-adds have 1.45e-16 (SU(3)) and 1.54e-16 (SU(4)).
+//
+// One hop, us, FP64 multiply-adds / this: SU(3) 24^3x48 nrhs 12 5826 / 1770, SU(4) 16^3x32 nrhs 16
+// 2480 / 736, SU(3) 14x10x6x18 nrhs 5 59 / 27, SU(3) 12^3x24 nrhs 1 44 / 27.  It is bound by instruction
+// issue and latency (SU(3): 8300 instructions a warp, 216 wide multiply-adds a hop; the multiplier 53%
+// busy, the integer pipe 43%, FP64 33%, 12 or 16 warps an SM); the small sizes by the latency of one
+// warp a scheduler.
+//
+// A common exponent keeps the digits of a part only down to its unit.  So a site takes the FP64
+// multiply-adds (fp64_site, the arithmetic of the other SU(N)) when the non-zero parts that it
+// multiplies span more than kFixSpan bits, when anything it reads is infinite or NaN, and when the
+// result could leave the normal range.
+#pragma once
+
+namespace qcu {
+namespace detail {
+
+// the FP64 SU(N) hops that run in fixed point (the accumulators hold sums over N = 4 at most)
+__host__ __device__ constexpr bool fix_hop(int prec, int N) { return prec == PREC_DOUBLE && (N == 3 || N == 4); }
+
+// A part 32 bits below the largest keeps 24 digits of its own.  One site in FP64 multiply-adds takes a
+// warp 27 us, as long as a small launch: at 24 bits, where 1e-5 of random sites span more, SU(3)
+// 14x10x6x18 nrhs 5 took 54 us against 27.
+constexpr int kFixSpan = 32;
+
+// Parts |F| < 2^59 as limbs F = hi 2^31 + lo, |hi| <= 2^28, |lo| < 2^31.  Over a component's 2N products:
+//   high  |sum uh hh|            <= 2N 2^56     (N = 4: 2^59)
+//   mid   |sum uh hl + ul hh|    <= 2N 2 2^28 (2^31 - 1)   (N = 4: 2^63 - 2^32, so the rounding bit fits)
+// A hop's sum in the accumulator's unit is high + (mid >> 31), below 2^59 + 2^32 at N = 4; eight of
+// them stay below 2^63.
+constexpr uint32_t kFixShift = 5;  // right shift of a mantissa whose top bit is bit 63
+
+struct Limbs {
+  int32_t hi, lo;
+};
+
+__device__ __forceinline__ uint32_t biased_exp(double x) { return ((uint32_t)__double2hiint(x) >> 20) & 0x7ffu; }
+
+// x over the biased exponent es - kFixShift of the largest part; flip 0x80000000 negates
+__device__ __forceinline__ Limbs to_limbs(double x, uint32_t es, uint32_t flip) {
+  const uint32_t hi = (uint32_t)__double2hiint(x), lo = (uint32_t)__double2loint(x);
+  const uint32_t mh = __funnelshift_l(lo, hi, 11) | 0x80000000u, ml = lo << 11;
+  const uint32_t s = es - ((hi >> 20) & 0x7ffu);  // a zero's is above 63
+  unsigned long long f;
+  asm("shr.u64 %0, %1, %2;" : "=l"(f) : "l"(((unsigned long long)mh << 32) | ml), "r"(s));  // shifts above 63 give 0
+  const int32_t sign = ((int32_t)(hi ^ flip) >> 31) | 1;
+  return Limbs{(int32_t)(uint32_t)(f >> 31) * sign, (int32_t)((uint32_t)f & 0x7fffffffu) * sign};
+}
+
+__device__ __forceinline__ long long asr64(long long v, uint32_t s) {
+  long long r;
+  asm("shr.s64 %0, %1, %2;" : "=l"(r) : "l"(v), "r"(s));  // shifts above 63 give the sign
+  return r;
+}
+
+// T as a double, rounded to nearest even: the result's biased exponent is e + 1 - clz(|T|); T = 0 gives +0
+__device__ __forceinline__ double from_fix(long long T, int e) {
+  const uint32_t sg = (uint32_t)((unsigned long long)T >> 63);
+  const unsigned long long m0 = (unsigned long long)(T < 0 ? -T : T);
+  const int z = __clzll((long long)m0);
+  const unsigned long long m = m0 << (z & 63);
+  unsigned long long q = m >> 11;
+  const uint32_t rem = (uint32_t)m & 0x7ffu;
+  q += (rem + ((uint32_t)q & 1u)) > 0x400u ? 1ull : 0ull;
+  const uint32_t qh = (uint32_t)(q >> 32) + ((uint32_t)(e - z) << 20) + (sg << 31);
+  return m0 ? __hiloint2double((int)qh, (int)(uint32_t)q) : 0.0;
+}
+
+// One link as limbs, in the order in which the hop multiplies (backward: conjugate transposed; the
+// boundary sign included), and the exponent of its largest part.
+template <int N>
+struct FixLink {
+  int4 u[N * N];  // re.hi, re.lo, im.hi, im.lo
+  uint32_t e;
+};
+
+template <int N>
+__device__ __forceinline__ FixLink<N> load_fix_link(const DslashArgs& A, const SiteXyzt& X, int h, uint32_t nb) {
+  const int mu = h >> 1;
+  const bool bwd = h & 1;
+  const uint32_t vh = (uint32_t)A.geo.vh, p = (uint32_t)A.parity;
+  const double2* lb = static_cast<const double2*>(A.gauge) +
+                      ((mu * 2u + (bwd ? 1u - p : p)) * (uint32_t)(N * N) * vh + (bwd ? nb : X.site));
+  const uint32_t sa = (bwd ? 1u : (uint32_t)N) * vh, sb = (bwd ? (uint32_t)N : 1u) * vh;
+  double2 u[N][N];
+  FixLink<N> L;
+  L.e = 0;
+#pragma unroll
+  for (int a = 0; a < N; a++)
+#pragma unroll
+    for (int b = 0; b < N; b++) u[a][b] = __ldg(lb + (a * sa + b * sb));
+#pragma unroll
+  for (int a = 0; a < N; a++)
+#pragma unroll
+    for (int b = 0; b < N; b++) L.e = max(L.e, max(biased_exp(u[a][b].x), biased_exp(u[a][b].y)));
+  const bool wrap = mu == 3 && A.antiperiodic_t && (bwd ? X.t == 0 : X.t == (uint32_t)A.geo.L[3] - 1);
+  const uint32_t rf = wrap ? 0x80000000u : 0u, jf = rf ^ (bwd ? 0x80000000u : 0u);
+#pragma unroll
+  for (int a = 0; a < N; a++)
+#pragma unroll
+    for (int b = 0; b < N; b++) {
+      const Limbs r = to_limbs(u[a][b].x, L.e + kFixShift, rf), i = to_limbs(u[a][b].y, L.e + kFixShift, jf);
+      L.u[a * N + b] = make_int4(r.hi, r.lo, i.hi, i.lo);
+    }
+  return L;
+}
+
+// Links of a block's sites in shared memory, converted once for all the RHS of a site (in each thread the
+// conversion was a third of the instructions: SU(3) 24^3x48 nrhs 12 3140 us, with 24 parts a hop converted
+// instead of the 12 projected ones, against 1770): [site][hop] records of the N^2 elements (int4), their
+// negated imaginary parts (int2), and the exponent
+template <int N>
+constexpr uint32_t kFixRec = N * N + N * N / 2 + 1;
+template <int N>
+constexpr uint32_t kFixSite = (8 * kFixRec<N>) | 1;  // int4; odd, so that two sites' records lie in other banks
+
+// the FP64 multiply-adds, out of line: predicated FP64 operations would hold the pipe in every warp
+template <int N>
+__device__ __noinline__ void fp64_site(const DslashArgs& A, const SiteXyzt& X, uint32_t rhs) {
+  site_rhs<PREC_DOUBLE, N, 1, false, false>(A, X, rhs, 0, 1);
+}
+
+// the sums of one site and RHS
+template <int N>
+struct FixAcc {
+  long long up[2][N][2];  // rows 0 and 1
+  long long lo[2][N][2];  // the rows that take the products of rows 0 and 1 (3 and 2 for x and y, 2 and 3 for z and t)
+  int E = 0, Emin = 8191;
+  bool bad = false;
+};
+
+// Hop h (IM: x or z, whose gamma is imaginary) into S.
+template <int N, bool SHARED, bool IM>
+__device__ __forceinline__ void fix_hop_into(FixAcc<N>& S, const DslashArgs& A, const SiteXyzt& X, uint32_t rhs,
+                                             const int4* links, int h) {
+  const int mu = h >> 1;
+  const bool bwd = h & 1;
+  const uint32_t nrhs = (uint32_t)A.nrhs;
+  const double2* __restrict__ in = static_cast<const double2*>(A.in);
+  const uint32_t cs_bytes = (uint32_t)A.geo.vh * nrhs * 16u;
+  const uint32_t nb = X.neighbour(A, h);
+
+  // the neighbour's spinor; rows 2 and 3 in the order in which rows 0 and 1 meet them
+  double2 x[2][N], y[2][N];
+  {
+    const char* base = reinterpret_cast<const char*>(in + (nb * nrhs + rhs));
+    const char* low = base + (uint64_t)(2 * N) * cs_bytes;
+    const uint64_t up = (uint64_t)N * cs_bytes, r0 = mu < 2 ? up : 0u, r1 = up - r0;
+#pragma unroll
+    for (int a = 0; a < N; a++) {
+      x[0][a] = __ldg(reinterpret_cast<const double2*>(base + (uint64_t)a * cs_bytes));
+      x[1][a] = __ldg(reinterpret_cast<const double2*>(base + (uint64_t)(N + a) * cs_bytes));
+      y[0][a] = __ldg(reinterpret_cast<const double2*>(low + r0 + (uint64_t)a * cs_bytes));
+      y[1][a] = __ldg(reinterpret_cast<const double2*>(low + r1 + (uint64_t)a * cs_bytes));
+    }
+  }
+  FixLink<SHARED ? 1 : N> own;
+  const int4* rec = links + h * kFixRec<N>;
+  uint32_t eu;
+  if constexpr (SHARED) {
+    eu = (uint32_t)reinterpret_cast<const int2*>(rec + N * N)[N * N].x;
+  } else {
+    own = load_fix_link<N>(A, X, h, nb);
+    eu = own.e;
+  }
+
+  // h_u = x_u + s g(u) y_u, into x
+  const uint32_t sgn = (bwd != (A.dagger != 0)) ? 0u : 0x80000000u;  // s = +1 / -1
+  const double k0 = __hiloint2double((int)(0x3ff00000u | (sgn ^ (mu == 1 ? 0x80000000u : 0u))), 0);
+  const double k1 = __hiloint2double((int)(0x3ff00000u | (sgn ^ (mu == 2 ? 0x80000000u : 0u))), 0);
+  uint32_t ep = 0, mn = 0xffffffffu;  // exponents: largest; smallest of the non-zero parts, less one
+#pragma unroll
+  for (int i = 0; i < 2; i++)
+#pragma unroll
+    for (int a = 0; a < N; a++) {
+      const double k = i ? k1 : k0;
+      x[i][a].x = fma(IM ? -k : k, IM ? y[i][a].y : y[i][a].x, x[i][a].x);
+      x[i][a].y = fma(k, IM ? y[i][a].x : y[i][a].y, x[i][a].y);
+      const uint32_t q0 = biased_exp(x[i][a].x), q1 = biased_exp(x[i][a].y);
+      ep = max(ep, max(q0, q1));
+      mn = min(mn, min(q0 - 1u, q1 - 1u));
+    }
+  S.bad |= ep == 0x7ffu || eu == 0x7ffu || eu < 200u;
+  int eh = (int)(ep + eu);
+  S.Emin = min(S.Emin, (int)min(mn, 4095u) + 1 + (int)eu);
+  uint32_t es = ep + kFixShift;
+  if (ep == 0) {  // zeros add nothing; subnormal parts: FP64
+    long long any = 0;
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+#pragma unroll
+      for (int a = 0; a < N; a++) any |= __double_as_longlong(x[i][a].x) | __double_as_longlong(x[i][a].y);
+    S.bad |= (any << 1) != 0;
+    eh = 0;
+    es = 64;
+  }
+  Limbs hr[2][N], hi[2][N];
+#pragma unroll
+  for (int i = 0; i < 2; i++)
+#pragma unroll
+    for (int a = 0; a < N; a++) {
+      hr[i][a] = to_limbs(x[i][a].x, es, 0u);
+      hi[i][a] = to_limbs(x[i][a].y, es, 0u);
+    }
+
+  // bring the sums so far and this hop to the larger exponent
+  if (eh > S.E) {
+    const uint32_t d = (uint32_t)(eh - S.E);
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+#pragma unroll
+      for (int a = 0; a < N; a++)
+#pragma unroll
+        for (int c = 0; c < 2; c++) {
+          S.up[i][a][c] = asr64(S.up[i][a][c], d);
+          S.lo[i][a][c] = asr64(S.lo[i][a][c], d);
+        }
+    S.E = eh;
+  }
+  const uint32_t dT = (uint32_t)(S.E - eh);
+
+  // lower rows: lo(u) += s g(u_perm) (im ? i : 1) t_u
+  const uint32_t g0 = sgn ^ (mu == 3 ? 0u : 0x80000000u), g1 = sgn ^ (mu == 0 ? 0x80000000u : 0u);
+#pragma unroll
+  for (int a = 0; a < N; a++) {
+    long long H[2][2], M[2][2];
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+#pragma unroll
+      for (int c = 0; c < 2; c++) H[i][c] = 0, M[i][c] = 1ll << 30;
+#pragma unroll
+    for (int b = 0; b < N; b++) {
+      int4 u;
+      int2 n;  // the negated imaginary part
+      if constexpr (SHARED) {
+        u = rec[a * N + b];
+        n = reinterpret_cast<const int2*>(rec + N * N)[a * N + b];
+      } else {
+        u = own.u[a * N + b];
+        n = make_int2(-u.z, -u.w);
+      }
+#pragma unroll
+      for (int i = 0; i < 2; i++) {
+        const Limbs re = hr[i][b], im = hi[i][b];
+        H[i][0] += (long long)u.x * re.hi;
+        M[i][0] += (long long)u.x * re.lo;
+        M[i][0] += (long long)u.y * re.hi;
+        H[i][0] += (long long)n.x * im.hi;
+        M[i][0] += (long long)n.x * im.lo;
+        M[i][0] += (long long)n.y * im.hi;
+        H[i][1] += (long long)u.x * im.hi;
+        M[i][1] += (long long)u.x * im.lo;
+        M[i][1] += (long long)u.y * im.hi;
+        H[i][1] += (long long)u.z * re.hi;
+        M[i][1] += (long long)u.z * re.lo;
+        M[i][1] += (long long)u.w * re.hi;
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+      long long t[2];
+#pragma unroll
+      for (int c = 0; c < 2; c++) {
+        t[c] = asr64(H[i][c] + (M[i][c] >> 31), dT);
+        S.up[i][a][c] += t[c];
+      }
+      const long long m = (long long)(int32_t)(i ? g1 : g0) >> 31;  // 0 or -1
+      if constexpr (IM) {
+        S.lo[i][a][0] -= (t[1] ^ m) - m;
+        S.lo[i][a][1] += (t[0] ^ m) - m;
+      } else {
+        S.lo[i][a][0] += (t[0] ^ m) - m;
+        S.lo[i][a][1] += (t[1] ^ m) - m;
+      }
+    }
+  }
+}
+
+// links: the site's records in shared memory (SHARED)
+template <int N, bool SHARED>
+__device__ __forceinline__ void fix_site(const DslashArgs& A, const SiteXyzt& X, uint32_t rhs, const int4* links) {
+  prefetch_x<PREC_DOUBLE, N, 1>(A, X.site, rhs);
+  FixAcc<N> S;
+#pragma unroll
+  for (int i = 0; i < 2; i++)
+#pragma unroll
+    for (int a = 0; a < N; a++) S.up[i][a][0] = S.up[i][a][1] = S.lo[i][a][0] = S.lo[i][a][1] = 0;
+  // two hop bodies (imaginary and real gamma) run four times each: eight of them would not fit the
+  // instruction cache
+#pragma unroll 1
+  for (int j = 0; j < 2; j++) {
+#pragma unroll 1
+    for (int b = 0; b < 2; b++) fix_hop_into<N, SHARED, true>(S, A, X, rhs, links, 4 * j + b);
+#pragma unroll 1
+    for (int b = 0; b < 2; b++) fix_hop_into<N, SHARED, false>(S, A, X, rhs, links, 4 * j + 2 + b);
+    if (j == 0) {
+#pragma unroll
+      for (int a = 0; a < N; a++)
+#pragma unroll
+        for (int c = 0; c < 2; c++) {
+          const long long v = S.lo[0][a][c];
+          S.lo[0][a][c] = S.lo[1][a][c];
+          S.lo[1][a][c] = v;
+        }
+    }
+  }
+
+  if (S.bad || (S.E != 0 && (S.E < 1100 || S.E > 3000 || S.E - S.Emin > kFixSpan))) {
+    fp64_site<N>(A, X, rhs);
+    return;
+  }
+  C2<double> out[4][N][1];
+  const int e = S.E - 1015;
+#pragma unroll
+  for (int i = 0; i < 2; i++)
+#pragma unroll
+    for (int a = 0; a < N; a++) {
+      out[i][a][0].x = from_fix(S.up[i][a][0], e);
+      out[i][a][0].y = from_fix(S.up[i][a][1], e);
+      out[2 + i][a][0].x = from_fix(S.lo[i][a][0], e);
+      out[2 + i][a][0].y = from_fix(S.lo[i][a][1], e);
+    }
+  store_out<PREC_DOUBLE, N, 1>(out, A, X.site, rhs);
+}
+
+// Sites whose links a block of `block` threads holds in shared memory (0: each thread converts its own).
+// Below four RHS groups a site's conversion is shared by too few threads to pay for its round trip.
+template <int N>
+__host__ __device__ constexpr uint32_t fix_shared_sites(uint32_t groups, uint32_t block) {
+  const uint32_t n = (block - 1) / groups + 2;
+  return groups >= 4 && n * kFixSite<N> * 16u <= 48u * 1024u ? n : 0;
+}
+
+// The block's threads gid0 .. gid0 + blockDim.x - 1 of a launch, R right-hand sides each.
+template <int N, int R>
+__device__ __forceinline__ void fix_block(const DslashArgs& A, uint32_t gid0) {
+  extern __shared__ int4 fix_smem[];
+  const uint32_t groups = A.div_groups.d, vh = (uint32_t)A.geo.vh;
+  const uint32_t ns = fix_shared_sites<N>(groups, blockDim.x);
+  uint32_t first, grp, site;
+  A.div_groups.divmod(gid0, first, grp);
+  if (ns) {
+    for (uint32_t i = threadIdx.x; i < 8u * ns; i += blockDim.x) {
+      const uint32_t h = i / ns, k = i - h * ns;
+      if (first + k >= vh) continue;
+      const SiteXyzt X = decode_site(A, first + k);
+      const FixLink<N> L = load_fix_link<N>(A, X, (int)h, X.neighbour(A, (int)h));
+      int4* d = fix_smem + (k * kFixSite<N> + h * kFixRec<N>);
+#pragma unroll
+      for (int c = 0; c < N * N; c++) {
+        d[c] = L.u[c];
+        reinterpret_cast<int2*>(d + N * N)[c] = make_int2(-L.u[c].z, -L.u[c].w);
+      }
+      reinterpret_cast<int2*>(d + N * N)[N * N] = make_int2((int)L.e, 0);
+    }
+    __syncthreads();
+  }
+  A.div_groups.divmod(gid0 + threadIdx.x, site, grp);
+  if (site >= vh) return;
+  const SiteXyzt X = decode_site(A, site);
+#pragma unroll 1
+  for (int r = 0; r < R; r++) {
+    const uint32_t rhs = grp * R + r;
+    if (A.mask && !A.mask[rhs]) continue;
+    if (ns)
+      fix_site<N, true>(A, X, rhs, fix_smem + (site - first) * kFixSite<N>);
+    else
+      fix_site<N, false>(A, X, rhs, nullptr);
+  }
+}
+
+}  // namespace detail
+}  // namespace qcu

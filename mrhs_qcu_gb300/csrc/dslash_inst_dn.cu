@@ -6,6 +6,8 @@ namespace {
 struct Register_dn {
   Register_dn() {
     register_dslash(PREC_DOUBLE, 4, 1, 1, 0, &launch_wilson_mrhs<PREC_DOUBLE, 4, 1, 1, false>);
+    register_dslash(PREC_DOUBLE, 4, 1, 2, 0, &launch_wilson_mrhs<PREC_DOUBLE, 4, 1, 2, false>);
+    register_dslash(PREC_DOUBLE, 4, 1, 7, 0, &launch_wilson_mrhs<PREC_DOUBLE, 4, 1, 7, false>);
     register_dslash(PREC_DOUBLE, 4, 2, 1, 0, &launch_wilson_mrhs<PREC_DOUBLE, 4, 2, 1, false>);
     register_dslash(PREC_DOUBLE, 5, 1, 1, 0, &launch_wilson_mrhs<PREC_DOUBLE, 5, 1, 1, false>);
     register_dslash(PREC_DOUBLE, 6, 1, 1, 0, &launch_wilson_mrhs<PREC_DOUBLE, 6, 1, 1, false>);

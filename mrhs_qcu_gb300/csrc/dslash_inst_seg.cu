@@ -16,7 +16,6 @@ struct RegisterSegments {
     reg<PREC_SINGLE, 3, 2, 2, false, false>();
     reg<PREC_SINGLE, 3, 1, 1, false, false>();
     reg<PREC_SINGLE, 4, 2, 1, false, false>();
-    reg<PREC_DOUBLE, 3, 1, 1, false, true>();
     reg<PREC_DOUBLE, 3, 1, 1, false, false>();
     reg<PREC_BF16, 3, 2, 2, true, true>();
   }

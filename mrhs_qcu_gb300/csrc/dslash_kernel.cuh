@@ -22,6 +22,7 @@
 // coefficients.
 #pragma once
 
+#include <algorithm>
 #include <type_traits>
 
 #include "qcu_common.cuh"
@@ -732,55 +733,86 @@ __device__ __forceinline__ void store_out(C2<typename Store<P>::real> (&acc)[4][
 
 // MINB: register-cap variant of the kernel (registers per thread, and with
 // them the resident warps per SM, against spills):
-//   1: no cap (255), 2: 128, 3: 85, 4: 112, 5: 96, 6: 104.
+//   1: no cap (255), 2: 128, 3: 85, 4: 112, 5: 96, 6: 104, 7: 168.
 // 2 and 3 are the caps of 2 and 3 resident 256-thread blocks per SM.
 template <int MINB>
 struct RegCap {
   static constexpr int regs =
-      MINB == 2 ? 128 : MINB == 3 ? 85 : MINB == 4 ? 112 : MINB == 5 ? 96 : MINB == 6 ? 104 : 255;
+      MINB == 2 ? 128 : MINB == 3 ? 85 : MINB == 4 ? 112 : MINB == 5 ? 96 : MINB == 6 ? 104 : MINB == 7 ? 168 : 255;
 };
 
 namespace detail {
 
-// The work of one thread of the register kernel: output site x R RHS number
-// gid of the launch (gid = site * G + RHS group).
+// the xpay field's lines into L2 while the hops run (each line by one of the lanes that share it)
+template <int P, int N, int R>
+__device__ __forceinline__ void prefetch_x(const DslashArgs& A, uint32_t site, uint32_t rhs0) {
+  using E = typename Store<P>::elem;
+  if (!A.x) return;
+  constexpr uint32_t kLanes = 128u / (R * sizeof(E)) < 32u ? 128u / (R * sizeof(E)) : 32u;
+  const E* x = static_cast<const E*>(A.x) + (site * (uint32_t)A.nrhs + rhs0);
+#pragma unroll
+  for (uint32_t c = 0; c < 4u * N; c += kLanes) {
+    const uint32_t k = c + (threadIdx.x & (kLanes - 1u));
+    if (k < 4u * N) prefetch_l2(x + k * ((uint32_t)A.geo.vh * (uint32_t)A.nrhs));
+  }
+}
+
+// One output site: its index on the output parity and its coordinates.
+struct SiteXyzt {
+  uint32_t site, xh, y, z, t;
+  // the input-parity site of hop h: X+, X-, Y+, Y-, Z+, Z-, T+, T-
+  __device__ __forceinline__ uint32_t neighbour(const DslashArgs& A, int h) const {
+    const uint32_t hx = A.geo.hx, Ly = A.geo.L[1], Lz = A.geo.L[2], Lt = A.geo.L[3];
+    const uint32_t pl = A.geo.plane, cb = A.geo.cube, p = A.parity, eo = (y + z + t) & 1u;
+    switch (h) {
+      case 0: return (eo != p) ? (xh == hx - 1 ? site - (hx - 1) : site + 1) : site;
+      case 1: return (eo == p) ? (xh == 0 ? site + (hx - 1) : site - 1) : site;
+      case 2: return (y == Ly - 1) ? site - (Ly - 1) * hx : site + hx;
+      case 3: return (y == 0) ? site + (Ly - 1) * hx : site - hx;
+      case 4: return (z == Lz - 1) ? site - (Lz - 1) * pl : site + pl;
+      case 5: return (z == 0) ? site + (Lz - 1) * pl : site - pl;
+      case 6: return (t == Lt - 1) ? site - (Lt - 1) * cb : site + cb;
+      default: return (t == 0) ? site + (Lt - 1) * cb : site - cb;
+    }
+  }
+};
+
+// the site-th site of the launch's order
+__device__ __forceinline__ SiteXyzt decode_site(const DslashArgs& A, uint32_t site) {
+  SiteXyzt X;
+  if (A.zb) {  // slab order: (slab, t, z in slab, y, x)
+    uint32_t q, r, q2, zz, slab;
+    A.div_plane.divmod(site, q, r);
+    A.div_zb.divmod(q, q2, zz);
+    A.div_lt.divmod(q2, slab, X.t);
+    X.z = slab * A.zb + zz;
+    A.geo.div_hx.divmod(r, X.y, X.xh);
+    site = (X.t * (uint32_t)A.geo.L[2] + X.z) * (uint32_t)A.geo.plane + r;
+  } else {
+    uint32_t rest, rest2;
+    A.geo.div_hx.divmod(site, rest, X.xh);
+    A.geo.div_y.divmod(rest, rest2, X.y);
+    A.geo.div_z.divmod(rest2, X.t, X.z);
+  }
+  X.site = site;
+  return X;
+}
+
+// The work of one thread of the register kernel: output site X x R RHS from
+// rhs0 on; grp of `groups` among the threads of the site.
 // PK: FP32 arithmetic on the packed FP32x2 pipe, two RHS per packed register
 // (FP32 / 16-bit storage, even R).
 // RC: SU(3) links read as their first two rows (gauge12), the third reconstructed.
 template <int P, int N, int R, bool PK, bool RC>
-__device__ __forceinline__ void wilson_site(const DslashArgs& A, uint32_t gid) {
+__device__ __forceinline__ void site_rhs(const DslashArgs& A, const SiteXyzt& X, uint32_t rhs0, uint32_t grp,
+                                         uint32_t groups) {
   using S = Store<P>;
   using T = typename S::real;
   using E = typename S::elem;
   static_assert(!PK || sizeof(T) == 4, "packed arithmetic is FP32 only");
   static_assert(!PK || R % 2 == 0, "packed arithmetic pairs the RHS of a thread");
 
-  uint32_t site, grp;
-  A.div_groups.divmod(gid, site, grp);
-  if (site >= (uint32_t)A.geo.vh) return;
-  uint32_t xh, y, z, t;
-  const uint32_t rhs0 = grp * R;
-  if (A.mask) {
-    bool any = false;
-#pragma unroll
-    for (int r = 0; r < R; r++) any |= A.mask[rhs0 + r] != 0;
-    if (!any) return;
-  }
-
-  if (A.zb) {  // the site-th site of the slab order: (slab, t, z in slab, y, x)
-    uint32_t q, r, q2, zz, slab;
-    A.div_plane.divmod(site, q, r);
-    A.div_zb.divmod(q, q2, zz);
-    A.div_lt.divmod(q2, slab, t);
-    z = slab * A.zb + zz;
-    A.geo.div_hx.divmod(r, y, xh);
-    site = (t * (uint32_t)A.geo.L[2] + z) * (uint32_t)A.geo.plane + r;
-  } else {
-    uint32_t rest, rest2;
-    A.geo.div_hx.divmod(site, rest, xh);
-    A.geo.div_y.divmod(rest, rest2, y);
-    A.geo.div_z.divmod(rest2, t, z);
-  }
+  const uint32_t site = X.site, xh = X.xh, y = X.y, z = X.z, t = X.t;
   const uint32_t hx = A.geo.hx, Ly = A.geo.L[1], Lz = A.geo.L[2], Lt = A.geo.L[3];
   const uint32_t p = A.parity;
   const uint32_t eo = (y + z + t) & 1u;
@@ -790,17 +822,7 @@ __device__ __forceinline__ void wilson_site(const DslashArgs& A, uint32_t gid) {
   const E* __restrict__ gauge = static_cast<const E*>(RC ? A.gauge12 : A.gauge);
   constexpr uint32_t NN = RC ? (N - 1) * N : N * N;  // stored components per link
 
-  // the xpay field's lines into L2 while the hops run (each line by one of the lanes that share it)
-  if (A.x) {
-    constexpr uint32_t kLanes = 128u / (R * sizeof(E)) < 32u ? 128u / (R * sizeof(E)) : 32u;
-    const E* x = static_cast<const E*>(A.x) + (site * (uint32_t)A.nrhs + rhs0);
-#pragma unroll
-    for (uint32_t c = 0; c < 4u * N; c += kLanes) {
-      const uint32_t k = c + (threadIdx.x & (kLanes - 1u));
-      if (k < 4u * N) prefetch_l2(x + k * (vh * (uint32_t)A.nrhs));
-    }
-  }
-
+  prefetch_x<P, N, R>(A, site, rhs0);
   HopAcc<T, N, R, PK> hacc;
   hacc.zero();
 
@@ -814,9 +836,10 @@ __device__ __forceinline__ void wilson_site(const DslashArgs& A, uint32_t gid) {
   const uint32_t lb = (1u - p) * NN * lvh;
   const uint32_t dmu = 2 * NN * lvh;  // one direction's links
   // FP32 and BF16 storage prefetch every hop's links (below; measured 4-19%
-  // faster).  FP64 is bound by its FMA pipe and FP16 (with its norm loads)
-  // measured 2-6% slower with the prefetch, so they run the hops without it,
-  // in the form that compiles best for them.
+  // faster).  FP64 (here SU(5) and up, and the sites that dslash_fix.cuh leaves)
+  // is bound by its FMA pipe and FP16 (with its norm loads) measured 2-6% slower
+  // with the prefetch, so they run the hops without it, in the form that
+  // compiles best for them.
   if constexpr (P == PREC_SINGLE || P == PREC_BF16) {
     const uint32_t pl = A.geo.plane, cb = A.geo.cube;
     const bool top = t == Lt - 1, bot = t == 0;
@@ -837,7 +860,7 @@ __device__ __forceinline__ void wilson_site(const DslashArgs& A, uint32_t gid) {
     // Prefetching all eight into L1 here, with no registers held, leaves the
     // hops waiting only on their neighbour spinors (mostly L2 hits); the
     // R-groups of a site split the link components between them.
-    for (uint32_t k = grp; k < NN; k += A.div_groups.d) {
+    for (uint32_t k = grp; k < NN; k += groups) {
 #pragma unroll
       for (int h = 0; h < 8; h++)
         prefetch_l1(gauge + ((h >> 1) * dmu + ((h & 1) ? lb + lsite(nbr(h)) : lf) + k * lcs));
@@ -893,10 +916,51 @@ __device__ __forceinline__ void wilson_site(const DslashArgs& A, uint32_t gid) {
 }
 
 }  // namespace detail
+}  // namespace qcu
+
+#include "dslash_fix.cuh"
+
+namespace qcu {
+namespace detail {
+
+// thread gid of the launch: gid = site * G + RHS group
+template <int P, int N, int R, bool PK, bool RC>
+__device__ __forceinline__ void wilson_site(const DslashArgs& A, uint32_t gid) {
+  uint32_t site, grp;
+  A.div_groups.divmod(gid, site, grp);
+  if (site >= (uint32_t)A.geo.vh) return;
+  const uint32_t rhs0 = grp * R;
+  if (A.mask) {
+    bool any = false;
+#pragma unroll
+    for (int r = 0; r < R; r++) any |= A.mask[rhs0 + r] != 0;
+    if (!any) return;
+  }
+  const SiteXyzt X = decode_site(A, site);
+  site_rhs<P, N, R, PK, RC>(A, X, rhs0, grp, A.div_groups.d);
+}
+
+// block `blk` of a launch
+template <int P, int N, int R, bool PK, bool RC>
+__device__ __forceinline__ void wilson_block(const DslashArgs& A, uint32_t blk) {
+  if constexpr (fix_hop(P, N) && !RC)
+    fix_block<N, R>(A, blk * blockDim.x);
+  else
+    wilson_site<P, N, R, PK, RC>(A, blk * blockDim.x + threadIdx.x);
+}
+
+// dynamic shared memory of that block
+template <int P, int N, bool RC>
+size_t wilson_smem(uint32_t groups, int block) {
+  if constexpr (fix_hop(P, N) && !RC) return (size_t)fix_shared_sites<N>(groups, (uint32_t)block) * kFixSite<N> * 16;
+  return 0;
+}
+
+}  // namespace detail
 
 template <int P, int N, int R, int MINB, bool PK, bool RC = false>
-__global__ void __maxnreg__(RegCap<MINB>::regs) wilson_mrhs_kernel(const DslashArgs A) {
-  detail::wilson_site<P, N, R, PK, RC>(A, blockIdx.x * blockDim.x + threadIdx.x);
+__global__ void __maxnreg__(RegCap<MINB>::regs) wilson_mrhs_kernel(const __grid_constant__ DslashArgs A) {
+  detail::wilson_block<P, N, R, PK, RC>(A, blockIdx.x);
 }
 
 // host-side launcher of one instantiation
@@ -905,7 +969,8 @@ void launch_wilson_mrhs(const DslashArgs& A, int block, cudaStream_t stream) {
   const int groups = A.nrhs / R;
   const int64_t threads = (int64_t)A.geo.vh * groups;
   const int grid = (int)((threads + block - 1) / block);
-  wilson_mrhs_kernel<P, N, R, MINB, PK, RC><<<grid, block, 0, stream>>>(A);
+  const size_t smem = detail::wilson_smem<P, N, RC>((uint32_t)groups, block);
+  wilson_mrhs_kernel<P, N, R, MINB, PK, RC><<<grid, block, smem, stream>>>(A);
 }
 
 // One launch over a work list of up to kMaxHopSegments segments: each
@@ -927,7 +992,7 @@ __global__ void __maxnreg__(RegCap<MINB>::regs) wilson_segments_kernel(const __g
   int s = 0;
 #pragma unroll 1
   while (s + 1 < S.count && blockIdx.x >= S.block_begin[s + 1]) s++;
-  detail::wilson_site<P, N, R, PK, RC>(S.A[s], (blockIdx.x - S.block_begin[s]) * blockDim.x + threadIdx.x);
+  detail::wilson_block<P, N, R, PK, RC>(S.A[s], blockIdx.x - S.block_begin[s]);
 }
 
 // the segments' div_groups must be set (nrhs / R); fills block_begin
@@ -940,7 +1005,9 @@ void launch_wilson_segments(HopSegments& S, int block, cudaStream_t stream) {
     total += (uint32_t)((threads + block - 1) / block);
   }
   S.block_begin[S.count] = total;
-  wilson_segments_kernel<P, N, R, MINB, PK, RC><<<total, block, 0, stream>>>(S);
+  size_t smem = 0;
+  for (int s = 0; s < S.count; s++) smem = std::max(smem, detail::wilson_smem<P, N, RC>((uint32_t)(S.A[s].nrhs / R), block));
+  wilson_segments_kernel<P, N, R, MINB, PK, RC><<<total, block, smem, stream>>>(S);
 }
 
 }  // namespace qcu

@@ -321,13 +321,13 @@ const void* Session::gauge12(int prec) {
   QCU_REQUIRE(gauge_loaded_, QCU_ERR_NO_GAUGE, "localGauge_ is nullptr, not loaded.\n");
   QCU_REQUIRE(prec_valid(prec), QCU_ERR_INVALID_ARGUMENT, "bad precision");
   if (prec == PREC_BF16S) prec = PREC_BF16;
-  if (N != 3) return nullptr;
+  if (N != 3 || prec == PREC_DOUBLE) return nullptr;  // the fixed-point FP64 hop takes the full links
   if (su3_dev_ < 0) {
     unsigned* scratch = static_cast<unsigned*>(su3_scratch_.ensure(16));
     su3_dev_ = su3_row_deviation(gauge_[PREC_DOUBLE].get(), geo.vh, scratch, stream());
   }
   // a reconstructed row must agree with the stored one to the rounding of the precision
-  const double tol = prec == PREC_DOUBLE ? 1e-13 : (prec == PREC_SINGLE ? 1e-7 : 1e-4);
+  const double tol = prec == PREC_SINGLE ? 1e-7 : 1e-4;
   if (!(su3_dev_ < tol)) return nullptr;
   if (!gauge12_valid_[prec]) {
     const size_t vhp = ((size_t)geo.vh + 31) / 32 * 32;  // the two-row layout's groups of 32 sites
