@@ -146,12 +146,24 @@ struct FixAcc {
   bool bad = false;
 };
 
-// Hop h (IM: x or z, whose gamma is imaginary) into S.
-template <int N, bool SHARED, bool IM>
-__device__ __forceinline__ void fix_hop_into(FixAcc<N>& S, const DslashArgs& A, const SiteXyzt& X, uint32_t rhs,
-                                             const int4* links, int h) {
+// s = +1 / -1 of hop h as a sign bit, and the sign s g(u_perm) with which the product of row i enters the lower row
+__device__ __forceinline__ uint32_t fix_sign(const DslashArgs& A, int h) {
+  return ((h & 1) != (A.dagger != 0)) ? 0u : 0x80000000u;
+}
+__device__ __forceinline__ long long fix_lower_sign(const DslashArgs& A, int h, int i) {  // 0 or -1
   const int mu = h >> 1;
-  const bool bwd = h & 1;
+  const uint32_t g = fix_sign(A, h) ^ ((i ? mu == 0 : mu != 3) ? 0x80000000u : 0u);
+  return (long long)(int32_t)g >> 31;
+}
+
+// Hop h: out.begin(exponent, smallest exponent, not for fixed point), then out.put(a, i, re, im) for the
+// products of colour a and projected row i in the hop's own unit.  IM: the gamma is imaginary (x, z) or not,
+// 2 = as h says.
+template <int N, bool SHARED, int IM, typename Out>
+__device__ __forceinline__ void fix_hop_products(Out& out, const DslashArgs& A, const SiteXyzt& X, uint32_t rhs,
+                                                 const int4* links, int h) {
+  const int mu = h >> 1;
+  const bool imag = IM == 2 ? !(mu & 1) : IM == 1;
   const uint32_t nrhs = (uint32_t)A.nrhs;
   const double2* __restrict__ in = static_cast<const double2*>(A.in);
   const uint32_t cs_bytes = (uint32_t)A.geo.vh * nrhs * 16u;
@@ -182,7 +194,7 @@ __device__ __forceinline__ void fix_hop_into(FixAcc<N>& S, const DslashArgs& A, 
   }
 
   // h_u = x_u + s g(u) y_u, into x
-  const uint32_t sgn = (bwd != (A.dagger != 0)) ? 0u : 0x80000000u;  // s = +1 / -1
+  const uint32_t sgn = fix_sign(A, h);
   const double k0 = __hiloint2double((int)(0x3ff00000u | (sgn ^ (mu == 1 ? 0x80000000u : 0u))), 0);
   const double k1 = __hiloint2double((int)(0x3ff00000u | (sgn ^ (mu == 2 ? 0x80000000u : 0u))), 0);
   uint32_t ep = 0, mn = 0xffffffffu;  // exponents: largest; smallest of the non-zero parts, less one
@@ -191,15 +203,14 @@ __device__ __forceinline__ void fix_hop_into(FixAcc<N>& S, const DslashArgs& A, 
 #pragma unroll
     for (int a = 0; a < N; a++) {
       const double k = i ? k1 : k0;
-      x[i][a].x = fma(IM ? -k : k, IM ? y[i][a].y : y[i][a].x, x[i][a].x);
-      x[i][a].y = fma(k, IM ? y[i][a].x : y[i][a].y, x[i][a].y);
+      x[i][a].x = fma(imag ? -k : k, imag ? y[i][a].y : y[i][a].x, x[i][a].x);
+      x[i][a].y = fma(k, imag ? y[i][a].x : y[i][a].y, x[i][a].y);
       const uint32_t q0 = biased_exp(x[i][a].x), q1 = biased_exp(x[i][a].y);
       ep = max(ep, max(q0, q1));
       mn = min(mn, min(q0 - 1u, q1 - 1u));
     }
-  S.bad |= ep == 0x7ffu || eu == 0x7ffu || eu < 200u;
+  bool bad = ep == 0x7ffu || eu == 0x7ffu || eu < 200u;
   int eh = (int)(ep + eu);
-  S.Emin = min(S.Emin, (int)min(mn, 4095u) + 1 + (int)eu);
   uint32_t es = ep + kFixShift;
   if (ep == 0) {  // zeros add nothing; subnormal parts: FP64
     long long any = 0;
@@ -207,7 +218,7 @@ __device__ __forceinline__ void fix_hop_into(FixAcc<N>& S, const DslashArgs& A, 
     for (int i = 0; i < 2; i++)
 #pragma unroll
       for (int a = 0; a < N; a++) any |= __double_as_longlong(x[i][a].x) | __double_as_longlong(x[i][a].y);
-    S.bad |= (any << 1) != 0;
+    bad |= (any << 1) != 0;
     eh = 0;
     es = 64;
   }
@@ -220,24 +231,8 @@ __device__ __forceinline__ void fix_hop_into(FixAcc<N>& S, const DslashArgs& A, 
       hi[i][a] = to_limbs(x[i][a].y, es, 0u);
     }
 
-  // bring the sums so far and this hop to the larger exponent
-  if (eh > S.E) {
-    const uint32_t d = (uint32_t)(eh - S.E);
-#pragma unroll
-    for (int i = 0; i < 2; i++)
-#pragma unroll
-      for (int a = 0; a < N; a++)
-#pragma unroll
-        for (int c = 0; c < 2; c++) {
-          S.up[i][a][c] = asr64(S.up[i][a][c], d);
-          S.lo[i][a][c] = asr64(S.lo[i][a][c], d);
-        }
-    S.E = eh;
-  }
-  const uint32_t dT = (uint32_t)(S.E - eh);
+  out.begin(eh, (int)min(mn, 4095u) + 1 + (int)eu, bad);
 
-  // lower rows: lo(u) += s g(u_perm) (im ? i : 1) t_u
-  const uint32_t g0 = sgn ^ (mu == 3 ? 0u : 0x80000000u), g1 = sgn ^ (mu == 0 ? 0x80000000u : 0u);
 #pragma unroll
   for (int a = 0; a < N; a++) {
     long long H[2][2], M[2][2];
@@ -274,23 +269,61 @@ __device__ __forceinline__ void fix_hop_into(FixAcc<N>& S, const DslashArgs& A, 
       }
     }
 #pragma unroll
-    for (int i = 0; i < 2; i++) {
-      long long t[2];
+    for (int i = 0; i < 2; i++) out.put(a, i, H[i][0] + (M[i][0] >> 31), H[i][1] + (M[i][1] >> 31));
+  }
+}
+
+// hop h added to a site's sums
+template <int N, int IM>
+struct FixAdd {
+  FixAcc<N>& S;
+  const DslashArgs& A;
+  int h;
+  uint32_t d = 0;  // the hop's shift to the sums' exponent
+  // brings the sums so far and this hop to the larger exponent
+  __device__ __forceinline__ void begin(int eh, int emin, bool bad) {
+    S.bad |= bad;
+    S.Emin = min(S.Emin, emin);
+    if (eh > S.E) {
+      const uint32_t up = (uint32_t)(eh - S.E);
 #pragma unroll
-      for (int c = 0; c < 2; c++) {
-        t[c] = asr64(H[i][c] + (M[i][c] >> 31), dT);
-        S.up[i][a][c] += t[c];
-      }
-      const long long m = (long long)(int32_t)(i ? g1 : g0) >> 31;  // 0 or -1
-      if constexpr (IM) {
-        S.lo[i][a][0] -= (t[1] ^ m) - m;
-        S.lo[i][a][1] += (t[0] ^ m) - m;
-      } else {
-        S.lo[i][a][0] += (t[0] ^ m) - m;
-        S.lo[i][a][1] += (t[1] ^ m) - m;
-      }
+      for (int i = 0; i < 2; i++)
+#pragma unroll
+        for (int a = 0; a < N; a++)
+#pragma unroll
+          for (int c = 0; c < 2; c++) {
+            S.up[i][a][c] = asr64(S.up[i][a][c], up);
+            S.lo[i][a][c] = asr64(S.lo[i][a][c], up);
+          }
+      S.E = eh;
+    }
+    d = (uint32_t)(S.E - eh);
+  }
+  // lower rows: lo(u) += s g(u_perm) (im ? i : 1) t_u
+  __device__ __forceinline__ void put(int a, int i, long long re, long long im) {
+    const long long t0 = asr64(re, d), t1 = asr64(im, d), m = fix_lower_sign(A, h, i);
+    S.up[i][a][0] += t0;
+    S.up[i][a][1] += t1;
+    if constexpr (IM) {
+      S.lo[i][a][0] -= (t1 ^ m) - m;
+      S.lo[i][a][1] += (t0 ^ m) - m;
+    } else {
+      S.lo[i][a][0] += (t0 ^ m) - m;
+      S.lo[i][a][1] += (t1 ^ m) - m;
     }
   }
+};
+
+template <int N, bool SHARED, int IM>
+__device__ __forceinline__ void fix_hop_into(FixAcc<N>& S, const DslashArgs& A, const SiteXyzt& X, uint32_t rhs,
+                                             const int4* links, int h) {
+  FixAdd<N, IM> add{S, A, h};
+  fix_hop_products<N, SHARED, IM>(add, A, X, rhs, links, h);
+}
+
+// whether a site's sums hold: E, Emin the largest and smallest exponents of its hops
+__device__ __forceinline__ bool fix_holds(bool bad, int E, int Emin) {
+  return !bad && (E == 0 || (E >= 1100 && E <= 3000 && E - Emin <= kFixSpan));
 }
 
 // links: the site's records in shared memory (SHARED)
@@ -307,9 +340,9 @@ __device__ __forceinline__ void fix_site(const DslashArgs& A, const SiteXyzt& X,
 #pragma unroll 1
   for (int j = 0; j < 2; j++) {
 #pragma unroll 1
-    for (int b = 0; b < 2; b++) fix_hop_into<N, SHARED, true>(S, A, X, rhs, links, 4 * j + b);
+    for (int b = 0; b < 2; b++) fix_hop_into<N, SHARED, 1>(S, A, X, rhs, links, 4 * j + b);
 #pragma unroll 1
-    for (int b = 0; b < 2; b++) fix_hop_into<N, SHARED, false>(S, A, X, rhs, links, 4 * j + 2 + b);
+    for (int b = 0; b < 2; b++) fix_hop_into<N, SHARED, 0>(S, A, X, rhs, links, 4 * j + 2 + b);
     if (j == 0) {
 #pragma unroll
       for (int a = 0; a < N; a++)
@@ -322,7 +355,7 @@ __device__ __forceinline__ void fix_site(const DslashArgs& A, const SiteXyzt& X,
     }
   }
 
-  if (S.bad || (S.E != 0 && (S.E < 1100 || S.E > 3000 || S.E - S.Emin > kFixSpan))) {
+  if (!fix_holds(S.bad, S.E, S.Emin)) {
     fp64_site<N>(A, X, rhs);
     return;
   }
@@ -383,6 +416,114 @@ __device__ __forceinline__ void fix_block(const DslashArgs& A, uint32_t gid0) {
       fix_site<N, true>(A, X, rhs, fix_smem + (site - first) * kFixSite<N>);
     else
       fix_site<N, false>(A, X, rhs, nullptr);
+  }
+}
+
+// The same site and RHS on eight threads, one a hop: thread h * U + u of a block of 8 U does hop h of the
+// block's u-th site and RHS, leaves its products in shared memory, and sums and stores the components h and
+// h + 8 (complex parts).  The sums take the hops in the same order and by the same shifts, so the result is
+// the same to the bit.  For launches with about a warp a scheduler, whose time is one thread's chain of
+// hops; where the GPU is full, the exchange and the links converted by every thread cost more.  One
+// thread a site and RHS / eight, us: SU(3) 8^4 nrhs 1 22 / 7.6, nrhs 4 22 / 11.7, 12^3x24 nrhs 1 27 / 19,
+// 14x10x6x18 nrhs 5 27 / 29, 24^3x48 nrhs 12 1723 / 2369; SU(4) 8^4 nrhs 2 37 / 10.7.  The autotuner
+// times both.
+template <int N>
+constexpr uint32_t kFixSplitUnit = 8 * (4 * N * 8 + 8);  // bytes of a site and RHS
+
+template <int N>
+struct FixShare {
+  long long* v;  // [4 N][U] of this hop: part (2 i N + 2 a + c)
+  int2* e;       // exponent, smallest exponent
+  uint32_t U;
+  static constexpr int kBad = -(1 << 20);
+  __device__ __forceinline__ void begin(int eh, int emin, bool bad) { *e = make_int2(eh, bad ? kBad : emin); }
+  __device__ __forceinline__ void put(int a, int i, long long re, long long im) {
+    v[(2 * (i * N + a)) * U] = re;
+    v[(2 * (i * N + a) + 1) * U] = im;
+  }
+};
+
+template <int N>
+__device__ __forceinline__ void fix_split_block(const DslashArgs& A, uint32_t blk) {
+  extern __shared__ int4 fix_smem[];
+  const uint32_t U = blockDim.x / 8, h = threadIdx.x / U, u = threadIdx.x - h * U;
+  long long* vals = reinterpret_cast<long long*>(fix_smem);
+  int2* exps = reinterpret_cast<int2*>(vals + 8 * 4 * N * U);
+  const uint32_t vh = (uint32_t)A.geo.vh, nrhs = (uint32_t)A.nrhs, cs = vh * nrhs;
+  uint32_t site, rhs;
+  A.div_groups.divmod(blk * U + u, site, rhs);
+  const bool live = site < vh && (!A.mask || A.mask[rhs]);
+  const SiteXyzt X = decode_site(A, live ? site : 0);
+  const uint32_t o = X.site * nrhs + rhs;
+  constexpr int K = (4 * N + 7) / 8;
+  double2 xv[K];
+  if (live) {
+    if (A.x) {
+#pragma unroll
+      for (int k = 0; k < K; k++)
+        if (h + 8 * k < 4 * N) xv[k] = __ldg(static_cast<const double2*>(A.x) + (o + (h + 8 * k) * cs));
+    }
+    FixShare<N> share{vals + (h * 4 * N * U + u), exps + (h * U + u), U};
+    fix_hop_products<N, false, 2>(share, A, X, rhs, nullptr, (int)h);
+  }
+  __syncthreads();
+  if (!live) return;
+
+  int E = 0, Emin = 8191;
+#pragma unroll
+  for (int g = 0; g < 8; g++) {
+    const int2 e = exps[g * U + u];
+    E = max(E, e.x);
+    Emin = min(Emin, e.y);
+  }
+  if (!fix_holds(Emin <= FixShare<N>::kBad, E, Emin)) {
+    if (h == 0) fp64_site<N>(A, X, rhs);
+    return;
+  }
+  const double ca = A.a_rhs_d ? A.a_rhs_d[rhs] : A.a;
+#pragma unroll
+  for (int k = 0; k < K; k++) {
+    const uint32_t comp = h + 8 * k;
+    if (comp >= 4 * N) break;
+    const int row = (int)comp / N, a = (int)comp - row * N;
+    long long s0 = 0, s1 = 0;
+    int Es = 0;
+#pragma unroll
+    for (int g = 0; g < 8; g++) {
+      const int mu = g >> 1, eg = exps[g * U + u].x;
+      if (eg > Es) {
+        s0 = asr64(s0, (uint32_t)(eg - Es));
+        s1 = asr64(s1, (uint32_t)(eg - Es));
+        Es = eg;
+      }
+      const int i = row < 2 ? row : mu < 2 ? 3 - row : row - 2;  // the projected row that feeds this one
+      const long long* v = vals + ((g * 4 * N + 2 * (i * N + a)) * U + u);
+      const long long t0 = asr64(v[0], (uint32_t)(Es - eg)), t1 = asr64(v[U], (uint32_t)(Es - eg));
+      if (row < 2) {
+        s0 += t0;
+        s1 += t1;
+      } else {
+        const long long m = fix_lower_sign(A, g, i);
+        if (!(mu & 1)) {
+          s0 -= (t1 ^ m) - m;
+          s1 += (t0 ^ m) - m;
+        } else {
+          s0 += (t0 ^ m) - m;
+          s1 += (t1 ^ m) - m;
+        }
+      }
+    }
+    double2 r = make_double2(from_fix(s0, Es - 1015), from_fix(s1, Es - 1015));
+    // store_out's operations
+    if (A.x) {
+      if (A.b == 1.0)
+        r = make_double2(fma(ca, r.x, xv[k].x), fma(ca, r.y, xv[k].y));
+      else
+        r = make_double2(fma(A.b, xv[k].x, ca * r.x), fma(A.b, xv[k].y, ca * r.y));
+    } else if (A.a_rhs_d || A.a != 1.0) {
+      r = make_double2(r.x * ca, r.y * ca);
+    }
+    static_cast<double2*>(A.out)[o + comp * cs] = r;
   }
 }
 

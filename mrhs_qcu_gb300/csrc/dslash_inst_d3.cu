@@ -8,6 +8,8 @@ struct Register_d3 {
     register_dslash(PREC_DOUBLE, 3, 1, 1, 0, &launch_wilson_mrhs<PREC_DOUBLE, 3, 1, 1, false>);
     register_dslash(PREC_DOUBLE, 3, 1, 2, 0, &launch_wilson_mrhs<PREC_DOUBLE, 3, 1, 2, false>);
     register_dslash(PREC_DOUBLE, 3, 1, 7, 0, &launch_wilson_mrhs<PREC_DOUBLE, 3, 1, 7, false>);
+    register_dslash(PREC_DOUBLE, 3, 1, 2, 1, &launch_wilson_mrhs<PREC_DOUBLE, 3, 1, 2, true>);
+    register_dslash(PREC_DOUBLE, 3, 1, 7, 1, &launch_wilson_mrhs<PREC_DOUBLE, 3, 1, 7, true>);
     register_dslash(PREC_DOUBLE, 3, 2, 1, 0, &launch_wilson_mrhs<PREC_DOUBLE, 3, 2, 1, false>);
     register_dslash(PREC_DOUBLE, 3, 3, 1, 0, &launch_wilson_mrhs<PREC_DOUBLE, 3, 3, 1, false>);
     register_dslash(PREC_DOUBLE, 3, 4, 1, 0, &launch_wilson_mrhs<PREC_DOUBLE, 3, 4, 1, false>);

@@ -17,6 +17,7 @@ struct RegisterSegments {
     reg<PREC_SINGLE, 3, 1, 1, false, false>();
     reg<PREC_SINGLE, 4, 2, 1, false, false>();
     reg<PREC_DOUBLE, 3, 1, 1, false, false>();
+    reg<PREC_DOUBLE, 3, 1, 2, true, false>();
     reg<PREC_BF16, 3, 2, 2, true, true>();
   }
 } register_segments_at_load;

@@ -940,19 +940,35 @@ __device__ __forceinline__ void wilson_site(const DslashArgs& A, uint32_t gid) {
   site_rhs<P, N, R, PK, RC>(A, X, rhs0, grp, A.div_groups.d);
 }
 
+// threads per site and group of R RHS: 8 in the split form of the fixed-point hop (PK at FP64)
+template <int P, int N, bool PK, bool RC>
+constexpr int kSiteThreads = fix_hop(P, N) && !RC && PK ? 8 : 1;
+
 // block `blk` of a launch
 template <int P, int N, int R, bool PK, bool RC>
 __device__ __forceinline__ void wilson_block(const DslashArgs& A, uint32_t blk) {
-  if constexpr (fix_hop(P, N) && !RC)
+  if constexpr (kSiteThreads<P, N, PK, RC> == 8) {
+    static_assert(R == 1, "one RHS per eight threads");
+    fix_split_block<N>(A, blk);
+  } else if constexpr (fix_hop(P, N) && !RC) {
     fix_block<N, R>(A, blk * blockDim.x);
-  else
+  } else {
     wilson_site<P, N, R, PK, RC>(A, blk * blockDim.x + threadIdx.x);
+  }
 }
 
-// dynamic shared memory of that block
-template <int P, int N, bool RC>
+// blocks of a launch, and dynamic shared memory of a block
+template <int P, int N, bool PK, bool RC>
+uint32_t wilson_blocks(const DslashArgs& A, int R, int block) {
+  const int64_t threads = (int64_t)A.geo.vh * (A.nrhs / R) * kSiteThreads<P, N, PK, RC>;
+  return (uint32_t)((threads + block - 1) / block);
+}
+template <int P, int N, bool PK, bool RC>
 size_t wilson_smem(uint32_t groups, int block) {
-  if constexpr (fix_hop(P, N) && !RC) return (size_t)fix_shared_sites<N>(groups, (uint32_t)block) * kFixSite<N> * 16;
+  if constexpr (kSiteThreads<P, N, PK, RC> == 8)
+    return (size_t)(block / 8) * kFixSplitUnit<N>;
+  else if constexpr (fix_hop(P, N) && !RC)
+    return (size_t)fix_shared_sites<N>(groups, (uint32_t)block) * kFixSite<N> * 16;
   return 0;
 }
 
@@ -967,9 +983,8 @@ __global__ void __maxnreg__(RegCap<MINB>::regs) wilson_mrhs_kernel(const __grid_
 template <int P, int N, int R, int MINB, bool PK = false, bool RC = false>
 void launch_wilson_mrhs(const DslashArgs& A, int block, cudaStream_t stream) {
   const int groups = A.nrhs / R;
-  const int64_t threads = (int64_t)A.geo.vh * groups;
-  const int grid = (int)((threads + block - 1) / block);
-  const size_t smem = detail::wilson_smem<P, N, RC>((uint32_t)groups, block);
+  const uint32_t grid = detail::wilson_blocks<P, N, PK, RC>(A, R, block);
+  const size_t smem = detail::wilson_smem<P, N, PK, RC>((uint32_t)groups, block);
   wilson_mrhs_kernel<P, N, R, MINB, PK, RC><<<grid, block, smem, stream>>>(A);
 }
 
@@ -1001,12 +1016,12 @@ void launch_wilson_segments(HopSegments& S, int block, cudaStream_t stream) {
   uint32_t total = 0;
   for (int s = 0; s < S.count; s++) {
     S.block_begin[s] = total;
-    const int64_t threads = (int64_t)S.A[s].geo.vh * (S.A[s].nrhs / R);
-    total += (uint32_t)((threads + block - 1) / block);
+    total += detail::wilson_blocks<P, N, PK, RC>(S.A[s], R, block);
   }
   S.block_begin[S.count] = total;
   size_t smem = 0;
-  for (int s = 0; s < S.count; s++) smem = std::max(smem, detail::wilson_smem<P, N, RC>((uint32_t)(S.A[s].nrhs / R), block));
+  for (int s = 0; s < S.count; s++)
+    smem = std::max(smem, detail::wilson_smem<P, N, PK, RC>((uint32_t)(S.A[s].nrhs / R), block));
   wilson_segments_kernel<P, N, R, MINB, PK, RC><<<total, block, smem, stream>>>(S);
 }
 

@@ -127,3 +127,31 @@ def test_not_finite(cuda, qcu_lib, bad):
     hit = ~np.isfinite(O.dslash(psi, g, L, 0, 0)).all(axis=(2, 3))
     assert np.array_equal(~np.isfinite(got).all(axis=(2, 3)), hit) and 0 < hit.sum() <= 8
     assert np.array_equal(got[~hit], clean[~hit])
+
+
+@pytest.mark.parametrize("n,L,nrhs", [(3, (4, 4, 4, 4), 1), (3, (6, 4, 2, 4), 5), (3, (4, 2, 2, 6), 12), (4, (6, 2, 2, 4), 3),
+                                      (4, (4, 4, 4, 4), 8)])
+def test_eight_threads_a_site(cuda, qcu_lib, n, L, nrhs):
+    """The split form is the other form bit for bit: every block size, sites that take FP64 among them, a
+    partial last block."""
+    g = S.random_gauge(L, n, seed=41)
+    psi = S.random_fermions(L, n, nrhs, seed=42)
+    psi[0, 1] *= 2.0 ** -45      # its neighbours span too much
+    psi[nrhs - 1, 4, 2, 1] = np.inf
+    psi[0, 6] = 0
+    for parity, dagger in ((0, 0), (1, 1)):
+        out = {}
+        for pk, minb in ((0, 1), (1, 2), (1, 7)):
+            for block in (32, 64, 128, 256):
+                os.environ["QCU_DSLASH_CONFIG"] = "1,%d,%d,%d,0" % (block, minb, pk)
+                try:
+                    out[pk, minb, block] = abi_dslash(cuda, qcu_lib, psi, g, L, parity, dagger, 2, antiperiodic_t=True)
+                    assert qcu_lib.last_dslash_shape()[2] == pk
+                finally:
+                    del os.environ["QCU_DSLASH_CONFIG"]
+        base = out[0, 1, 32]
+        want = O.dslash(psi, g, L, parity, dagger, True)
+        ok = np.isfinite(want).all(axis=(2, 3))
+        assert rel(base[ok], want[ok]) < 1e-15
+        for got in out.values():
+            assert np.array_equal(got, base, equal_nan=True)
