@@ -50,7 +50,7 @@ __device__ __forceinline__ void st(float2* p, double2 v) { *p = Store<PREC_SINGL
 // FP64 sum of FP32 products in groups of four.  One conversion and FP64
 // addition per product is bound by the FP64 pipe (2 lanes a cycle and SM, and
 // the conversion issues there too): the norm of 24^3x48 SU(3) nrhs 12 FP32
-// took 195 us against 56 us of HBM time.  So the products of a group are added in
+// took 195 us against 56 us of HBM time (75 now).  So the products of a group are added in
 // FP32 with their rounding errors kept (Knuth's TwoSum), and two values go to
 // FP64.  A group that leaves FP32's range, or is not finite, is added product
 // by product (a call: as predicated instructions it would hold the FP64 pipe).
@@ -165,6 +165,13 @@ __device__ __forceinline__ double2 add_mul(double2 a, double2 x, double2 y) {
 __device__ __forceinline__ void coeff(double2 a, float2& c) { c = tof(a); }
 __device__ __forceinline__ void coeff(double2 a, double2& c) { c = a; }
 
+// dynamic shared memory of the reducing kernels: R values of each thread (reduce_bytes)
+template <typename A>
+__device__ __forceinline__ A* reduce_smem() {
+  extern __shared__ double2 blas_smem[];
+  return reinterpret_cast<A*>(blas_smem);
+}
+
 // block-level per-RHS reduction of `vals` (R values per thread) into
 // out[blockIdx.x * nrhs + r]
 template <typename A>
@@ -268,8 +275,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1) axpby_kernel(const double2* __
     }
   }
   if (NORM) {
-    __shared__ double sm[1024 * 2];
-    block_reduce<double>(sm, acc, R, s.G, s.nrhs, partials);
+    block_reduce<double>(reduce_smem<double>(), acc, R, s.G, s.nrhs, partials);
   }
 }
 
@@ -377,8 +383,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1) reduce_kernel(const void* __re
     }
     double acc[R];
     totals(acc, sum);
-    __shared__ double sm[1024 * 2];
-    block_reduce<double>(sm, acc, R, s.G, s.nrhs, static_cast<double*>(partials));
+    block_reduce<double>(reduce_smem<double>(), acc, R, s.G, s.nrhs, static_cast<double*>(partials));
   } else {
     static_assert(PX == PY, "one precision");
     DotSum<PS> sum[R];
@@ -401,8 +406,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1) reduce_kernel(const void* __re
     }
     double2 acc[R];
     totals(acc, sum);
-    __shared__ double2 sm2[1024 * 2];
-    block_reduce<double2>(sm2, acc, R, s.G, s.nrhs, static_cast<double2*>(partials));
+    block_reduce<double2>(reduce_smem<double2>(), acc, R, s.G, s.nrhs, static_cast<double2*>(partials));
   }
 }
 
@@ -462,10 +466,9 @@ __global__ void __launch_bounds__(kMaxThreads, 1) cg_update_kernel(const double2
   double accs[R], accr[R];
   totals(accs, sums);
   totals(accr, sumr);
-  __shared__ double sm[1024 * 2];
-  block_reduce<double>(sm, accs, R, sh.G, sh.nrhs, part);
+  block_reduce<double>(reduce_smem<double>(), accs, R, sh.G, sh.nrhs, part);
   __syncthreads();
-  block_reduce<double>(sm, accr, R, sh.G, sh.nrhs, part2);
+  block_reduce<double>(reduce_smem<double>(), accr, R, sh.G, sh.nrhs, part2);
 }
 
 // x += a p, p = r + b p (a and b real)
@@ -536,10 +539,9 @@ __global__ void __launch_bounds__(kMaxThreads, 1) dot_norm_kernel(const void* __
   double accn[R];
   totals(accd, dot);
   totals(accn, nrm);
-  __shared__ double2 sm[1024 * 2];
-  block_reduce<double2>(sm, accd, R, sh.G, sh.nrhs, part2);
+  block_reduce<double2>(reduce_smem<double2>(), accd, R, sh.G, sh.nrhs, part2);
   __syncthreads();
-  block_reduce<double>(reinterpret_cast<double*>(sm), accn, R, sh.G, sh.nrhs, part);
+  block_reduce<double>(reduce_smem<double>(), accn, R, sh.G, sh.nrhs, part);
 }
 
 // x += a p + o s, s -= o t; partial |s|^2 (part) and <r0, s> (part2)
@@ -598,10 +600,9 @@ __global__ void __launch_bounds__(kMaxThreads, 1) bicg_update_kernel(const doubl
   double accn[R];
   totals(accd, dot);
   totals(accn, nrm);
-  __shared__ double2 sm[1024 * 2];
-  block_reduce<double2>(sm, accd, R, sh.G, sh.nrhs, part2);
+  block_reduce<double2>(reduce_smem<double2>(), accd, R, sh.G, sh.nrhs, part2);
   __syncthreads();
-  block_reduce<double>(reinterpret_cast<double*>(sm), accn, R, sh.G, sh.nrhs, part);
+  block_reduce<double>(reduce_smem<double>(), accn, R, sh.G, sh.nrhs, part);
 }
 
 // ---- masked moves between fields of selected RHS (no arithmetic on the others) ----
@@ -668,8 +669,7 @@ __global__ void residual_kernel(const int* __restrict__ sel, const double2* __re
         if (c + u * stride < sh.nchunks) st(y + c + u * stride, v[u]);
       }
     }
-  __shared__ double sm[1024];
-  block_reduce<double>(sm, acc, 1, sh.G, sh.nrhs, part);
+  block_reduce<double>(reduce_smem<double>(), acc, 1, sh.G, sh.nrhs, part);
 }
 
 // one warp per RHS: lane l sums the block partials l, l + 32, ... in order,
@@ -722,13 +722,38 @@ int pick_r(const FieldRef& f, const void* other = nullptr, const void* third = n
 int block_size(int G) {
   int b = G;
   while (b % 32) b += G;
-  while (b < 128 && b * 2 <= 1024) b *= 2;
+  while (b < 192 && b * 2 <= 1024) b *= 2;
   return b;
 }
 
 int grid_for(int64_t nchunks, int block) {
   int64_t g = (nchunks + block - 1) / block;
   return (int)std::max<int64_t>(1, std::min<int64_t>(g, kMaxBlocks));
+}
+
+int device_sms() {
+  static const int sms = [] {
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+      n = 0;
+    return n > 0 ? n : 152;
+  }();
+  return sms;
+}
+
+// Grid of a reducing kernel: one even wave.  1024 threads an SM always fit (at most 64 registers a thread,
+// 32 KB of shared memory), so every SM takes the same number of blocks at once.  1024 blocks of 128 threads
+// with 32 KB each made 1.12 waves of 6 blocks, and left the second half of the time to a tenth of the
+// blocks: at 16^3x32 SU(4) nrhs 16, us, before / now: BiCGStab update 274 / 158, <x, y> with |x|^2 119 / 89,
+// <x, y> 84 / 62.
+int reduce_grid(int64_t nchunks, int block) {
+  const int64_t g = (nchunks + block - 1) / block;
+  const int64_t wave = (int64_t)device_sms() * std::max(1, 1024 / block);
+  return (int)std::max<int64_t>(1, std::min<int64_t>(g, std::min<int64_t>(wave, kMaxBlocks)));
+}
+template <typename A>
+size_t reduce_bytes(int block, int R) {
+  return (size_t)block * R * sizeof(A);
 }
 
 void check_field(const FieldRef& f) {
@@ -773,14 +798,15 @@ void Blas::axpby_norm(const double2* a, const FieldRef& x, const double2* b, con
   Shape s = make_shape(x, R);
   const int B = block_size(s.G);
   QCU_REQUIRE(B <= 1024, QCU_ERR_UNSUPPORTED, "nrhs too large for BLAS block");
-  const int grid = grid_for(s.nchunks, B);
+  const int grid = reduce_grid(s.nchunks, B);
+  const size_t sm = reduce_bytes<double>(B, R);
   QCU_REQUIRE(grid <= max_blocks_, QCU_ERR_INVALID_ARGUMENT, "partials too small");
   if (x.prec == PREC_DOUBLE)
-    axpby_kernel<PREC_DOUBLE, PREC_DOUBLE, 1, true><<<grid, B, 0, st>>>(a, x.data, b, y.data, s, partials_);
+    axpby_kernel<PREC_DOUBLE, PREC_DOUBLE, 1, true><<<grid, B, sm, st>>>(a, x.data, b, y.data, s, partials_);
   else if (R == 2)
-    axpby_kernel<PREC_SINGLE, PREC_SINGLE, 2, true><<<grid, B, 0, st>>>(a, x.data, b, y.data, s, partials_);
+    axpby_kernel<PREC_SINGLE, PREC_SINGLE, 2, true><<<grid, B, sm, st>>>(a, x.data, b, y.data, s, partials_);
   else
-    axpby_kernel<PREC_SINGLE, PREC_SINGLE, 1, true><<<grid, B, 0, st>>>(a, x.data, b, y.data, s, partials_);
+    axpby_kernel<PREC_SINGLE, PREC_SINGLE, 1, true><<<grid, B, sm, st>>>(a, x.data, b, y.data, s, partials_);
   QCU_CHECK_CUDA(cudaGetLastError());
   finalize<double>(partials_, grid, x.nrhs, out, st);
   QCU_CHECK_CUDA(cudaGetLastError());
@@ -811,17 +837,18 @@ void Blas::norm2(const FieldRef& x, double* out, cudaStream_t st, bool exact) {
   Shape s = make_shape(x, R);
   const int B = block_size(s.G);
   QCU_REQUIRE(B <= 1024, QCU_ERR_UNSUPPORTED, "nrhs too large for BLAS block");
-  const int grid = grid_for(s.nchunks, B);
+  const int grid = reduce_grid(s.nchunks, B);
+  const size_t sm = reduce_bytes<double>(B, R);
   if (x.prec == PREC_DOUBLE)
-    reduce_kernel<PREC_DOUBLE, PREC_DOUBLE, 1, 0><<<grid, B, 0, st>>>(x.data, x.data, s, partials_);
+    reduce_kernel<PREC_DOUBLE, PREC_DOUBLE, 1, 0><<<grid, B, sm, st>>>(x.data, x.data, s, partials_);
   else if (R == 2 && exact)
-    reduce_kernel<PREC_SINGLE, PREC_SINGLE, 2, 0><<<grid, B, 0, st>>>(x.data, x.data, s, partials_);
+    reduce_kernel<PREC_SINGLE, PREC_SINGLE, 2, 0><<<grid, B, sm, st>>>(x.data, x.data, s, partials_);
   else if (R == 2)
-    reduce_kernel<PREC_SINGLE, PREC_SINGLE, 2, 0, true><<<grid, B, 0, st>>>(x.data, x.data, s, partials_);
+    reduce_kernel<PREC_SINGLE, PREC_SINGLE, 2, 0, true><<<grid, B, sm, st>>>(x.data, x.data, s, partials_);
   else if (exact)
-    reduce_kernel<PREC_SINGLE, PREC_SINGLE, 1, 0><<<grid, B, 0, st>>>(x.data, x.data, s, partials_);
+    reduce_kernel<PREC_SINGLE, PREC_SINGLE, 1, 0><<<grid, B, sm, st>>>(x.data, x.data, s, partials_);
   else
-    reduce_kernel<PREC_SINGLE, PREC_SINGLE, 1, 0, true><<<grid, B, 0, st>>>(x.data, x.data, s, partials_);
+    reduce_kernel<PREC_SINGLE, PREC_SINGLE, 1, 0, true><<<grid, B, sm, st>>>(x.data, x.data, s, partials_);
   QCU_CHECK_CUDA(cudaGetLastError());
   finalize<double>(partials_, grid, x.nrhs, out, st);
   QCU_CHECK_CUDA(cudaGetLastError());
@@ -836,14 +863,15 @@ void Blas::cdot(const FieldRef& x, const FieldRef& y, double2* out, cudaStream_t
   Shape s = make_shape(x, R);
   const int B = block_size(s.G);
   QCU_REQUIRE(B <= 1024, QCU_ERR_UNSUPPORTED, "nrhs too large for BLAS block");
-  const int grid = grid_for(s.nchunks, B);
+  const int grid = reduce_grid(s.nchunks, B);
+  const size_t sm = reduce_bytes<double2>(B, R);
   double2* p2 = reinterpret_cast<double2*>(partials_);
   if (x.prec == PREC_DOUBLE)
-    reduce_kernel<PREC_DOUBLE, PREC_DOUBLE, 1, 1><<<grid, B, 0, st>>>(x.data, y.data, s, p2);
+    reduce_kernel<PREC_DOUBLE, PREC_DOUBLE, 1, 1><<<grid, B, sm, st>>>(x.data, y.data, s, p2);
   else if (R == 2)
-    reduce_kernel<PREC_SINGLE, PREC_SINGLE, 2, 1, true><<<grid, B, 0, st>>>(x.data, y.data, s, p2);
+    reduce_kernel<PREC_SINGLE, PREC_SINGLE, 2, 1, true><<<grid, B, sm, st>>>(x.data, y.data, s, p2);
   else
-    reduce_kernel<PREC_SINGLE, PREC_SINGLE, 1, 1, true><<<grid, B, 0, st>>>(x.data, y.data, s, p2);
+    reduce_kernel<PREC_SINGLE, PREC_SINGLE, 1, 1, true><<<grid, B, sm, st>>>(x.data, y.data, s, p2);
   QCU_CHECK_CUDA(cudaGetLastError());
   finalize<double2>(p2, grid, x.nrhs, out, st);
   QCU_CHECK_CUDA(cudaGetLastError());
@@ -854,7 +882,9 @@ double* Blas::norms(int k) const { return partials_ + (size_t)(2 + k) * max_bloc
 namespace {
 struct Launch {
   Shape s;
-  int R, block, grid;
+  int R, block, grid;   // grid of a kernel without reductions
+  int rgrid;            // of a reducing kernel
+  size_t norm_sm, dot_sm;  // its shared memory
 };
 Launch plan(const FieldRef& f, int R) {
   Launch l;
@@ -863,6 +893,9 @@ Launch plan(const FieldRef& f, int R) {
   l.block = block_size(l.s.G);
   QCU_REQUIRE(l.block <= 1024, QCU_ERR_UNSUPPORTED, "nrhs too large for BLAS block");
   l.grid = grid_for(l.s.nchunks, l.block);
+  l.rgrid = reduce_grid(l.s.nchunks, l.block);
+  l.norm_sm = reduce_bytes<double>(l.block, R);
+  l.dot_sm = reduce_bytes<double2>(l.block, R);
   return l;
 }
 void check_same(const FieldRef& a, const FieldRef& b, const char* what) {
@@ -878,39 +911,39 @@ Partials Blas::norm2_partials(const FieldRef& x, cudaStream_t st) {
   const Launch l = plan(x, pick_r(x));
   double* p = norms(0);
   if (x.prec == PREC_DOUBLE)
-    reduce_kernel<PREC_DOUBLE, PREC_DOUBLE, 1, 0><<<l.grid, l.block, 0, st>>>(x.data, x.data, l.s, p);
+    reduce_kernel<PREC_DOUBLE, PREC_DOUBLE, 1, 0><<<l.rgrid, l.block, l.norm_sm, st>>>(x.data, x.data, l.s, p);
   else if (l.R == 2)
-    reduce_kernel<PREC_SINGLE, PREC_SINGLE, 2, 0, true><<<l.grid, l.block, 0, st>>>(x.data, x.data, l.s, p);
+    reduce_kernel<PREC_SINGLE, PREC_SINGLE, 2, 0, true><<<l.rgrid, l.block, l.norm_sm, st>>>(x.data, x.data, l.s, p);
   else
-    reduce_kernel<PREC_SINGLE, PREC_SINGLE, 1, 0, true><<<l.grid, l.block, 0, st>>>(x.data, x.data, l.s, p);
+    reduce_kernel<PREC_SINGLE, PREC_SINGLE, 1, 0, true><<<l.rgrid, l.block, l.norm_sm, st>>>(x.data, x.data, l.s, p);
   QCU_CHECK_CUDA(cudaGetLastError());
-  return Partials{p, nullptr, nullptr, l.grid};
+  return Partials{p, nullptr, nullptr, l.rgrid};
 }
 
 Partials Blas::dot_partials(const FieldRef& x, const FieldRef& y, cudaStream_t st) {
   check_same(x, y, "dot");
   const Launch l = plan(x, pick_r(x, y.data));
   if (x.prec == PREC_DOUBLE)
-    reduce_kernel<PREC_DOUBLE, PREC_DOUBLE, 1, 1><<<l.grid, l.block, 0, st>>>(x.data, y.data, l.s, dots());
+    reduce_kernel<PREC_DOUBLE, PREC_DOUBLE, 1, 1><<<l.rgrid, l.block, l.dot_sm, st>>>(x.data, y.data, l.s, dots());
   else if (l.R == 2)
-    reduce_kernel<PREC_SINGLE, PREC_SINGLE, 2, 1, true><<<l.grid, l.block, 0, st>>>(x.data, y.data, l.s, dots());
+    reduce_kernel<PREC_SINGLE, PREC_SINGLE, 2, 1, true><<<l.rgrid, l.block, l.dot_sm, st>>>(x.data, y.data, l.s, dots());
   else
-    reduce_kernel<PREC_SINGLE, PREC_SINGLE, 1, 1, true><<<l.grid, l.block, 0, st>>>(x.data, y.data, l.s, dots());
+    reduce_kernel<PREC_SINGLE, PREC_SINGLE, 1, 1, true><<<l.rgrid, l.block, l.dot_sm, st>>>(x.data, y.data, l.s, dots());
   QCU_CHECK_CUDA(cudaGetLastError());
-  return Partials{nullptr, nullptr, dots(), l.grid};
+  return Partials{nullptr, nullptr, dots(), l.rgrid};
 }
 
 Partials Blas::dot_norm(const FieldRef& x, const FieldRef& y, cudaStream_t st) {
   check_same(x, y, "dot_norm");
   const Launch l = plan(x, pick_r(x, y.data));
   if (x.prec == PREC_DOUBLE)
-    dot_norm_kernel<PREC_DOUBLE, 1><<<l.grid, l.block, 0, st>>>(x.data, y.data, l.s, norms(0), dots());
+    dot_norm_kernel<PREC_DOUBLE, 1><<<l.rgrid, l.block, l.dot_sm, st>>>(x.data, y.data, l.s, norms(0), dots());
   else if (l.R == 2)
-    dot_norm_kernel<PREC_SINGLE, 2><<<l.grid, l.block, 0, st>>>(x.data, y.data, l.s, norms(0), dots());
+    dot_norm_kernel<PREC_SINGLE, 2><<<l.rgrid, l.block, l.dot_sm, st>>>(x.data, y.data, l.s, norms(0), dots());
   else
-    dot_norm_kernel<PREC_SINGLE, 1><<<l.grid, l.block, 0, st>>>(x.data, y.data, l.s, norms(0), dots());
+    dot_norm_kernel<PREC_SINGLE, 1><<<l.rgrid, l.block, l.dot_sm, st>>>(x.data, y.data, l.s, norms(0), dots());
   QCU_CHECK_CUDA(cudaGetLastError());
-  return Partials{norms(0), nullptr, dots(), l.grid};
+  return Partials{norms(0), nullptr, dots(), l.rgrid};
 }
 
 Partials Blas::cg_update(const double2* a, const FieldRef& q, const FieldRef& s, const FieldRef& w, const FieldRef& r,
@@ -921,13 +954,13 @@ Partials Blas::cg_update(const double2* a, const FieldRef& q, const FieldRef& s,
   const int R = std::min(pick_r(q, s.data), pick_r(w, r.data));
   const Launch l = plan(q, R);
   if (q.prec == PREC_DOUBLE)
-    cg_update_kernel<PREC_DOUBLE, 1><<<l.grid, l.block, 0, st>>>(a, q.data, s.data, w.data, r.data, l.s, norms(0), norms(1));
+    cg_update_kernel<PREC_DOUBLE, 1><<<l.rgrid, l.block, l.norm_sm, st>>>(a, q.data, s.data, w.data, r.data, l.s, norms(0), norms(1));
   else if (R == 2)
-    cg_update_kernel<PREC_SINGLE, 2><<<l.grid, l.block, 0, st>>>(a, q.data, s.data, w.data, r.data, l.s, norms(0), norms(1));
+    cg_update_kernel<PREC_SINGLE, 2><<<l.rgrid, l.block, l.norm_sm, st>>>(a, q.data, s.data, w.data, r.data, l.s, norms(0), norms(1));
   else
-    cg_update_kernel<PREC_SINGLE, 1><<<l.grid, l.block, 0, st>>>(a, q.data, s.data, w.data, r.data, l.s, norms(0), norms(1));
+    cg_update_kernel<PREC_SINGLE, 1><<<l.rgrid, l.block, l.norm_sm, st>>>(a, q.data, s.data, w.data, r.data, l.s, norms(0), norms(1));
   QCU_CHECK_CUDA(cudaGetLastError());
-  return Partials{norms(0), norms(1), nullptr, l.grid};
+  return Partials{norms(0), norms(1), nullptr, l.rgrid};
 }
 
 void Blas::cg_direction(const double2* a, const double2* b, const FieldRef& r, const FieldRef& p, const FieldRef& x,
@@ -953,13 +986,13 @@ Partials Blas::bicg_update(const double2* a, const double2* o, const FieldRef& p
   const int R = std::min(pick_r(p, s.data, t.data), pick_r(r0, x.data));
   const Launch l = plan(p, R);
   if (p.prec == PREC_DOUBLE)
-    bicg_update_kernel<PREC_DOUBLE, 1><<<l.grid, l.block, 0, st>>>(a, o, p.data, s.data, t.data, r0.data, x.data, l.s, norms(0), dots());
+    bicg_update_kernel<PREC_DOUBLE, 1><<<l.rgrid, l.block, l.dot_sm, st>>>(a, o, p.data, s.data, t.data, r0.data, x.data, l.s, norms(0), dots());
   else if (R == 2)
-    bicg_update_kernel<PREC_SINGLE, 2><<<l.grid, l.block, 0, st>>>(a, o, p.data, s.data, t.data, r0.data, x.data, l.s, norms(0), dots());
+    bicg_update_kernel<PREC_SINGLE, 2><<<l.rgrid, l.block, l.dot_sm, st>>>(a, o, p.data, s.data, t.data, r0.data, x.data, l.s, norms(0), dots());
   else
-    bicg_update_kernel<PREC_SINGLE, 1><<<l.grid, l.block, 0, st>>>(a, o, p.data, s.data, t.data, r0.data, x.data, l.s, norms(0), dots());
+    bicg_update_kernel<PREC_SINGLE, 1><<<l.rgrid, l.block, l.dot_sm, st>>>(a, o, p.data, s.data, t.data, r0.data, x.data, l.s, norms(0), dots());
   QCU_CHECK_CUDA(cudaGetLastError());
-  return Partials{norms(0), nullptr, dots(), l.grid};
+  return Partials{norms(0), nullptr, dots(), l.rgrid};
 }
 
 // the masked moves keep one RHS per thread (R = 1), so a thread is selected or leaves at once
@@ -1001,11 +1034,11 @@ void Blas::residual(const int* sel, const FieldRef& x, const FieldRef& y, double
   const Launch l = plan(x, 1);
   const double2* xp = static_cast<const double2*>(x.data);
   if (y.prec == PREC_DOUBLE)
-    residual_kernel<PREC_DOUBLE><<<l.grid, l.block, 0, st>>>(sel, xp, y.data, l.s, norms(0));
+    residual_kernel<PREC_DOUBLE><<<l.rgrid, l.block, l.norm_sm, st>>>(sel, xp, y.data, l.s, norms(0));
   else
-    residual_kernel<PREC_SINGLE><<<l.grid, l.block, 0, st>>>(sel, xp, y.data, l.s, norms(0));
+    residual_kernel<PREC_SINGLE><<<l.rgrid, l.block, l.norm_sm, st>>>(sel, xp, y.data, l.s, norms(0));
   QCU_CHECK_CUDA(cudaGetLastError());
-  finalize<double>(norms(0), l.grid, x.nrhs, out, st);
+  finalize<double>(norms(0), l.rgrid, x.nrhs, out, st);
   QCU_CHECK_CUDA(cudaGetLastError());
 }
 

@@ -32,7 +32,14 @@ __device__ __forceinline__ double2 shfl_xor(double2 v, int off) {
 template <typename A>
 __device__ __forceinline__ A sum_partials(const A* __restrict__ partials, int nblocks, int nrhs, int r, int lane) {
   A s = A{};
-  for (int b = lane; b < nblocks; b += 32) s = s + partials[(int64_t)b * nrhs + r];
+  constexpr int U = 8;  // partials loaded together: their latency, not their sum, is the kernel's time
+  for (int b = lane; b < nblocks; b += 32 * U) {
+    A v[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) v[u] = b + 32 * u < nblocks ? partials[(int64_t)(b + 32 * u) * nrhs + r] : A{};
+#pragma unroll
+    for (int u = 0; u < U; u++) s = s + v[u];
+  }
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) s = s + shfl_xor(s, off);
   return s;
