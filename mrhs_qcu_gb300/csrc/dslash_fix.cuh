@@ -17,8 +17,8 @@
 // but by the right shifts to the accumulator's unit.  Relative L2 error against quad precision on random
 // fields: 0.84e-16, where the FP64 multiply-adds have 1.45e-16 (SU(3)) and 1.54e-16 (SU(4)).
 //
-// One hop, us, FP64 multiply-adds / this: SU(3) 24^3x48 nrhs 12 5826 / 1770, SU(4) 16^3x32 nrhs 16
-// 2480 / 736, SU(3) 14x10x6x18 nrhs 5 59 / 27, SU(3) 12^3x24 nrhs 1 44 / 27.  It is bound by instruction
+// One hop, us, FP64 multiply-adds / this: SU(3) 24^3x48 nrhs 12 5826 / 1685, SU(4) 16^3x32 nrhs 16
+// 2480 / 757, SU(3) 14x10x6x18 nrhs 5 59 / 27, SU(3) 12^3x24 nrhs 1 44 / 27.  It is bound by instruction
 // issue and latency (SU(3): 8300 instructions a warp, 216 wide multiply-adds a hop; the multiplier 53%
 // busy, the integer pipe 43%, FP64 33%, 12 or 16 warps an SM); the small sizes by the latency of one
 // warp a scheduler.
@@ -124,7 +124,7 @@ __device__ __forceinline__ FixLink<N> load_fix_link(const DslashArgs& A, const S
 
 // Links of a block's sites in shared memory, converted once for all the RHS of a site (in each thread the
 // conversion was a third of the instructions: SU(3) 24^3x48 nrhs 12 3140 us, with 24 parts a hop converted
-// instead of the 12 projected ones, against 1770): [site][hop] records of the N^2 elements (int4), their
+// instead of the 12 projected ones, against 1685): [site][hop] records of the N^2 elements (int4), their
 // negated imaginary parts (int2), and the exponent
 template <int N>
 constexpr uint32_t kFixRec = N * N + N * N / 2 + 1;
@@ -157,13 +157,12 @@ __device__ __forceinline__ long long fix_lower_sign(const DslashArgs& A, int h, 
 }
 
 // Hop h: out.begin(exponent, smallest exponent, not for fixed point), then out.put(a, i, re, im) for the
-// products of colour a and projected row i in the hop's own unit.  IM: the gamma is imaginary (x, z) or not,
-// 2 = as h says.
-template <int N, bool SHARED, int IM, typename Out>
+// products of colour a and projected row i in the hop's own unit.
+template <int N, bool SHARED, typename Out>
 __device__ __forceinline__ void fix_hop_products(Out& out, const DslashArgs& A, const SiteXyzt& X, uint32_t rhs,
                                                  const int4* links, int h) {
   const int mu = h >> 1;
-  const bool imag = IM == 2 ? !(mu & 1) : IM == 1;
+  const bool imag = !(mu & 1);
   const uint32_t nrhs = (uint32_t)A.nrhs;
   const double2* __restrict__ in = static_cast<const double2*>(A.in);
   const uint32_t cs_bytes = (uint32_t)A.geo.vh * nrhs * 16u;
@@ -274,7 +273,7 @@ __device__ __forceinline__ void fix_hop_products(Out& out, const DslashArgs& A, 
 }
 
 // hop h added to a site's sums
-template <int N, int IM>
+template <int N>
 struct FixAdd {
   FixAcc<N>& S;
   const DslashArgs& A;
@@ -304,21 +303,18 @@ struct FixAdd {
     const long long t0 = asr64(re, d), t1 = asr64(im, d), m = fix_lower_sign(A, h, i);
     S.up[i][a][0] += t0;
     S.up[i][a][1] += t1;
-    if constexpr (IM) {
-      S.lo[i][a][0] -= (t1 ^ m) - m;
-      S.lo[i][a][1] += (t0 ^ m) - m;
-    } else {
-      S.lo[i][a][0] += (t0 ^ m) - m;
-      S.lo[i][a][1] += (t1 ^ m) - m;
-    }
+    const bool imag = !((h >> 1) & 1);
+    const long long mr = m ^ (imag ? -1ll : 0ll);
+    S.lo[i][a][0] += ((imag ? t1 : t0) ^ mr) - mr;
+    S.lo[i][a][1] += ((imag ? t0 : t1) ^ m) - m;
   }
 };
 
-template <int N, bool SHARED, int IM>
+template <int N, bool SHARED>
 __device__ __forceinline__ void fix_hop_into(FixAcc<N>& S, const DslashArgs& A, const SiteXyzt& X, uint32_t rhs,
                                              const int4* links, int h) {
-  FixAdd<N, IM> add{S, A, h};
-  fix_hop_products<N, SHARED, IM>(add, A, X, rhs, links, h);
+  FixAdd<N> add{S, A, h};
+  fix_hop_products<N, SHARED>(add, A, X, rhs, links, h);
 }
 
 // whether a site's sums hold: E, Emin the largest and smallest exponents of its hops
@@ -335,15 +331,13 @@ __device__ __forceinline__ void fix_site(const DslashArgs& A, const SiteXyzt& X,
   for (int i = 0; i < 2; i++)
 #pragma unroll
     for (int a = 0; a < N; a++) S.up[i][a][0] = S.up[i][a][1] = S.lo[i][a][0] = S.lo[i][a][1] = 0;
-  // two hop bodies (imaginary and real gamma) run four times each: eight of them would not fit the
-  // instruction cache
+  // one hop body for all eight (its gamma chosen by selects): with a body each for the imaginary and the
+  // real gammas the instruction cache cost more than the selects, 1720 against 1685 us at SU(3) 24^3x48
+  // nrhs 12, and 914 against 772 at SU(4) 16^3x32 nrhs 16, 128 registers
 #pragma unroll 1
-  for (int j = 0; j < 2; j++) {
-#pragma unroll 1
-    for (int b = 0; b < 2; b++) fix_hop_into<N, SHARED, 1>(S, A, X, rhs, links, 4 * j + b);
-#pragma unroll 1
-    for (int b = 0; b < 2; b++) fix_hop_into<N, SHARED, 0>(S, A, X, rhs, links, 4 * j + 2 + b);
-    if (j == 0) {
+  for (int h = 0; h < 8; h++) {
+    fix_hop_into<N, SHARED>(S, A, X, rhs, links, h);
+    if (h == 3) {
 #pragma unroll
       for (int a = 0; a < N; a++)
 #pragma unroll
@@ -425,7 +419,7 @@ __device__ __forceinline__ void fix_block(const DslashArgs& A, uint32_t gid0) {
 // the same to the bit.  For launches with about a warp a scheduler, whose time is one thread's chain of
 // hops; where the GPU is full, the exchange and the links converted by every thread cost more.  One
 // thread a site and RHS / eight, us: SU(3) 8^4 nrhs 1 22 / 7.6, nrhs 4 22 / 11.7, 12^3x24 nrhs 1 27 / 19,
-// 14x10x6x18 nrhs 5 27 / 29, 24^3x48 nrhs 12 1723 / 2369; SU(4) 8^4 nrhs 2 37 / 10.7.  The autotuner
+// 14x10x6x18 nrhs 5 27 / 29, 24^3x48 nrhs 12 1685 / 2369; SU(4) 8^4 nrhs 2 37 / 10.7.  The autotuner
 // times both.
 template <int N>
 constexpr uint32_t kFixSplitUnit = 8 * (4 * N * 8 + 8);  // bytes of a site and RHS
@@ -464,7 +458,7 @@ __device__ __forceinline__ void fix_split_block(const DslashArgs& A, uint32_t bl
         if (h + 8 * k < 4 * N) xv[k] = __ldg(static_cast<const double2*>(A.x) + (o + (h + 8 * k) * cs));
     }
     FixShare<N> share{vals + (h * 4 * N * U + u), exps + (h * U + u), U};
-    fix_hop_products<N, false, 2>(share, A, X, rhs, nullptr, (int)h);
+    fix_hop_products<N, false>(share, A, X, rhs, nullptr, (int)h);
   }
   __syncthreads();
   if (!live) return;
