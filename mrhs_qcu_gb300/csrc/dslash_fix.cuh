@@ -1,4 +1,4 @@
-// FP64 Wilson hop of SU(3) and SU(4) with the colour multiply in block fixed point.
+// FP64 Wilson hop with the colour multiply in block fixed point.
 //
 // The FP64 pipe of sm_103a takes 2 multiply-adds per clock and SM, and 840 of them a site and RHS kept
 // it 97% busy at SU(3).  32 x 32 -> 64-bit integer multiply-adds run at about 16 times that rate.  So
@@ -15,16 +15,18 @@
 //
 // No sum can overflow (the bounds stand beside the constants), and none rounds before the last step
 // but by the right shifts to the accumulator's unit.  Relative L2 error against quad precision on random
-// fields: 0.84e-16, where the FP64 multiply-adds have 1.45e-16 (SU(3)) and 1.54e-16 (SU(4)).
+// fields: SU(3), SU(4) 0.84e-16, SU(5) to SU(8) 1.20e-16 to 1.24e-16, where the FP64 multiply-adds have
+// 1.45e-16, 1.54e-16 and 1.62e-16 to 1.8e-16.
 //
 // One hop, us, FP64 multiply-adds / this: SU(3) 24^3x48 nrhs 12 5826 / 1685, SU(4) 16^3x32 nrhs 16
-// 2480 / 757, SU(3) 14x10x6x18 nrhs 5 59 / 27, SU(3) 12^3x24 nrhs 1 44 / 27.  It is bound by instruction
+// 2480 / 757, SU(3) 14x10x6x18 nrhs 5 59 / 27, SU(3) 12^3x24 nrhs 1 44 / 19 (split form, as the next), SU(6) 16^3x32 nrhs 16 4983 / 2286,
+// SU(8) 8383 / 4037, SU(6) 8^3x16 nrhs 1 100 / 19.  It is bound by instruction
 // issue and latency (SU(3): 8300 instructions a warp, 216 wide multiply-adds a hop; the multiplier 53%
 // busy, the integer pipe 43%, FP64 33%, 12 or 16 warps an SM); the small sizes by the latency of one
 // warp a scheduler.
 //
 // A common exponent keeps the digits of a part only down to its unit.  So a site takes the FP64
-// multiply-adds (fp64_site, the arithmetic of the other SU(N)) when the non-zero parts that it
+// multiply-adds (fp64_site) when the non-zero parts that it
 // multiplies span more than kFixSpan bits, when anything it reads is infinite or NaN, and when the
 // result could leave the normal range.
 #pragma once
@@ -32,8 +34,10 @@
 namespace qcu {
 namespace detail {
 
-// the FP64 SU(N) hops that run in fixed point (the accumulators hold sums over N = 4 at most)
-__host__ __device__ constexpr bool fix_hop(int prec, int N) { return prec == PREC_DOUBLE && (N == 3 || N == 4); }
+// the FP64 SU(N) hops that run in fixed point; from SU(5) on only in the split form (a thread cannot hold
+// the sums of 8N parts)
+__host__ __device__ constexpr bool fix_hop(int prec, int N) { return prec == PREC_DOUBLE && N >= 3 && N <= 8; }
+__host__ __device__ constexpr bool fix_split_only(int N) { return N > 4; }
 
 // A part 32 bits below the largest keeps 24 digits of its own.  One site in FP64 multiply-adds takes a
 // warp 27 us, as long as a small launch: at 24 bits, where 1e-5 of random sites span more, SU(3)
@@ -44,8 +48,10 @@ constexpr int kFixSpan = 32;
 //   high  |sum uh hh|            <= 2N 2^56     (N = 4: 2^59)
 //   mid   |sum uh hl + ul hh|    <= 2N 2 2^28 (2^31 - 1)   (N = 4: 2^63 - 2^32, so the rounding bit fits)
 // A hop's sum in the accumulator's unit is high + (mid >> 31), below 2^59 + 2^32 at N = 4; eight of
-// them stay below 2^63.
-constexpr uint32_t kFixShift = 5;  // right shift of a mantissa whose top bit is bit 63
+// them stay below 2^63.  From SU(5) on |F| < 2^58, which bounds N = 8 by the same sums, and lo is
+// balanced, |lo| <= 2^30: the 2N products low x low that are left out would otherwise cost 2e-16.
+template <int N>
+constexpr uint32_t kFixShift = N <= 4 ? 5 : 6;  // right shift of a mantissa whose top bit is bit 63
 
 struct Limbs {
   int32_t hi, lo;
@@ -54,6 +60,7 @@ struct Limbs {
 __device__ __forceinline__ uint32_t biased_exp(double x) { return ((uint32_t)__double2hiint(x) >> 20) & 0x7ffu; }
 
 // x over the biased exponent es - kFixShift of the largest part; flip 0x80000000 negates
+template <int N>
 __device__ __forceinline__ Limbs to_limbs(double x, uint32_t es, uint32_t flip) {
   const uint32_t hi = (uint32_t)__double2hiint(x), lo = (uint32_t)__double2loint(x);
   const uint32_t mh = __funnelshift_l(lo, hi, 11) | 0x80000000u, ml = lo << 11;
@@ -61,6 +68,10 @@ __device__ __forceinline__ Limbs to_limbs(double x, uint32_t es, uint32_t flip) 
   unsigned long long f;
   asm("shr.u64 %0, %1, %2;" : "=l"(f) : "l"(((unsigned long long)mh << 32) | ml), "r"(s));  // shifts above 63 give 0
   const int32_t sign = ((int32_t)(hi ^ flip) >> 31) | 1;
+  if constexpr (fix_split_only(N)) {
+    const uint32_t top = (uint32_t)((f + (1u << 30)) >> 31);
+    return Limbs{(int32_t)top * sign, (int32_t)((uint32_t)f - (top << 31)) * sign};
+  }
   return Limbs{(int32_t)(uint32_t)(f >> 31) * sign, (int32_t)((uint32_t)f & 0x7fffffffu) * sign};
 }
 
@@ -70,6 +81,9 @@ __device__ __forceinline__ long long asr64(long long v, uint32_t s) {
   return r;
 }
 
+// a sum T over hops of largest exponent E is T 2^(E - 2110 + 2 kFixShift): from_fix(T, E + kFixBias)
+template <int N>
+constexpr int kFixBias = 2 * (int)kFixShift<N> - 1025;
 // T as a double, rounded to nearest even: the result's biased exponent is e + 1 - clz(|T|); T = 0 gives +0
 __device__ __forceinline__ double from_fix(long long T, int e) {
   const uint32_t sg = (uint32_t)((unsigned long long)T >> 63);
@@ -91,34 +105,49 @@ struct FixLink {
   uint32_t e;
 };
 
+// where hop h's link lies, and the signs of its parts
+template <int N>
+struct FixLinkAt {
+  const double2* lb;
+  uint32_t sa, sb;  // strides of a and b
+  uint32_t rf, jf;  // sign flips of the real and imaginary parts
+  __device__ __forceinline__ FixLinkAt(const DslashArgs& A, const SiteXyzt& X, int h, uint32_t nb) {
+    const int mu = h >> 1;
+    const bool bwd = h & 1;
+    const uint32_t vh = (uint32_t)A.geo.vh, p = (uint32_t)A.parity;
+    lb = static_cast<const double2*>(A.gauge) +
+         ((mu * 2u + (bwd ? 1u - p : p)) * (uint32_t)(N * N) * vh + (bwd ? nb : X.site));
+    sa = (bwd ? 1u : (uint32_t)N) * vh;
+    sb = (bwd ? (uint32_t)N : 1u) * vh;
+    const bool wrap = mu == 3 && A.antiperiodic_t && (bwd ? X.t == 0 : X.t == (uint32_t)A.geo.L[3] - 1);
+    rf = wrap ? 0x80000000u : 0u;
+    jf = rf ^ (bwd ? 0x80000000u : 0u);
+  }
+  __device__ __forceinline__ double2 load(int a, int b) const { return __ldg(lb + (a * sa + b * sb)); }
+  __device__ __forceinline__ int4 limbs(double2 v, uint32_t e) const {
+    const Limbs r = to_limbs<N>(v.x, e + kFixShift<N>, rf), i = to_limbs<N>(v.y, e + kFixShift<N>, jf);
+    return make_int4(r.hi, r.lo, i.hi, i.lo);
+  }
+};
+
 template <int N>
 __device__ __forceinline__ FixLink<N> load_fix_link(const DslashArgs& A, const SiteXyzt& X, int h, uint32_t nb) {
-  const int mu = h >> 1;
-  const bool bwd = h & 1;
-  const uint32_t vh = (uint32_t)A.geo.vh, p = (uint32_t)A.parity;
-  const double2* lb = static_cast<const double2*>(A.gauge) +
-                      ((mu * 2u + (bwd ? 1u - p : p)) * (uint32_t)(N * N) * vh + (bwd ? nb : X.site));
-  const uint32_t sa = (bwd ? 1u : (uint32_t)N) * vh, sb = (bwd ? (uint32_t)N : 1u) * vh;
+  const FixLinkAt<N> at(A, X, h, nb);
   double2 u[N][N];
   FixLink<N> L;
   L.e = 0;
 #pragma unroll
   for (int a = 0; a < N; a++)
 #pragma unroll
-    for (int b = 0; b < N; b++) u[a][b] = __ldg(lb + (a * sa + b * sb));
+    for (int b = 0; b < N; b++) u[a][b] = at.load(a, b);
 #pragma unroll
   for (int a = 0; a < N; a++)
 #pragma unroll
     for (int b = 0; b < N; b++) L.e = max(L.e, max(biased_exp(u[a][b].x), biased_exp(u[a][b].y)));
-  const bool wrap = mu == 3 && A.antiperiodic_t && (bwd ? X.t == 0 : X.t == (uint32_t)A.geo.L[3] - 1);
-  const uint32_t rf = wrap ? 0x80000000u : 0u, jf = rf ^ (bwd ? 0x80000000u : 0u);
 #pragma unroll
   for (int a = 0; a < N; a++)
 #pragma unroll
-    for (int b = 0; b < N; b++) {
-      const Limbs r = to_limbs(u[a][b].x, L.e + kFixShift, rf), i = to_limbs(u[a][b].y, L.e + kFixShift, jf);
-      L.u[a * N + b] = make_int4(r.hi, r.lo, i.hi, i.lo);
-    }
+    for (int b = 0; b < N; b++) L.u[a * N + b] = at.limbs(u[a][b], L.e);
   return L;
 }
 
@@ -182,11 +211,22 @@ __device__ __forceinline__ void fix_hop_products(Out& out, const DslashArgs& A, 
       y[1][a] = __ldg(reinterpret_cast<const double2*>(low + r1 + (uint64_t)a * cs_bytes));
     }
   }
-  FixLink<SHARED ? 1 : N> own;
+  // SHARED: records in shared memory; else in registers, or from SU(5) on, where they would not fit, read
+  // twice, for the exponent and (from L1) for each product
+  constexpr bool kTwice = !SHARED && fix_split_only(N);
+  FixLink<SHARED || kTwice ? 1 : N> own;
+  const FixLinkAt<N> at(A, X, h, nb);
   const int4* rec = links + h * kFixRec<N>;
   uint32_t eu;
   if constexpr (SHARED) {
     eu = (uint32_t)reinterpret_cast<const int2*>(rec + N * N)[N * N].x;
+  } else if constexpr (kTwice) {
+    eu = 0;
+#pragma unroll 4
+    for (int k = 0; k < N * N; k++) {
+      const double2 v = at.load(k / N, k % N);
+      eu = max(eu, max(biased_exp(v.x), biased_exp(v.y)));
+    }
   } else {
     own = load_fix_link<N>(A, X, h, nb);
     eu = own.e;
@@ -210,7 +250,7 @@ __device__ __forceinline__ void fix_hop_products(Out& out, const DslashArgs& A, 
     }
   bool bad = ep == 0x7ffu || eu == 0x7ffu || eu < 200u;
   int eh = (int)(ep + eu);
-  uint32_t es = ep + kFixShift;
+  uint32_t es = ep + kFixShift<N>;
   if (ep == 0) {  // zeros add nothing; subnormal parts: FP64
     long long any = 0;
 #pragma unroll
@@ -226,13 +266,13 @@ __device__ __forceinline__ void fix_hop_products(Out& out, const DslashArgs& A, 
   for (int i = 0; i < 2; i++)
 #pragma unroll
     for (int a = 0; a < N; a++) {
-      hr[i][a] = to_limbs(x[i][a].x, es, 0u);
-      hi[i][a] = to_limbs(x[i][a].y, es, 0u);
+      hr[i][a] = to_limbs<N>(x[i][a].x, es, 0u);
+      hi[i][a] = to_limbs<N>(x[i][a].y, es, 0u);
     }
 
   out.begin(eh, (int)min(mn, 4095u) + 1 + (int)eu, bad);
 
-#pragma unroll
+#pragma unroll fix_split_only(N) ? 1 : N
   for (int a = 0; a < N; a++) {
     long long H[2][2], M[2][2];
 #pragma unroll
@@ -247,7 +287,7 @@ __device__ __forceinline__ void fix_hop_products(Out& out, const DslashArgs& A, 
         u = rec[a * N + b];
         n = reinterpret_cast<const int2*>(rec + N * N)[a * N + b];
       } else {
-        u = own.u[a * N + b];
+        u = kTwice ? at.limbs(at.load(a, b), eu) : own.u[kTwice ? 0 : a * N + b];
         n = make_int2(-u.z, -u.w);
       }
 #pragma unroll
@@ -354,7 +394,7 @@ __device__ __forceinline__ void fix_site(const DslashArgs& A, const SiteXyzt& X,
     return;
   }
   C2<double> out[4][N][1];
-  const int e = S.E - 1015;
+  const int e = S.E + kFixBias<N>;
 #pragma unroll
   for (int i = 0; i < 2; i++)
 #pragma unroll
@@ -423,6 +463,12 @@ __device__ __forceinline__ void fix_block(const DslashArgs& A, uint32_t gid0) {
 // times both.
 template <int N>
 constexpr uint32_t kFixSplitUnit = 8 * (4 * N * 8 + 8);  // bytes of a site and RHS
+// the largest block up to `block` whose products stay within 48 KB
+template <int N>
+int fix_split_block_size(int block) {
+  while (block > 32 && (uint32_t)block / 8 * kFixSplitUnit<N> > 48u * 1024u) block -= 32;
+  return block;
+}
 
 template <int N>
 struct FixShare {
@@ -507,7 +553,7 @@ __device__ __forceinline__ void fix_split_block(const DslashArgs& A, uint32_t bl
         }
       }
     }
-    double2 r = make_double2(from_fix(s0, Es - 1015), from_fix(s1, Es - 1015));
+    double2 r = make_double2(from_fix(s0, Es + kFixBias<N>), from_fix(s1, Es + kFixBias<N>));
     // store_out's operations
     if (A.x) {
       if (A.b == 1.0)

@@ -836,8 +836,7 @@ __device__ __forceinline__ void site_rhs(const DslashArgs& A, const SiteXyzt& X,
   const uint32_t lb = (1u - p) * NN * lvh;
   const uint32_t dmu = 2 * NN * lvh;  // one direction's links
   // FP32 and BF16 storage prefetch every hop's links (below; measured 4-19%
-  // faster).  FP64 (here SU(5) and up, and the sites that dslash_fix.cuh leaves)
-  // is bound by its FMA pipe and FP16 (with its norm loads) measured 2-6% slower
+  // faster).  FP64 (here the sites that dslash_fix.cuh leaves) is bound by its FMA pipe and FP16 (with its norm loads) measured 2-6% slower
   // with the prefetch, so they run the hops without it, in the form that
   // compiles best for them.
   if constexpr (P == PREC_SINGLE || P == PREC_BF16) {
@@ -940,9 +939,10 @@ __device__ __forceinline__ void wilson_site(const DslashArgs& A, uint32_t gid) {
   site_rhs<P, N, R, PK, RC>(A, X, rhs0, grp, A.div_groups.d);
 }
 
-// threads per site and group of R RHS: 8 in the split form of the fixed-point hop (PK at FP64)
+// threads per site and group of R RHS: 8 in the split form of the fixed-point hop (PK at FP64; every shape
+// from SU(5) on)
 template <int P, int N, bool PK, bool RC>
-constexpr int kSiteThreads = fix_hop(P, N) && !RC && PK ? 8 : 1;
+constexpr int kSiteThreads = fix_hop(P, N) && !RC && (PK || fix_split_only(N)) ? 8 : 1;
 
 // block `blk` of a launch
 template <int P, int N, int R, bool PK, bool RC>
@@ -964,6 +964,11 @@ uint32_t wilson_blocks(const DslashArgs& A, int R, int block) {
   return (uint32_t)((threads + block - 1) / block);
 }
 template <int P, int N, bool PK, bool RC>
+int wilson_block_size(int block) {
+  if constexpr (kSiteThreads<P, N, PK, RC> == 8) return fix_split_block_size<N>(block);
+  return block;
+}
+template <int P, int N, bool PK, bool RC>
 size_t wilson_smem(uint32_t groups, int block) {
   if constexpr (kSiteThreads<P, N, PK, RC> == 8)
     return (size_t)(block / 8) * kFixSplitUnit<N>;
@@ -983,6 +988,7 @@ __global__ void __maxnreg__(RegCap<MINB>::regs) wilson_mrhs_kernel(const __grid_
 template <int P, int N, int R, int MINB, bool PK = false, bool RC = false>
 void launch_wilson_mrhs(const DslashArgs& A, int block, cudaStream_t stream) {
   const int groups = A.nrhs / R;
+  block = detail::wilson_block_size<P, N, PK, RC>(block);
   const uint32_t grid = detail::wilson_blocks<P, N, PK, RC>(A, R, block);
   const size_t smem = detail::wilson_smem<P, N, PK, RC>((uint32_t)groups, block);
   wilson_mrhs_kernel<P, N, R, MINB, PK, RC><<<grid, block, smem, stream>>>(A);
@@ -1014,6 +1020,7 @@ __global__ void __maxnreg__(RegCap<MINB>::regs) wilson_segments_kernel(const __g
 template <int P, int N, int R, int MINB, bool PK = false, bool RC = false>
 void launch_wilson_segments(HopSegments& S, int block, cudaStream_t stream) {
   uint32_t total = 0;
+  block = detail::wilson_block_size<P, N, PK, RC>(block);
   for (int s = 0; s < S.count; s++) {
     S.block_begin[s] = total;
     total += detail::wilson_blocks<P, N, PK, RC>(S.A[s], R, block);
