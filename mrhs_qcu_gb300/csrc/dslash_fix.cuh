@@ -19,16 +19,15 @@
 // 1.45e-16, 1.54e-16 and 1.62e-16 to 1.8e-16.
 //
 // One hop, us, FP64 multiply-adds / this: SU(3) 24^3x48 nrhs 12 5826 / 1685, SU(4) 16^3x32 nrhs 16
-// 2480 / 757, SU(3) 14x10x6x18 nrhs 5 59 / 27, SU(3) 12^3x24 nrhs 1 44 / 19 (split form, as the next), SU(6) 16^3x32 nrhs 16 4983 / 2286,
-// SU(8) 8383 / 4037, SU(6) 8^3x16 nrhs 1 100 / 19.  It is bound by instruction
-// issue and latency (SU(3): 8300 instructions a warp, 216 wide multiply-adds a hop; the multiplier 53%
-// busy, the integer pipe 43%, FP64 33%, 12 or 16 warps an SM); the small sizes by the latency of one
-// warp a scheduler.
+// 2480 / 757, SU(3) 14x10x6x18 nrhs 5 59 / 27; in the split form SU(3) 12^3x24 nrhs 1 44 / 19, SU(6)
+// 16^3x32 nrhs 16 4983 / 2286, SU(8) 8383 / 4037, SU(6) 8^3x16 nrhs 1 100 / 19.  It is bound by
+// instruction issue and latency (SU(3): 8300 instructions a warp, 216 wide multiply-adds a hop; the
+// multiplier 53% busy, the integer pipe 43%, FP64 33%, 12 or 16 warps an SM); the small sizes by the
+// latency of one warp a scheduler.
 //
 // A common exponent keeps the digits of a part only down to its unit.  So a site takes the FP64
-// multiply-adds (fp64_site) when the non-zero parts that it
-// multiplies span more than kFixSpan bits, when anything it reads is infinite or NaN, and when the
-// result could leave the normal range.
+// multiply-adds (fp64_site) when the non-zero parts that it multiplies span more than kFixSpan bits,
+// when anything it reads is infinite or NaN, and when the result could leave the normal range.
 #pragma once
 
 namespace qcu {
