@@ -18,8 +18,8 @@
 // fields: SU(3), SU(4) 0.84e-16, SU(5) to SU(8) 1.20e-16 to 1.24e-16, where the FP64 multiply-adds have
 // 1.45e-16, 1.54e-16 and 1.62e-16 to 1.8e-16.
 //
-// One hop, us, FP64 multiply-adds / this: SU(3) 24^3x48 nrhs 12 5826 / 1685, SU(4) 16^3x32 nrhs 16
-// 2480 / 757, SU(3) 14x10x6x18 nrhs 5 59 / 27; in the split form SU(3) 12^3x24 nrhs 1 44 / 19, SU(6)
+// One hop, us, FP64 multiply-adds / this: SU(3) 24^3x48 nrhs 12 5826 / 1660, SU(4) 16^3x32 nrhs 16
+// 2480 / 743, SU(3) 14x10x6x18 nrhs 5 59 / 27; in the split form SU(3) 12^3x24 nrhs 1 44 / 19, SU(6)
 // 16^3x32 nrhs 16 4983 / 2286, SU(8) 8383 / 4037, SU(6) 8^3x16 nrhs 1 100 / 19.  It is bound by
 // instruction issue and latency (SU(3): 8300 instructions a warp, 216 wide multiply-adds a hop; the
 // multiplier 53% busy, the integer pipe 43%, FP64 33%, 12 or 16 warps an SM); the small sizes by the
@@ -38,10 +38,10 @@ namespace detail {
 __host__ __device__ constexpr bool fix_hop(int prec, int N) { return prec == PREC_DOUBLE && N >= 3 && N <= 8; }
 __host__ __device__ constexpr bool fix_split_only(int N) { return N > 4; }
 
-// A part 32 bits below the largest keeps 24 digits of its own.  One site in FP64 multiply-adds takes a
+// A part 31 bits below the largest keeps 25 digits of its own.  One site in FP64 multiply-adds takes a
 // warp 27 us, as long as a small launch: at 24 bits, where 1e-5 of random sites span more, SU(3)
 // 14x10x6x18 nrhs 5 took 54 us against 27.
-constexpr int kFixSpan = 32;
+constexpr int kFixSpan = 31;
 
 // Parts |F| < 2^59 as limbs F = hi 2^31 + lo, |hi| <= 2^28, |lo| < 2^31.  Over a component's 2N products:
 //   high  |sum uh hh|            <= 2N 2^56     (N = 4: 2^59)
@@ -74,10 +74,12 @@ __device__ __forceinline__ Limbs to_limbs(double x, uint32_t es, uint32_t flip) 
   return Limbs{(int32_t)(uint32_t)(f >> 31) * sign, (int32_t)((uint32_t)f & 0x7fffffffu) * sign};
 }
 
-__device__ __forceinline__ long long asr64(long long v, uint32_t s) {
-  long long r;
-  asm("shr.s64 %0, %1, %2;" : "=l"(r) : "l"(v), "r"(s));  // shifts above 63 give the sign
-  return r;
+// v >> s for s up to 31, which a site's shifts are while its span holds (kFixSpan); with larger ones, whose
+// sites take FP64, it is any value (a 64-bit shift instruction pair costs 1.5% of the hop)
+__device__ __forceinline__ long long asr(long long v, uint32_t s) {
+  const int32_t h = (int32_t)(v >> 32);
+  const uint32_t lo = __funnelshift_r((uint32_t)v, (uint32_t)h, s);
+  return (long long)(((unsigned long long)(uint32_t)(h >> (s & 31u)) << 32) | lo);
 }
 
 // a sum T over hops of largest exponent E is T 2^(E - 2110 + 2 kFixShift): from_fix(T, E + kFixBias)
@@ -330,8 +332,8 @@ struct FixAdd {
         for (int a = 0; a < N; a++)
 #pragma unroll
           for (int c = 0; c < 2; c++) {
-            S.up[i][a][c] = asr64(S.up[i][a][c], up);
-            S.lo[i][a][c] = asr64(S.lo[i][a][c], up);
+            S.up[i][a][c] = asr(S.up[i][a][c], up);
+            S.lo[i][a][c] = asr(S.lo[i][a][c], up);
           }
       S.E = eh;
     }
@@ -339,7 +341,7 @@ struct FixAdd {
   }
   // lower rows: lo(u) += s g(u_perm) (im ? i : 1) t_u
   __device__ __forceinline__ void put(int a, int i, long long re, long long im) {
-    const long long t0 = asr64(re, d), t1 = asr64(im, d), m = fix_lower_sign(A, h, i);
+    const long long t0 = asr(re, d), t1 = asr(im, d), m = fix_lower_sign(A, h, i);
     S.up[i][a][0] += t0;
     S.up[i][a][1] += t1;
     const bool imag = !((h >> 1) & 1);
@@ -531,13 +533,13 @@ __device__ __forceinline__ void fix_split_block(const DslashArgs& A, uint32_t bl
     for (int g = 0; g < 8; g++) {
       const int mu = g >> 1, eg = exps[g * U + u].x;
       if (eg > Es) {
-        s0 = asr64(s0, (uint32_t)(eg - Es));
-        s1 = asr64(s1, (uint32_t)(eg - Es));
+        s0 = asr(s0, (uint32_t)(eg - Es));
+        s1 = asr(s1, (uint32_t)(eg - Es));
         Es = eg;
       }
       const int i = row < 2 ? row : mu < 2 ? 3 - row : row - 2;  // the projected row that feeds this one
       const long long* v = vals + ((g * 4 * N + 2 * (i * N + a)) * U + u);
-      const long long t0 = asr64(v[0], (uint32_t)(Es - eg)), t1 = asr64(v[U], (uint32_t)(Es - eg));
+      const long long t0 = asr(v[0], (uint32_t)(Es - eg)), t1 = asr(v[U], (uint32_t)(Es - eg));
       if (row < 2) {
         s0 += t0;
         s1 += t1;
