@@ -1,4 +1,6 @@
-// Dslash instances for PREC_DOUBLE; registered at library load.
+// Dslash instances for PREC_DOUBLE; registered at library load.  All of them
+// run the fixed-point hop (dslash_fix.cuh): R > 1 takes the RHS of a thread one
+// after another, PK is the split form.
 #include "dslash.h"
 
 namespace qcu {

@@ -836,9 +836,10 @@ __device__ __forceinline__ void site_rhs(const DslashArgs& A, const SiteXyzt& X,
   const uint32_t lb = (1u - p) * NN * lvh;
   const uint32_t dmu = 2 * NN * lvh;  // one direction's links
   // FP32 and BF16 storage prefetch every hop's links (below; measured 4-19%
-  // faster).  FP64 (here the sites that dslash_fix.cuh leaves) is bound by its FMA pipe and FP16 (with its norm loads) measured 2-6% slower
-  // with the prefetch, so they run the hops without it, in the form that
-  // compiles best for them.
+  // faster).  FP64 (here the sites that dslash_fix.cuh leaves) is bound by its
+  // FMA pipe and FP16 (with its norm loads) measured 2-6% slower with the
+  // prefetch, so they run the hops without it, in the form that compiles best
+  // for them.
   if constexpr (P == PREC_SINGLE || P == PREC_BF16) {
     const uint32_t pl = A.geo.plane, cb = A.geo.cube;
     const bool top = t == Lt - 1, bot = t == 0;
