@@ -63,7 +63,7 @@ template <int N>
 __device__ __forceinline__ Limbs to_limbs(double x, uint32_t es, uint32_t flip) {
   const uint32_t hi = (uint32_t)__double2hiint(x), lo = (uint32_t)__double2loint(x);
   const uint32_t mh = __funnelshift_l(lo, hi, 11) | 0x80000000u, ml = lo << 11;
-  const uint32_t s = es - ((hi >> 20) & 0x7ffu);  // a zero's is above 63
+  const uint32_t s = es - ((hi >> 20) & 0x7ffu);  // a zero's is es, above 63
   unsigned long long f;
   asm("shr.u64 %0, %1, %2;" : "=l"(f) : "l"(((unsigned long long)mh << 32) | ml), "r"(s));  // shifts above 63 give 0
   const int32_t sign = ((int32_t)(hi ^ flip) >> 31) | 1;
@@ -252,6 +252,7 @@ __device__ __forceinline__ void fix_hop_products(Out& out, const DslashArgs& A, 
   bool bad = ep == 0x7ffu || eu == 0x7ffu || eu < 200u;
   int eh = (int)(ep + eu);
   uint32_t es = ep + kFixShift<N>;
+  bad |= ep != 0 && es < 64;  // a zero's shift, es, would leave its implicit leading bit (to_limbs)
   if (ep == 0) {  // zeros add nothing; subnormal parts: FP64
     long long any = 0;
 #pragma unroll
