@@ -6,28 +6,32 @@
 // and the sum over hops are done in integers:
 //
 //   projected spinor   the 4N real parts of a neighbour's two rows, 59 bits over their common exponent
-//   link               its 2N^2 real parts, 59 bits over theirs
-//   product            limbs of 28 and 31 bits, the three larger limb products summed exactly in two
-//                      64-bit accumulators a component; only low x low (2^-56 of the operands' largest
-//                      parts, at most) is left out
+//   link               its 2N^2 real parts, 59 bits over theirs (SU(8): both 58)
+//   product            limbs of 28 and 31 bits, the low ones balanced (SU(8): 28 and 30), the three larger limb
+//                      products summed exactly in two 64-bit accumulators a component; only low x low (2^-58 of
+//                      the operands' largest parts, at most) is left out
 //   sum over hops      64-bit integers over the largest hop's exponent
 //   result             rounded once to double (nearest even); the xpay epilogue stays FP64
 //
 // No sum can overflow (the bounds stand beside the constants), and none rounds before the last step
 // but by the right shifts to the accumulator's unit.  Relative L2 error against quad precision on random
-// fields: SU(3), SU(4) 0.84e-16, SU(5) to SU(8) 1.20e-16 to 1.24e-16, where the FP64 multiply-adds have
-// 1.45e-16, 1.54e-16 and 1.62e-16 to 1.8e-16.
+// fields: SU(3), SU(4) 0.71e-16, SU(5) to SU(8) 0.74e-16, where the FP64 multiply-adds have 1.46e-16, 1.54e-16
+// and 1.61e-16 to 1.80e-16.
 //
-// One hop, us, FP64 multiply-adds / this: SU(3) 24^3x48 nrhs 12 5826 / 1660, SU(4) 16^3x32 nrhs 16
-// 2480 / 743, SU(3) 14x10x6x18 nrhs 5 59 / 27; in the split form SU(3) 12^3x24 nrhs 1 44 / 19, SU(6)
-// 16^3x32 nrhs 16 4983 / 2286, SU(8) 8383 / 4037, SU(6) 8^3x16 nrhs 1 100 / 19.  It is bound by
+// One hop, us, FP64 multiply-adds / this: SU(3) 24^3x48 nrhs 12 5763 / 1747, SU(4) 16^3x32 nrhs 16
+// 2460 / 779, SU(3) 14x10x6x18 nrhs 5 62 / 27; in the split form SU(3) 12^3x24 nrhs 1 46 / 21, SU(6)
+// 16^3x32 nrhs 16 4978 / 2486, SU(8) 8378 / 4187, SU(6) 8^3x16 nrhs 1 99 / 19.  It is bound by
 // instruction issue and latency (SU(3): 8300 instructions a warp, 216 wide multiply-adds a hop; the
 // multiplier 53% busy, the integer pipe 43%, FP64 33%, 12 or 16 warps an SM); the small sizes by the
 // latency of one warp a scheduler.
 //
-// A common exponent keeps the digits of a part only down to its unit.  So a site takes the FP64
-// multiply-adds (fp64_site) when the non-zero parts that it multiplies span more than kFixSpan bits,
-// when anything it reads is infinite or NaN, and when the result could leave the normal range.
+// A common exponent keeps the digits of a part only down to its unit.  So a site takes the FP64 multiply-adds
+// (fp64_site) when a part of its result is made up of small products only (fix_parts_hold), when its hops lie more
+// than kFixSpan binades apart, when anything it reads is infinite or NaN, and when the result could leave the
+// normal range.  Where a field's structure sends every site there, a hop takes the time of both: one-colour
+// spinors on near-unit links, us, against FP64 multiply-adds alone: SU(3) 24^3x48 nrhs 12 6850 / 5763, SU(4)
+// 16^3x32 nrhs 16 2970 / 2460, SU(6) 16^3x32 nrhs 16 15100 / 4978 (one thread
+// of eight does the FP64 site).
 #pragma once
 
 namespace qcu {
@@ -38,19 +42,27 @@ namespace detail {
 __host__ __device__ constexpr bool fix_hop(int prec, int N) { return prec == PREC_DOUBLE && N >= 3 && N <= 8; }
 __host__ __device__ constexpr bool fix_split_only(int N) { return N > 4; }
 
-// A part 31 bits below the largest keeps 25 digits of its own.  One site in FP64 multiply-adds takes a
-// warp 27 us, as long as a small launch: at 24 bits, where 1e-5 of random sites span more, SU(3)
-// 14x10x6x18 nrhs 5 took 54 us against 27.
+// The hops of a site may lie this many binades apart (the shift that asr takes).
 constexpr int kFixSpan = 31;
 
-// Parts |F| < 2^59 as limbs F = hi 2^31 + lo, |hi| <= 2^28, |lo| < 2^31.  Over a component's 2N products:
-//   high  |sum uh hh|            <= 2N 2^56     (N = 4: 2^59)
-//   mid   |sum uh hl + ul hh|    <= 2N 2 2^28 (2^31 - 1)   (N = 4: 2^63 - 2^32, so the rounding bit fits)
-// A hop's sum in the accumulator's unit is high + (mid >> 31), below 2^59 + 2^32 at N = 4; eight of
-// them stay below 2^63.  From SU(5) on |F| < 2^58, which bounds N = 8 by the same sums, and lo is
-// balanced, |lo| <= 2^30: the 2N products low x low that are left out would otherwise cost 2e-16.
+// A part is |F| < 2^B over its common exponent, B = 64 - kFixShift, as limbs F = hi 2^s + lo, s = kFixSplit,
+// |hi| <= 2^(B - s), |lo| <= 2^(s - 1).  Over a component's 2N products:
+//   high  |sum uh hh|            <= 2N 2^(2B - 2s)
+//   mid   |sum uh hl + ul hh|    <= 2N 2^B          (N = 7: 2^62.8, and the rounding bits fit)
+// A hop's product in the accumulator's unit 2^(2s - x), x = kFixExtra, is (high << x) + (mid >> (s - x)).  Its
+// exact value is at most 2N F^2 / 2^(2s - x) <= 2^60 - 2^8 for every N, and what is left out and rounded is at
+// most 5 units, so eight of them stay below 2^63.
 template <int N>
-constexpr uint32_t kFixShift = N <= 4 ? 5 : 6;  // right shift of a mantissa whose top bit is bit 63
+constexpr uint32_t kFixShift = N <= 7 ? 5 : 6;  // right shift of a mantissa whose top bit is bit 63
+template <int N>
+constexpr uint32_t kFixSplit = N <= 7 ? 31 : 30;
+template <int N>
+constexpr uint32_t kFixExtra = N <= 4 ? 1 : 0;
+
+// A part of the result holds when its eight products add up to this many times 2^48 units (2^57, 2^56 for N > 4,
+// is a largest product): fix_parts_hold.
+template <int N>
+constexpr uint32_t kFixMag = N <= 4 ? 24 : 32;
 
 struct Limbs {
   int32_t hi, lo;
@@ -58,33 +70,33 @@ struct Limbs {
 
 __device__ __forceinline__ uint32_t biased_exp(double x) { return ((uint32_t)__double2hiint(x) >> 20) & 0x7ffu; }
 
-// x over the biased exponent es - kFixShift of the largest part; flip 0x80000000 negates
+// x over the biased exponent es - kFixShift of the largest part; flip 0x80000000 negates.  A zero's shift is es,
+// so es must be above 63.
 template <int N>
 __device__ __forceinline__ Limbs to_limbs(double x, uint32_t es, uint32_t flip) {
+  constexpr uint32_t kSplit = kFixSplit<N>;
   const uint32_t hi = (uint32_t)__double2hiint(x), lo = (uint32_t)__double2loint(x);
   const uint32_t mh = __funnelshift_l(lo, hi, 11) | 0x80000000u, ml = lo << 11;
-  const uint32_t s = es - ((hi >> 20) & 0x7ffu);  // a zero's is es, above 63
+  const uint32_t s = es - ((hi >> 20) & 0x7ffu);
   unsigned long long f;
   asm("shr.u64 %0, %1, %2;" : "=l"(f) : "l"(((unsigned long long)mh << 32) | ml), "r"(s));  // shifts above 63 give 0
   const int32_t sign = ((int32_t)(hi ^ flip) >> 31) | 1;
-  if constexpr (fix_split_only(N)) {
-    const uint32_t top = (uint32_t)((f + (1u << 30)) >> 31);
-    return Limbs{(int32_t)top * sign, (int32_t)((uint32_t)f - (top << 31)) * sign};
-  }
-  return Limbs{(int32_t)(uint32_t)(f >> 31) * sign, (int32_t)((uint32_t)f & 0x7fffffffu) * sign};
+  const uint32_t top = (uint32_t)((f + (1u << (kSplit - 1))) >> kSplit);
+  return Limbs{(int32_t)top * sign, (int32_t)((uint32_t)f - (top << kSplit)) * sign};
 }
 
-// v >> s for s up to 31, which a site's shifts are while its span holds (kFixSpan); with larger ones, whose
-// sites take FP64, it is any value (a 64-bit shift instruction pair costs 1.5% of the hop)
+// v >> s for s up to 31, which a site's shifts are while its hops lie within kFixSpan (or v is 0); with larger
+// ones, whose sites take FP64, it is any value (a 64-bit shift instruction pair costs 1.5% of the hop)
 __device__ __forceinline__ long long asr(long long v, uint32_t s) {
   const int32_t h = (int32_t)(v >> 32);
   const uint32_t lo = __funnelshift_r((uint32_t)v, (uint32_t)h, s);
   return (long long)(((unsigned long long)(uint32_t)(h >> (s & 31u)) << 32) | lo);
 }
 
-// a sum T over hops of largest exponent E is T 2^(E - 2110 + 2 kFixShift): from_fix(T, E + kFixBias)
+// a sum T over hops of largest exponent E is T 2^(E - 2172 + 2 kFixShift + 2 kFixSplit - kFixExtra):
+// from_fix(T, E + kFixBias)
 template <int N>
-constexpr int kFixBias = 2 * (int)kFixShift<N> - 1025;
+constexpr int kFixBias = 2 * (int)kFixShift<N> + 2 * (int)kFixSplit<N> - (int)kFixExtra<N> - 1087;
 // T as a double, rounded to nearest even: the result's biased exponent is e + 1 - clz(|T|); T = 0 gives +0
 __device__ __forceinline__ double from_fix(long long T, int e) {
   const uint32_t sg = (uint32_t)((unsigned long long)T >> 63);
@@ -154,7 +166,7 @@ __device__ __forceinline__ FixLink<N> load_fix_link(const DslashArgs& A, const S
 
 // Links of a block's sites in shared memory, converted once for all the RHS of a site (in each thread the
 // conversion was a third of the instructions: SU(3) 24^3x48 nrhs 12 3140 us, with 24 parts a hop converted
-// instead of the 12 projected ones, against 1685): [site][hop] records of the N^2 elements (int4), their
+// instead of the 12 projected ones, against 1685 as the rest of the kernel was then): [site][hop] records of the N^2 elements (int4), their
 // negated imaginary parts (int2), and the exponent
 template <int N>
 constexpr uint32_t kFixRec = N * N + N * N / 2 + 1;
@@ -172,9 +184,21 @@ template <int N>
 struct FixAcc {
   long long up[2][N][2];  // rows 0 and 1
   long long lo[2][N][2];  // the rows that take the products of rows 0 and 1 (3 and 2 for x and y, 2 and 3 for z and t)
-  int E = 0, Emin = 8191;
+  uint32_t mag[N] = {};     // sums of fix_mag of the products of row 0 (low half) and row 1: of x and y, then of z and t
+  uint32_t mag_xy[N];       // those of x and y, over the exponent E_xy
+  int E = 0, E_xy = 0;      // largest exponent of a hop; of one of x and y
+  uint32_t rows = 0;        // bit i: projected row i is not zero in some hop of x or y; bit 2 + i: of z or t
   bool bad = false;
 };
+
+// |re| and |im| of a product, whichever is smaller, in 2^32 units
+__device__ __forceinline__ uint32_t fix_least(long long re, long long im) {
+  return (uint32_t)min(abs((int32_t)(re >> 32)), abs((int32_t)(im >> 32)));
+}
+// both halves of m shifted right by s
+__device__ __forceinline__ uint32_t fix_mag_shift(uint32_t m, uint32_t s) {
+  return s > 15u ? 0u : (m >> s) & ((0xffffu >> s) * 0x10001u);
+}
 
 // s = +1 / -1 of hop h as a sign bit, and the sign s g(u_perm) with which the product of row i enters the lower row
 __device__ __forceinline__ uint32_t fix_sign(const DslashArgs& A, int h) {
@@ -186,32 +210,49 @@ __device__ __forceinline__ long long fix_lower_sign(const DslashArgs& A, int h, 
   return (long long)(int32_t)g >> 31;
 }
 
-// Hop h: out.begin(exponent, smallest exponent, not for fixed point), then out.put(a, i, re, im) for the
-// products of colour a and projected row i in the hop's own unit.
+// the neighbour's spinor; rows 2 and 3 (y) in the order in which rows 0 and 1 (x) meet them
+template <int N>
+__device__ __forceinline__ void fix_load(double2 (&x)[2][N], double2 (&y)[2][N], const DslashArgs& A, uint32_t nb,
+                                         uint32_t rhs, int mu) {
+  const uint32_t nrhs = (uint32_t)A.nrhs, cs_bytes = (uint32_t)A.geo.vh * nrhs * 16u;
+  const char* base = reinterpret_cast<const char*>(static_cast<const double2*>(A.in) + (nb * nrhs + rhs));
+  const char* low = base + (uint64_t)(2 * N) * cs_bytes;
+  const uint64_t up = (uint64_t)N * cs_bytes, r0 = mu < 2 ? up : 0u, r1 = up - r0;
+#pragma unroll
+  for (int a = 0; a < N; a++) {
+    x[0][a] = __ldg(reinterpret_cast<const double2*>(base + (uint64_t)a * cs_bytes));
+    x[1][a] = __ldg(reinterpret_cast<const double2*>(base + (uint64_t)(N + a) * cs_bytes));
+    y[0][a] = __ldg(reinterpret_cast<const double2*>(low + r0 + (uint64_t)a * cs_bytes));
+    y[1][a] = __ldg(reinterpret_cast<const double2*>(low + r1 + (uint64_t)a * cs_bytes));
+  }
+}
+// h_u = x_u + s g(u) y_u, into x
+template <int N>
+__device__ __forceinline__ void fix_project(double2 (&x)[2][N], const double2 (&y)[2][N], const DslashArgs& A, int h) {
+  const int mu = h >> 1;
+  const bool imag = !(mu & 1);
+  const uint32_t sgn = fix_sign(A, h);
+  const double k0 = __hiloint2double((int)(0x3ff00000u | (sgn ^ (mu == 1 ? 0x80000000u : 0u))), 0);
+  const double k1 = __hiloint2double((int)(0x3ff00000u | (sgn ^ (mu == 2 ? 0x80000000u : 0u))), 0);
+#pragma unroll
+  for (int i = 0; i < 2; i++)
+#pragma unroll
+    for (int a = 0; a < N; a++) {
+      const double k = i ? k1 : k0;
+      x[i][a].x = fma(imag ? -k : k, imag ? y[i][a].y : y[i][a].x, x[i][a].x);
+      x[i][a].y = fma(k, imag ? y[i][a].x : y[i][a].y, x[i][a].y);
+    }
+}
+
+// Hop h: out.begin(exponent, bits of the rows that are not zero, not for fixed point), then
+// out.put(a, t) for the products of colour a, t[projected row][re, im], in the hop's own unit.
 template <int N, bool SHARED, typename Out>
 __device__ __forceinline__ void fix_hop_products(Out& out, const DslashArgs& A, const SiteXyzt& X, uint32_t rhs,
                                                  const int4* links, int h) {
   const int mu = h >> 1;
-  const bool imag = !(mu & 1);
-  const uint32_t nrhs = (uint32_t)A.nrhs;
-  const double2* __restrict__ in = static_cast<const double2*>(A.in);
-  const uint32_t cs_bytes = (uint32_t)A.geo.vh * nrhs * 16u;
   const uint32_t nb = X.neighbour(A, h);
-
-  // the neighbour's spinor; rows 2 and 3 in the order in which rows 0 and 1 meet them
   double2 x[2][N], y[2][N];
-  {
-    const char* base = reinterpret_cast<const char*>(in + (nb * nrhs + rhs));
-    const char* low = base + (uint64_t)(2 * N) * cs_bytes;
-    const uint64_t up = (uint64_t)N * cs_bytes, r0 = mu < 2 ? up : 0u, r1 = up - r0;
-#pragma unroll
-    for (int a = 0; a < N; a++) {
-      x[0][a] = __ldg(reinterpret_cast<const double2*>(base + (uint64_t)a * cs_bytes));
-      x[1][a] = __ldg(reinterpret_cast<const double2*>(base + (uint64_t)(N + a) * cs_bytes));
-      y[0][a] = __ldg(reinterpret_cast<const double2*>(low + r0 + (uint64_t)a * cs_bytes));
-      y[1][a] = __ldg(reinterpret_cast<const double2*>(low + r1 + (uint64_t)a * cs_bytes));
-    }
-  }
+  fix_load<N>(x, y, A, nb, rhs, mu);
   // SHARED: records in shared memory; else in registers, or from SU(5) on, where they would not fit, read
   // twice, for the exponent and (from L1) for each product
   constexpr bool kTwice = !SHARED && fix_split_only(N);
@@ -233,33 +274,27 @@ __device__ __forceinline__ void fix_hop_products(Out& out, const DslashArgs& A, 
     eu = own.e;
   }
 
-  // h_u = x_u + s g(u) y_u, into x
-  const uint32_t sgn = fix_sign(A, h);
-  const double k0 = __hiloint2double((int)(0x3ff00000u | (sgn ^ (mu == 1 ? 0x80000000u : 0u))), 0);
-  const double k1 = __hiloint2double((int)(0x3ff00000u | (sgn ^ (mu == 2 ? 0x80000000u : 0u))), 0);
-  uint32_t ep = 0, mn = 0xffffffffu;  // exponents: largest; smallest of the non-zero parts, less one
+  fix_project<N>(x, y, A, h);
+  uint32_t er[2] = {0, 0};  // the rows' largest exponents
 #pragma unroll
   for (int i = 0; i < 2; i++)
 #pragma unroll
-    for (int a = 0; a < N; a++) {
-      const double k = i ? k1 : k0;
-      x[i][a].x = fma(imag ? -k : k, imag ? y[i][a].y : y[i][a].x, x[i][a].x);
-      x[i][a].y = fma(k, imag ? y[i][a].x : y[i][a].y, x[i][a].y);
-      const uint32_t q0 = biased_exp(x[i][a].x), q1 = biased_exp(x[i][a].y);
-      ep = max(ep, max(q0, q1));
-      mn = min(mn, min(q0 - 1u, q1 - 1u));
-    }
+    for (int a = 0; a < N; a++) er[i] = max(er[i], max(biased_exp(x[i][a].x), biased_exp(x[i][a].y)));
+  const uint32_t ep = max(er[0], er[1]);
   bool bad = ep == 0x7ffu || eu == 0x7ffu || eu < 200u;
   int eh = (int)(ep + eu);
   uint32_t es = ep + kFixShift<N>;
-  bad |= ep != 0 && es < 64;  // a zero's shift, es, would leave its implicit leading bit (to_limbs)
-  if (ep == 0) {  // zeros add nothing; subnormal parts: FP64
-    long long any = 0;
+  if (er[0] == 0 || er[1] == 0) {  // rows of zeros add nothing; of subnormal parts: FP64
 #pragma unroll
-    for (int i = 0; i < 2; i++)
+    for (int i = 0; i < 2; i++) {
+      long long any = 0;
 #pragma unroll
       for (int a = 0; a < N; a++) any |= __double_as_longlong(x[i][a].x) | __double_as_longlong(x[i][a].y);
-    bad |= (any << 1) != 0;
+      bad |= er[i] == 0 && (any << 1) != 0;
+    }
+  }
+  if (es < 64) {  // no shift takes a zero's implicit leading bit away (to_limbs): zeros only, or FP64
+    bad |= ep != 0;
     eh = 0;
     es = 64;
   }
@@ -272,7 +307,7 @@ __device__ __forceinline__ void fix_hop_products(Out& out, const DslashArgs& A, 
       hi[i][a] = to_limbs<N>(x[i][a].y, es, 0u);
     }
 
-  out.begin(eh, (int)min(mn, 4095u) + 1 + (int)eu, bad);
+  out.begin(eh, (er[0] ? 1u : 0u) | (er[1] ? 2u : 0u), bad);
 
 #pragma unroll fix_split_only(N) ? 1 : N
   for (int a = 0; a < N; a++) {
@@ -280,7 +315,7 @@ __device__ __forceinline__ void fix_hop_products(Out& out, const DslashArgs& A, 
 #pragma unroll
     for (int i = 0; i < 2; i++)
 #pragma unroll
-      for (int c = 0; c < 2; c++) H[i][c] = 0, M[i][c] = 1ll << 30;
+      for (int c = 0; c < 2; c++) H[i][c] = 0, M[i][c] = 1ll << (kFixSplit<N> - kFixExtra<N> - 1);
 #pragma unroll
     for (int b = 0; b < N; b++) {
       int4 u;
@@ -309,8 +344,12 @@ __device__ __forceinline__ void fix_hop_products(Out& out, const DslashArgs& A, 
         M[i][1] += (long long)u.w * re.hi;
       }
     }
+    long long t[2][2];
 #pragma unroll
-    for (int i = 0; i < 2; i++) out.put(a, i, H[i][0] + (M[i][0] >> 31), H[i][1] + (M[i][1] >> 31));
+    for (int i = 0; i < 2; i++)
+#pragma unroll
+      for (int c = 0; c < 2; c++) t[i][c] = (H[i][c] << kFixExtra<N>) + (M[i][c] >> (kFixSplit<N> - kFixExtra<N>));
+    out.put(a, t);
   }
 }
 
@@ -322,33 +361,44 @@ struct FixAdd {
   int h;
   uint32_t d = 0;  // the hop's shift to the sums' exponent
   // brings the sums so far and this hop to the larger exponent
-  __device__ __forceinline__ void begin(int eh, int emin, bool bad) {
+  __device__ __forceinline__ void begin(int eh, uint32_t rows, bool bad) {
     S.bad |= bad;
-    S.Emin = min(S.Emin, emin);
+    S.rows |= rows << (h < 4 ? 0 : 2);
+    d = (uint32_t)(S.E - eh);
     if (eh > S.E) {
       const uint32_t up = (uint32_t)(eh - S.E);
+      S.bad |= S.E != 0 && up > kFixSpan;
 #pragma unroll
-      for (int i = 0; i < 2; i++)
+      for (int a = 0; a < N; a++) {
 #pragma unroll
-        for (int a = 0; a < N; a++)
+        for (int i = 0; i < 2; i++)
 #pragma unroll
           for (int c = 0; c < 2; c++) {
             S.up[i][a][c] = asr(S.up[i][a][c], up);
             S.lo[i][a][c] = asr(S.lo[i][a][c], up);
           }
+        S.mag[a] = fix_mag_shift(S.mag[a], up);
+      }
       S.E = eh;
+      d = 0;
     }
-    d = (uint32_t)(S.E - eh);
+    S.bad |= eh != 0 && d > kFixSpan;
   }
   // lower rows: lo(u) += s g(u_perm) (im ? i : 1) t_u
-  __device__ __forceinline__ void put(int a, int i, long long re, long long im) {
-    const long long t0 = asr(re, d), t1 = asr(im, d), m = fix_lower_sign(A, h, i);
-    S.up[i][a][0] += t0;
-    S.up[i][a][1] += t1;
-    const bool imag = !((h >> 1) & 1);
-    const long long mr = m ^ (imag ? -1ll : 0ll);
-    S.lo[i][a][0] += ((imag ? t1 : t0) ^ mr) - mr;
-    S.lo[i][a][1] += ((imag ? t0 : t1) ^ m) - m;
+  __device__ __forceinline__ void put(int a, const long long (&t)[2][2]) {
+    uint32_t least[2];
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+      const long long t0 = asr(t[i][0], d), t1 = asr(t[i][1], d), m = fix_lower_sign(A, h, i);
+      S.up[i][a][0] += t0;
+      S.up[i][a][1] += t1;
+      const bool imag = !((h >> 1) & 1);
+      const long long mr = m ^ (imag ? -1ll : 0ll);
+      S.lo[i][a][0] += ((imag ? t1 : t0) ^ mr) - mr;
+      S.lo[i][a][1] += ((imag ? t0 : t1) ^ m) - m;
+      least[i] = fix_least(t0, t1);
+    }
+    S.mag[a] += __byte_perm(least[0], least[1], 0x7632);
   }
 };
 
@@ -359,9 +409,34 @@ __device__ __forceinline__ void fix_hop_into(FixAcc<N>& S, const DslashArgs& A, 
   fix_hop_products<N, SHARED>(add, A, X, rhs, links, h);
 }
 
-// whether a site's sums hold: E, Emin the largest and smallest exponents of its hops
-__device__ __forceinline__ bool fix_holds(bool bad, int E, int Emin) {
-  return !bad && (E == 0 || (E >= 1100 && E <= 3000 && E - Emin <= kFixSpan));
+// whether a site's exponents are within the format (E: the largest of a hop; 0: all zeros)
+__device__ __forceinline__ bool fix_exponent_holds(int E) { return E == 0 || (E >= 1100 && E <= 3000); }
+
+// A site's sums carry an absolute error of about a unit (1.3 to 1.6 rms: the left-out low x low products and the
+// roundings to the unit).  FP64 multiply-adds have none where all the products of a part are small, and a link
+// part or a spinor part 2^-k of its largest has only B - k bits here.  So a part holds if the magnitudes of its
+// eight hops' products add up to kFixMag 2^48 units, or if they are exact zeros (its projected rows are zero in
+// every hop), and a site with a part that does not hold takes FP64.  Over random, near-unit, unit and widely scaled
+// links and full, one-colour, one-spin, real, point-like and widely scaled spinors the error of the parts that hold,
+// relative to the sum of their products' magnitudes, is below that of FP64 multiply-adds: for SU(3) rms 0.07 to
+// 0.63 2^-53 against 0.19 to 0.71, largest 0.6 to 4.6 2^-53 against 1.5 to 4.7.  Of random sites (Haar links,
+// Gaussian spinors) about 1e-8 do not hold.  For SU(3) and SU(4) the smaller of a complex product's two parts
+// stands for both, and one register holds both rows of a colour: with a sum for every part the registers spill,
+// SU(3) 24^3x48 nrhs 12 2330 us against 1747.
+template <int N>
+__device__ __forceinline__ bool fix_parts_hold(const FixAcc<N>& S) {
+  bool ok = true;
+#pragma unroll
+  for (int a = 0; a < N; a++) {
+    const uint32_t m = fix_mag_shift(S.mag_xy[a], (uint32_t)(S.E - S.E_xy));
+    const uint32_t xy[2] = {m & 0xffffu, m >> 16}, zt[2] = {S.mag[a] & 0xffffu, S.mag[a] >> 16};
+#pragma unroll
+    for (int i = 0; i < 2; i++) {  // the upper row i, and the lower row 2 + i, which takes the other row of x and y
+      ok &= (S.rows & (5u << i)) == 0 || xy[i] + zt[i] >= kFixMag<N>;
+      ok &= (S.rows & ((2u >> i) | (4u << i))) == 0 || xy[1 - i] + zt[i] >= kFixMag<N>;
+    }
+  }
+  return ok;
 }
 
 // links: the site's records in shared memory (SHARED)
@@ -374,24 +449,28 @@ __device__ __forceinline__ void fix_site(const DslashArgs& A, const SiteXyzt& X,
 #pragma unroll
     for (int a = 0; a < N; a++) S.up[i][a][0] = S.up[i][a][1] = S.lo[i][a][0] = S.lo[i][a][1] = 0;
   // one hop body for all eight (its gamma chosen by selects): with a body each for the imaginary and the
-  // real gammas the instruction cache cost more than the selects, 1720 against 1685 us at SU(3) 24^3x48
-  // nrhs 12, and 914 against 772 at SU(4) 16^3x32 nrhs 16, 128 registers
+  // real gammas the instruction cache cost more than the selects, by 2% at SU(3) 24^3x48 nrhs 12 and by 18%
+  // at SU(4) 16^3x32 nrhs 16, 128 registers
 #pragma unroll 1
   for (int h = 0; h < 8; h++) {
     fix_hop_into<N, SHARED>(S, A, X, rhs, links, h);
     if (h == 3) {
+      S.E_xy = S.E;
 #pragma unroll
-      for (int a = 0; a < N; a++)
+      for (int a = 0; a < N; a++) {
 #pragma unroll
         for (int c = 0; c < 2; c++) {
           const long long v = S.lo[0][a][c];
           S.lo[0][a][c] = S.lo[1][a][c];
           S.lo[1][a][c] = v;
         }
+        S.mag_xy[a] = S.mag[a];
+        S.mag[a] = 0;
+      }
     }
   }
 
-  if (!fix_holds(S.bad, S.E, S.Emin)) {
+  if (S.bad || !fix_exponent_holds(S.E) || !fix_parts_hold(S)) {
     fp64_site<N>(A, X, rhs);
     return;
   }
@@ -460,11 +539,11 @@ __device__ __forceinline__ void fix_block(const DslashArgs& A, uint32_t gid0) {
 // h + 8 (complex parts).  The sums take the hops in the same order and by the same shifts, so the result is
 // the same to the bit.  For launches with about a warp a scheduler, whose time is one thread's chain of
 // hops; where the GPU is full, the exchange and the links converted by every thread cost more.  One
-// thread a site and RHS / eight, us: SU(3) 8^4 nrhs 1 22 / 7.6, nrhs 4 22 / 11.7, 12^3x24 nrhs 1 27 / 19,
-// 14x10x6x18 nrhs 5 27 / 29, 24^3x48 nrhs 12 1685 / 2369; SU(4) 8^4 nrhs 2 37 / 10.7.  The autotuner
+// thread a site and RHS / eight, us: SU(3) 8^4 nrhs 1 23 / 8.6, nrhs 4 23 / 12.7, 12^3x24 nrhs 1 29 / 21,
+// 14x10x6x18 nrhs 5 27 / 33, 24^3x48 nrhs 12 1747 / 2808; SU(4) 8^4 nrhs 2 36 / 10.9.  The autotuner
 // times both.
 template <int N>
-constexpr uint32_t kFixSplitUnit = 8 * (4 * N * 8 + 8);  // bytes of a site and RHS
+constexpr uint32_t kFixSplitUnit = 8 * (4 * N * 8 + 8) + 8;  // bytes of a site and RHS
 // the largest block up to `block` whose products stay within 48 KB
 template <int N>
 int fix_split_block_size(int block) {
@@ -475,13 +554,16 @@ int fix_split_block_size(int block) {
 template <int N>
 struct FixShare {
   long long* v;  // [4 N][U] of this hop: part (2 i N + 2 a + c)
-  int2* e;       // exponent, smallest exponent
+  int2* e;       // exponent; rows that are not zero, and bit 2: not for fixed point
   uint32_t U;
-  static constexpr int kBad = -(1 << 20);
-  __device__ __forceinline__ void begin(int eh, int emin, bool bad) { *e = make_int2(eh, bad ? kBad : emin); }
-  __device__ __forceinline__ void put(int a, int i, long long re, long long im) {
-    v[(2 * (i * N + a)) * U] = re;
-    v[(2 * (i * N + a) + 1) * U] = im;
+  __device__ __forceinline__ void begin(int eh, uint32_t rows, bool bad) {
+    *e = make_int2(eh, (int)(rows | (bad ? 4u : 0u)));
+  }
+  __device__ __forceinline__ void put(int a, const long long (&t)[2][2]) {
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+#pragma unroll
+      for (int c = 0; c < 2; c++) v[(2 * (i * N + a) + c) * U] = t[i][c];
   }
 };
 
@@ -491,6 +573,7 @@ __device__ __forceinline__ void fix_split_block(const DslashArgs& A, uint32_t bl
   const uint32_t U = blockDim.x / 8, h = threadIdx.x / U, u = threadIdx.x - h * U;
   long long* vals = reinterpret_cast<long long*>(fix_smem);
   int2* exps = reinterpret_cast<int2*>(vals + 8 * 4 * N * U);
+  int* fails = reinterpret_cast<int*>(exps + 8 * U);  // [U] the site does not hold
   const uint32_t vh = (uint32_t)A.geo.vh, nrhs = (uint32_t)A.nrhs, cs = vh * nrhs;
   uint32_t site, rhs;
   A.div_groups.divmod(blk * U + u, site, rhs);
@@ -499,6 +582,7 @@ __device__ __forceinline__ void fix_split_block(const DslashArgs& A, uint32_t bl
   const uint32_t o = X.site * nrhs + rhs;
   constexpr int K = (4 * N + 7) / 8;
   double2 xv[K];
+  if (h == 0) fails[u] = 0;
   if (live) {
     if (A.x) {
 #pragma unroll
@@ -509,16 +593,74 @@ __device__ __forceinline__ void fix_split_block(const DslashArgs& A, uint32_t bl
     fix_hop_products<N, false>(share, A, X, rhs, nullptr, (int)h);
   }
   __syncthreads();
-  if (!live) return;
 
-  int E = 0, Emin = 8191;
+  double2 r[K];
+  bool bad = false;
+  if (live) {
+    uint32_t rows = 0;
+    int E = 0;
 #pragma unroll
-  for (int g = 0; g < 8; g++) {
-    const int2 e = exps[g * U + u];
-    E = max(E, e.x);
-    Emin = min(Emin, e.y);
+    for (int g = 0; g < 8; g++) {
+      const int2 e = exps[g * U + u];
+      rows |= (uint32_t)(e.y & 3) << (g < 4 ? 0 : 2);
+      bad |= (e.y & 4) != 0 || (E != 0 && e.x - E > kFixSpan) || (e.x != 0 && E - e.x > kFixSpan);
+      E = max(E, e.x);
+    }
+    bad |= !fix_exponent_holds(E);
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+      const uint32_t comp = h + 8 * k;
+      if (comp >= 4 * N) break;
+      const int row = (int)comp / N, a = (int)comp - row * N;
+      // the projected rows that feed this one, of x and y and of z and t
+      const int i0 = row < 2 ? row : 3 - row, i1 = row < 2 ? row : row - 2;
+      long long s0 = 0, s1 = 0;
+      uint32_t m0 = 0, m1 = 0;  // SU(3), SU(4): as FixAcc::mag and mag_xy; else |real part| and |imaginary part|
+      int Es = 0;
+#pragma unroll
+      for (int g = 0; g < 8; g++) {
+        const int mu = g >> 1, eg = exps[g * U + u].x, i = mu < 2 ? i0 : i1;
+        if (eg > Es) {
+          const uint32_t up = (uint32_t)(eg - Es);
+          s0 = asr(s0, up);
+          s1 = asr(s1, up);
+          m0 = fix_mag_shift(m0, up);
+          m1 = fix_mag_shift(m1, up);
+          Es = eg;
+        }
+        const uint32_t d = (uint32_t)(Es - eg);
+        const long long* v = vals + ((g * 4 * N + 2 * (i * N + a)) * U + u);
+        const long long t0 = asr(v[0], d), t1 = asr(v[U], d);
+        if constexpr (fix_split_only(N)) {
+          const bool imag = row >= 2 && !(mu & 1);
+          m0 += (uint32_t)abs((int32_t)((imag ? t1 : t0) >> 32)) >> 16;
+          m1 += (uint32_t)abs((int32_t)((imag ? t0 : t1) >> 32)) >> 16;
+        } else {
+          m0 += fix_least(t0, t1) >> 16;
+          if (g == 3) m1 = m0, m0 = 0;
+        }
+        if (row < 2) {
+          s0 += t0;
+          s1 += t1;
+        } else {
+          const long long m = fix_lower_sign(A, g, i);
+          if (!(mu & 1)) {
+            s0 -= (t1 ^ m) - m;
+            s1 += (t0 ^ m) - m;
+          } else {
+            s0 += (t0 ^ m) - m;
+            s1 += (t1 ^ m) - m;
+          }
+        }
+      }
+      bad |= (rows & ((1u << i0) | (4u << i1))) != 0 && (fix_split_only(N) ? min(m0, m1) : m0 + m1) < kFixMag<N>;
+      r[k] = make_double2(from_fix(s0, Es + kFixBias<N>), from_fix(s1, Es + kFixBias<N>));
+    }
+    if (bad) fails[u] = 1;
   }
-  if (!fix_holds(Emin <= FixShare<N>::kBad, E, Emin)) {
+  const bool any = __syncthreads_or(bad);
+  if (!live) return;
+  if (any && fails[u]) {
     if (h == 0) fp64_site<N>(A, X, rhs);
     return;
   }
@@ -527,45 +669,16 @@ __device__ __forceinline__ void fix_split_block(const DslashArgs& A, uint32_t bl
   for (int k = 0; k < K; k++) {
     const uint32_t comp = h + 8 * k;
     if (comp >= 4 * N) break;
-    const int row = (int)comp / N, a = (int)comp - row * N;
-    long long s0 = 0, s1 = 0;
-    int Es = 0;
-#pragma unroll
-    for (int g = 0; g < 8; g++) {
-      const int mu = g >> 1, eg = exps[g * U + u].x;
-      if (eg > Es) {
-        s0 = asr(s0, (uint32_t)(eg - Es));
-        s1 = asr(s1, (uint32_t)(eg - Es));
-        Es = eg;
-      }
-      const int i = row < 2 ? row : mu < 2 ? 3 - row : row - 2;  // the projected row that feeds this one
-      const long long* v = vals + ((g * 4 * N + 2 * (i * N + a)) * U + u);
-      const long long t0 = asr(v[0], (uint32_t)(Es - eg)), t1 = asr(v[U], (uint32_t)(Es - eg));
-      if (row < 2) {
-        s0 += t0;
-        s1 += t1;
-      } else {
-        const long long m = fix_lower_sign(A, g, i);
-        if (!(mu & 1)) {
-          s0 -= (t1 ^ m) - m;
-          s1 += (t0 ^ m) - m;
-        } else {
-          s0 += (t0 ^ m) - m;
-          s1 += (t1 ^ m) - m;
-        }
-      }
-    }
-    double2 r = make_double2(from_fix(s0, Es + kFixBias<N>), from_fix(s1, Es + kFixBias<N>));
     // store_out's operations
     if (A.x) {
       if (A.b == 1.0)
-        r = make_double2(fma(ca, r.x, xv[k].x), fma(ca, r.y, xv[k].y));
+        r[k] = make_double2(fma(ca, r[k].x, xv[k].x), fma(ca, r[k].y, xv[k].y));
       else
-        r = make_double2(fma(A.b, xv[k].x, ca * r.x), fma(A.b, xv[k].y, ca * r.y));
+        r[k] = make_double2(fma(A.b, xv[k].x, ca * r[k].x), fma(A.b, xv[k].y, ca * r[k].y));
     } else if (A.a_rhs_d || A.a != 1.0) {
-      r = make_double2(r.x * ca, r.y * ca);
+      r[k] = make_double2(r[k].x * ca, r[k].y * ca);
     }
-    static_cast<double2*>(A.out)[o + comp * cs] = r;
+    static_cast<double2*>(A.out)[o + comp * cs] = r[k];
   }
 }
 
