@@ -30,8 +30,7 @@
 // than kFixSpan binades apart, when anything it reads is infinite or NaN, and when the result could leave the
 // normal range.  Where a field's structure sends every site there, a hop takes the time of both: one-colour
 // spinors on near-unit links, us, against FP64 multiply-adds alone: SU(3) 24^3x48 nrhs 12 6850 / 5763, SU(4)
-// 16^3x32 nrhs 16 2970 / 2460, SU(6) 16^3x32 nrhs 16 15100 / 4978 (one thread
-// of eight does the FP64 site).
+// 16^3x32 nrhs 16 2970 / 2460, SU(6) 16^3x32 nrhs 16 8340 / 4978.
 #pragma once
 
 namespace qcu {
@@ -541,7 +540,7 @@ __device__ __forceinline__ void fix_block(const DslashArgs& A, uint32_t gid0) {
 // hops; where the GPU is full, the exchange and the links converted by every thread cost more.  One
 // thread a site and RHS / eight, us: SU(3) 8^4 nrhs 1 23 / 8.6, nrhs 4 23 / 12.7, 12^3x24 nrhs 1 29 / 21,
 // 14x10x6x18 nrhs 5 27 / 33, 24^3x48 nrhs 12 1747 / 2808; SU(4) 8^4 nrhs 2 36 / 10.9.  The autotuner
-// times both.
+// times both.  A site that takes FP64 does so on its eight threads too.
 template <int N>
 constexpr uint32_t kFixSplitUnit = 8 * (4 * N * 8 + 8) + 8;  // bytes of a site and RHS
 // the largest block up to `block` whose products stay within 48 KB
@@ -566,6 +565,60 @@ struct FixShare {
       for (int c = 0; c < 2; c++) v[(2 * (i * N + a) + c) * U] = t[i][c];
   }
 };
+
+// hop h's products in FP64 multiply-adds, by fp64_site's operations, to where FixShare has them
+template <int N>
+__device__ __noinline__ void fp64_hop_products(double* v, uint32_t U, const DslashArgs& A, const SiteXyzt& X, uint32_t rhs,
+                                               int h) {
+  const uint32_t nb = X.neighbour(A, h);
+  double2 x[2][N], y[2][N];
+  fix_load<N>(x, y, A, nb, rhs, h >> 1);
+  fix_project<N>(x, y, A, h);
+  const FixLinkAt<N> at(A, X, h, nb);
+#pragma unroll 1
+  for (int a = 0; a < N; a++) {
+    double2 t[2];
+#pragma unroll
+    for (int b = 0; b < N; b++) {
+      const double2 u = at.load(a, b);
+      const double ur = flip_sign(u.x, at.rf != 0), ui = flip_sign(u.y, at.jf != 0);
+#pragma unroll
+      for (int i = 0; i < 2; i++) {
+        t[i].x = b ? fma(ur, x[i][b].x, t[i].x) : ur * x[i][b].x;
+        t[i].y = b ? fma(ur, x[i][b].y, t[i].y) : ur * x[i][b].y;
+        t[i].x = fma(-ui, x[i][b].y, t[i].x);
+        t[i].y = fma(ui, x[i][b].x, t[i].y);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+      v[(2 * (i * N + a)) * U] = t[i].x;
+      v[(2 * (i * N + a) + 1) * U] = t[i].y;
+    }
+  }
+}
+
+// the component comp (complex part of row comp / N) of a site and RHS: the eight hops' products summed in FP64
+template <int N>
+__device__ __noinline__ double2 fp64_sum(const double* vals, uint32_t U, uint32_t u, const DslashArgs& A, uint32_t comp) {
+  const int row = (int)comp / N, a = (int)comp - row * N;
+  double2 s;
+#pragma unroll 1
+  for (int g = 0; g < 8; g++) {
+    const int mu = g >> 1, i = row < 2 ? row : mu < 2 ? 3 - row : row - 2;
+    const double* v = vals + ((g * 4 * N + 2 * (i * N + a)) * U + u);
+    double re = v[0], im = v[U];
+    if (row >= 2) {
+      const bool neg = fix_lower_sign(A, g, i) != 0, imag = !(mu & 1);
+      const double t = re;
+      re = flip_sign(imag ? im : re, neg != imag);
+      im = flip_sign(imag ? t : im, neg);
+    }
+    s.x = g ? s.x + re : re;
+    s.y = g ? s.y + im : im;
+  }
+  return s;
+}
 
 template <int N>
 __device__ __forceinline__ void fix_split_block(const DslashArgs& A, uint32_t blk) {
@@ -658,12 +711,18 @@ __device__ __forceinline__ void fix_split_block(const DslashArgs& A, uint32_t bl
     }
     if (bad) fails[u] = 1;
   }
-  const bool any = __syncthreads_or(bad);
-  if (!live) return;
-  if (any && fails[u]) {
-    if (h == 0) fp64_site<N>(A, X, rhs);
-    return;
+  if (__syncthreads_or(bad)) {  // FP64 multiply-adds for the sites that do not hold, one hop a thread
+    const bool again = live && fails[u];
+    double* d = reinterpret_cast<double*>(vals);
+    if (again) fp64_hop_products<N>(d + (h * 4 * N * U + u), U, A, X, rhs, (int)h);
+    __syncthreads();
+    if (again) {
+#pragma unroll
+      for (int k = 0; k < K; k++)
+        if (h + 8 * k < 4 * N) r[k] = fp64_sum<N>(d, U, u, A, h + 8 * k);
+    }
   }
+  if (!live) return;
   const double ca = A.a_rhs_d ? A.a_rhs_d[rhs] : A.a;
 #pragma unroll
   for (int k = 0; k < K; k++) {
