@@ -277,6 +277,12 @@ Session::~Session() {
   if (own_stream_) cudaStreamDestroy(own_stream_);
 }
 
+bool Session::capturing() {
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  QCU_CHECK_CUDA(cudaStreamIsCapturing(stream(), &cs));
+  return cs != cudaStreamCaptureStatusNone;
+}
+
 cudaStream_t Session::stream() {
   if (user_stream_) return user_stream_;
   if (!own_stream_)
@@ -323,6 +329,7 @@ const void* Session::gauge12(int prec) {
   if (prec == PREC_BF16S) prec = PREC_BF16;
   if (N != 3 || prec == PREC_DOUBLE) return nullptr;  // the fixed-point FP64 hop takes the full links
   if (su3_dev_ < 0) {
+    if (capturing()) return nullptr;
     unsigned* scratch = static_cast<unsigned*>(su3_scratch_.ensure(16));
     su3_dev_ = su3_row_deviation(gauge_[PREC_DOUBLE].get(), geo.vh, scratch, stream());
   }
@@ -330,6 +337,7 @@ const void* Session::gauge12(int prec) {
   const double tol = prec == PREC_SINGLE ? 1e-7 : 1e-4;
   if (!(su3_dev_ < tol)) return nullptr;
   if (!gauge12_valid_[prec]) {
+    if (capturing()) return nullptr;
     const size_t vhp = ((size_t)geo.vh + 31) / 32 * 32;  // the two-row layout's groups of 32 sites
     void* d = gauge12_[prec].ensure(48 * vhp * prec_complex_bytes(prec));
     compress_gauge_su3(gauge_[PREC_DOUBLE].get(), prec, d, geo.vh, stream());
@@ -341,6 +349,7 @@ const void* Session::gauge12(int prec) {
 const void* Session::gauge_tc() {
   QCU_REQUIRE(gauge_loaded_, QCU_ERR_NO_GAUGE, "localGauge_ is nullptr, not loaded.\n");
   if (!gauge_tc_valid_) {
+    if (capturing()) return nullptr;
     void* d = gauge_tc_.ensure(tc_links_bytes(geo.vh));
     gauge_tc_records_bf16(N, gauge_[PREC_DOUBLE].get(), d, geo, stream());
     gauge_tc_valid_ = true;
@@ -352,6 +361,7 @@ const void* Session::gauge_rec(int prec) {
   QCU_REQUIRE(gauge_loaded_, QCU_ERR_NO_GAUGE, "localGauge_ is nullptr, not loaded.\n");
   const int i = prec == PREC_HALF ? 0 : 1;
   if (!gauge_rec_valid_[i]) {
+    if (capturing()) return nullptr;
     void* d = gauge_rec_[i].ensure(site_records_bytes(geo.vh, N));
     gauge_site_records(prec == PREC_HALF ? PREC_HALF : PREC_BF16, N, gauge_[PREC_DOUBLE].get(), d, geo, stream());
     gauge_rec_valid_[i] = true;
@@ -429,9 +439,7 @@ bool Session::prefer_site_major(FieldView a, FieldView b) {
   bool known = false;
   const bool cached = tuner.layout_site_major(N, nrhs, geo.vh, &known);
   if (known) return cached;
-  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-  QCU_CHECK_CUDA(cudaStreamIsCapturing(stream(), &cs));
-  if (cs != cudaStreamCaptureStatusNone) return false;
+  if (capturing()) return false;
   // zero input (the bytes are the same in both layouts), then each layout's
   // tuned dslash: one untimed application (tunes it), three timed
   QCU_CHECK_CUDA(cudaMemsetAsync(a.data, 0, field_bytes(PREC_BF16, nrhs), stream()));
@@ -493,13 +501,9 @@ void Session::hop(FieldView out, FieldView in, FieldView x, int parity, int dagg
   A.antiperiodic_t = antiperiodic_t ? 1 : 0;
   bool found = false;
   DslashConfig c = tuner.lookup(in.prec, N, in.nrhs, geo.vh, &found);
-  bool tunes = false;
-  if (!found && tuner.enabled()) {
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    QCU_CHECK_CUDA(cudaStreamIsCapturing(stream(), &cs));
-    tunes = cs == cudaStreamCaptureStatusNone;
-  }
-  if (tunes || c.rc) A.gauge12 = gauge12(in.prec);  // measured and built on first use
+  const bool tunes = !found && tuner.enabled() && !capturing();
+  // built by the first hop on the loaded links, whatever its shape: a captured hop of another shape finds them
+  A.gauge12 = gauge12(in.prec);
   tensor_links(A, in.prec, tunes ? -1 : c.tc);
   if (tunes) c = tuner.tune(A, in.prec, N, stream());
   launch_dslash(A, in.prec, N, c, stream());
@@ -509,6 +513,11 @@ void Session::tensor_links(DslashArgs& A, int prec, int tc) {
   if (!prec_is16(prec) || A.nrhs % 4) return;  // the RHS counts that these kernels take
   if (tc < 0 || tc == kMmaVariant) A.gauge_rec = gauge_rec(prec);
   if (prec_bf16(prec) && (tc < 0 || (tc >= 4 && tc != kMmaVariant))) A.gauge_tc = gauge_tc();
+  // captured before the form that tc reads was built: site-major fields have only these kernels
+  if (prec_site_major(prec) && !A.gauge_rec && !A.gauge_tc) {
+    A.gauge_rec = gauge_rec_valid_[1] ? gauge_rec_[1].get() : nullptr;
+    A.gauge_tc = gauge_tc_valid_ ? gauge_tc_.get() : nullptr;
+  }
 }
 
 Blas& Session::blas() {

@@ -159,6 +159,7 @@ class Session {
   // capture CUDA graphs on worker threads, and a capture on a blocking stream
   // makes every legacy-stream call of other threads fail meanwhile.
   bool nonblocking_stream = false;
+  bool capturing();  // whether the stream is being captured
   cudaStream_t stream();
   void set_user_stream(cudaStream_t s) { user_stream_ = s; }
   void sync();
@@ -179,6 +180,8 @@ class Session {
   // (layout.h gauge_site_records), for the register-fragment MMA dslash;
   // built on first use
   const void* gauge_rec(int prec);
+  // These forms are not built while the stream is captured (nullptr unless
+  // they are there): the launch then takes a kernel that reads what is.
   // sets in A the link forms that tensor-core variant tc reads (0: none; -1: any, for tuning)
   void tensor_links(DslashArgs& A, int prec, int tc);
 
