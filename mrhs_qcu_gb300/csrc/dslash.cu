@@ -162,7 +162,7 @@ void launch_dslash(const DslashArgs& A_in, int prec, int N, const DslashConfig& 
   DslashArgs A = A_in;
   A.site_major = prec_site_major(prec) ? 1 : 0;
   if (A.site_major && !(cfg.tc >= 4 && tc_runs(A, prec, N, cfg.tc))) {
-    // site-major fields have only the spinor-operand tensor-core kernels: the first that runs
+    // site-major fields have only the tensor-core kernels from variant 4 on: the first that runs
     cfg = DslashConfig{};
     for (int v = 4; v <= kTcVariants && !cfg.tc; v++)
       if (tc_runs(A, prec, N, v)) cfg.tc = v;

@@ -147,8 +147,8 @@ void Autotuner::store_layout(int N, int nrhs, int vh, bool site_major) {
 
 DslashConfig Autotuner::heuristic(int prec, int N, int nrhs) {
   DslashConfig c;
-  if (prec_site_major(prec)) {  // only the spinor-operand tensor-core kernels take site-major fields
-    c.tc = 4;
+  if (prec_site_major(prec)) {  // only tensor-core kernels take site-major fields
+    c.tc = kMmaVariant;
     return c;
   }
   int opts[8];
@@ -206,12 +206,14 @@ DslashConfig Autotuner::tune(const DslashArgs& A, int prec, int N, cudaStream_t 
     c.tma = ts[i];
     if (tma_runs(A, prec, N, c)) cand.push_back(c);
   }
-  // the tensor-core kernels, where these arguments fit them; at N <= 4 the
-  // CUDA-core kernels were faster than the tcgen05 ones at every RHS count
-  // measured (16^3x32, nrhs 16-64), so component-major fields do not time those there
+  // the tensor-core kernels, where these arguments fit them.  The register-fragment MMAs took
+  // at most 0.88 of the time of the best tcgen05 variant at every shape measured (N = 3..8, nrhs 4-128 in
+  // both layouts, 4^3x8, 8^3x16 and 16^3x32), so these are timed only where it does not run (nrhs not
+  // a multiple of 4), and not at N <= 4, where the CUDA-core kernels were faster than they at every
+  // RHS count (16^3x32, nrhs 16-64)
   for (int variant = 1; variant <= kTcVariants; variant++) {
+    if (variant != kMmaVariant && (N <= 4 || tc_runs(A, prec, N, kMmaVariant))) continue;
     if (!tc_runs(A, prec, N, variant)) continue;
-    if (N <= 4 && !prec_site_major(prec) && variant != kMmaVariant) continue;
     DslashConfig c;
     c.tc = variant;
     cand.push_back(c);
@@ -511,8 +513,15 @@ void Session::hop(FieldView out, FieldView in, FieldView x, int parity, int dagg
 
 void Session::tensor_links(DslashArgs& A, int prec, int tc) {
   if (!prec_is16(prec) || A.nrhs % 4) return;  // the RHS counts that these kernels take
-  if (tc < 0 || tc == kMmaVariant) A.gauge_rec = gauge_rec(prec);
-  if (prec_bf16(prec) && (tc < 0 || (tc >= 4 && tc != kMmaVariant))) A.gauge_tc = gauge_tc();
+  if (tc < 0 || tc == kMmaVariant) {
+    try {
+      A.gauge_rec = gauge_rec(prec);
+    } catch (const Error&) {
+      if (prec_site_major(prec)) throw;
+      A.gauge_rec = nullptr;  // no memory for them: the register kernels need none
+    }
+  }
+  if (prec_bf16(prec) && tc >= 4 && tc != kMmaVariant) A.gauge_tc = gauge_tc();
   // captured before the form that tc reads was built: site-major fields have only these kernels
   if (prec_site_major(prec) && !A.gauge_rec && !A.gauge_tc) {
     A.gauge_rec = gauge_rec_valid_[1] ? gauge_rec_[1].get() : nullptr;

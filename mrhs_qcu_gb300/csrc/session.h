@@ -182,7 +182,7 @@ class Session {
   const void* gauge_rec(int prec);
   // These forms are not built while the stream is captured (nullptr unless
   // they are there): the launch then takes a kernel that reads what is.
-  // sets in A the link forms that tensor-core variant tc reads (0: none; -1: any, for tuning)
+  // sets in A the link forms that tensor-core variant tc reads (0: none; -1: of the variants that tuning times)
   void tensor_links(DslashArgs& A, int prec, int tc);
 
   // ---- clover term (clover.h) ---------------------------------------------
