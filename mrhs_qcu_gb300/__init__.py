@@ -332,12 +332,22 @@ def dslash_segments(segments, n_colors: int, precision: int, stream=None) -> Non
     (qcuDslashSegments).  `segments`: dicts with keys lattice, gauge,
     gauge_two_row (or None), in_, out, x (or None), a, b, nrhs, parity,
     dagger, antiperiodic_t; pointers are device addresses."""
-    data = b"".join(
-        _SEGMENT.pack(*d["lattice"], d["gauge"] or 0, d.get("gauge_two_row") or 0, d["in_"] or 0, d["out"] or 0,
-                      d.get("x") or 0, d.get("a", 1.0), d.get("b", 0.0), d["nrhs"], d.get("parity", 0), d.get("dagger", 0),
-                      bool(d.get("antiperiodic_t", False))) for d in segments)
     n = len(segments)
-    arr = (QcuHopSegment * n).from_buffer_copy(data) if n else (QcuHopSegment * 1)()
+    try:
+        data = b"".join(
+            _SEGMENT.pack(*d["lattice"], d["gauge"] or 0, d.get("gauge_two_row") or 0, d["in_"] or 0, d["out"] or 0,
+                          d.get("x") or 0, d.get("a", 1.0), d.get("b", 0.0), d["nrhs"], d.get("parity", 0),
+                          d.get("dagger", 0), bool(d.get("antiperiodic_t", False))) for d in segments)
+        arr = (QcuHopSegment * n).from_buffer_copy(data) if n else (QcuHopSegment * 1)()
+    except (struct.error, TypeError, OverflowError):  # values that are no plain numbers: the fields' own conversions
+        arr = (QcuHopSegment * max(1, n))()
+        for g, d in zip(arr, segments):
+            g.lattice = (ctypes.c_int * 4)(*d["lattice"])
+            g.gauge, g.gauge_two_row = d["gauge"], d.get("gauge_two_row")
+            g.in_, g.out, g.x = d["in_"], d["out"], d.get("x")
+            g.a, g.b = d.get("a", 1.0), d.get("b", 0.0)
+            g.nrhs, g.parity, g.dagger = d["nrhs"], d.get("parity", 0), d.get("dagger", 0)
+            g.antiperiodic_t = int(bool(d.get("antiperiodic_t", False)))
     _raise_if(lib().qcuDslashSegments(arr, n, int(n_colors), int(precision), _p(stream)))
 
 
