@@ -6,6 +6,8 @@
 // instead of terminating the process (the reference's errorQcu / CHECK_CUDA
 // call exit(1), include/qcu_macro.cuh:16-40); QCU_ABORT_ON_ERROR=1 restores
 // that behaviour.
+#include <cudaTypedefs.h>
+
 #include <atomic>
 #include <cstdio>
 #include <cstdlib>
@@ -127,15 +129,77 @@ void caller_dslash(Session& s, int prec, void* const* outs, void* const* ins, in
   if (wait) s.sync();
 }
 
+// The driver's number of a context, unique for the life of the process: a device reset gives the device's
+// primary context a new one (its handle stays the same, and its memory is gone).  0: no such context.
+class ContextId {
+ public:
+  static unsigned long long current() {
+    const Fns& f = fns();
+    CUcontext c = nullptr;
+    unsigned long long id = 0;
+    if (!f.ok || f.get_current(&c) != CUDA_SUCCESS || !c || f.get_id(c, &id) != CUDA_SUCCESS) return 0;
+    return id;
+  }
+  static unsigned long long primary(int device) {
+    const Fns& f = fns();
+    CUdevice d;
+    CUcontext c;
+    unsigned flags = 0;
+    int active = 0;
+    unsigned long long id = 0;
+    if (!f.ok || f.device(&d, device) != CUDA_SUCCESS || f.state(d, &flags, &active) != CUDA_SUCCESS || !active ||
+        f.retain(&c, d) != CUDA_SUCCESS)
+      return 0;
+    if (f.get_id(c, &id) != CUDA_SUCCESS) id = 0;
+    f.release(d);
+    return id;
+  }
+
+ private:
+  struct Fns {
+    PFN_cuCtxGetCurrent_v4000 get_current = nullptr;
+    PFN_cuCtxGetId_v12000 get_id = nullptr;
+    PFN_cuDeviceGet_v2000 device = nullptr;
+    PFN_cuDevicePrimaryCtxGetState_v7000 state = nullptr;
+    PFN_cuDevicePrimaryCtxRetain_v7000 retain = nullptr;
+    PFN_cuDevicePrimaryCtxRelease_v11000 release = nullptr;
+    bool ok = true;
+    template <typename F>
+    void load(F& f, const char* name, unsigned version) {
+      void* p = nullptr;
+      cudaDriverEntryPointQueryResult q;
+      ok &= cudaGetDriverEntryPointByVersion(name, &p, version, cudaEnableDefault, &q) == cudaSuccess &&
+            q == cudaDriverEntryPointSuccess;
+      f = reinterpret_cast<F>(p);
+    }
+    Fns() {
+      load(get_current, "cuCtxGetCurrent", 4000);
+      load(get_id, "cuCtxGetId", 12000);
+      load(device, "cuDeviceGet", 2000);
+      load(state, "cuDevicePrimaryCtxGetState", 7000);
+      load(retain, "cuDevicePrimaryCtxRetain", 7000);
+      load(release, "cuDevicePrimaryCtxRelease", 11000);
+    }
+  };
+  static const Fns& fns() {
+    static const Fns f;
+    return f;
+  }
+};
+
 // The session of the one-call operators (dslashQcu, fullDslashQcu).  Between
 // calls on one lattice and device it keeps its stream and buffers: setting
 // them up and freeing them took 0.4 of the 0.59 ms of a 12^3x24 call.  At most kKeepBytes stay
 // allocated; another lattice, initGridSize and an allocation that would fail
-// free them.  Used under the API lock; `busy` keeps an allocation of a solve
+// free them.  A device reset frees them too, without a word to the library, and may give
+// their addresses to the program's next allocations: a session is kept only in a device's
+// primary context, and one whose context is gone is forgotten, not freed.
+// Used under the API lock; `busy` keeps an allocation of a solve
 // server's thread from freeing it during a call.
 class OneCall {
  public:
   static constexpr size_t kKeepBytes = (size_t)256 << 20;
+  ~OneCall() { (void)s_.release(); }  // the process ends: its memory goes with its contexts
   template <typename F>
   void run(const QcuParam& p, F&& f) {
     while (busy_.exchange(true)) std::this_thread::yield();
@@ -143,19 +207,27 @@ class OneCall {
       OneCall& o;
       bool ok = false;
       ~Done() {
-        if (!ok || (o.s_ && o.s_->device_bytes() > kKeepBytes)) o.s_.reset();
+        const unsigned long long now = ContextId::current();
+        o.context_ = now && now == ContextId::primary(o.device_) ? now : 0;
+        if (!ok || !o.context_ || (o.s_ && o.s_->device_bytes() > kKeepBytes)) o.s_.reset();
         o.busy_.store(false);
       }
-    } done{*this};
+    };
     int dev = 0;
-    QCU_CHECK_CUDA(cudaGetDevice(&dev));
-    bool same = s_ && dev == device_;
-    for (int i = 0; same && i < 4; i++) same = s_->latt.dim[i] == p.lattice_size[i];
-    if (!same) {
-      s_.reset();
+    try {
+      QCU_CHECK_CUDA(cudaGetDevice(&dev));
+      bool same = s_ && dev == device_ && context_ == ContextId::current();
+      for (int i = 0; same && i < 4; i++) same = s_->latt.dim[i] == p.lattice_size[i];
+      if (!same) drop();
+    } catch (...) {
+      busy_.store(false);
+      throw;
+    }
+    device_ = dev;
+    Done done{*this};
+    if (!s_) {
       const int g[4] = {1, 1, 1, 1};
       s_.reset(new Session(p.lattice_size, g, 3));
-      device_ = dev;
     }
     apply_settings(*s_);
     f(*s_);
@@ -163,15 +235,28 @@ class OneCall {
   }
   bool release() {
     if (busy_.exchange(true)) return false;
-    const bool had = s_ != nullptr;
-    s_.reset();
+    const bool freed = drop();
     busy_.store(false);
-    return had;
+    return freed;
   }
 
  private:
+  // true if there was a session and its memory is freed
+  bool drop() {
+    if (!s_) return false;
+    if (!context_ || context_ != ContextId::primary(device_)) {
+      (void)s_.release();
+      return false;
+    }
+    int dev = 0;
+    const bool other = cudaGetDevice(&dev) == cudaSuccess && dev != device_ && cudaSetDevice(device_) == cudaSuccess;
+    s_.reset();
+    if (other) cudaSetDevice(dev);
+    return true;
+  }
   std::unique_ptr<Session> s_;
   int device_ = 0;
+  unsigned long long context_ = 0;  // of the session between calls
   std::atomic<bool> busy_{false};
 };
 OneCall g_one_call;
