@@ -3,9 +3,9 @@
 #pragma once
 
 #include <cstring>
-#include <mutex>
 #include <type_traits>
 
+#include "context.h"
 #include "dslash.h"
 #include "dslash_mma.cuh"
 #include "dslash_tc.cuh"
@@ -56,11 +56,8 @@ void launch_wilson_tcs(const DslashArgs& A, cudaStream_t st) {
   T.err = tma_error_flag();
   const size_t smem = tcs::smem_bytes(NST, NB, HV);
   const void* k = reinterpret_cast<const void*>(&wilson_tcs_kernel<N, NST, NB, HV>);
-  static size_t smem_set = 0;
-  if (smem > 48 * 1024 && smem > smem_set) {
-    QCU_CHECK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    smem_set = smem;
-  }
+  static DynamicSmem limit;
+  limit.ensure(k, smem);
   const int grid = tc_grid(k, T.ntiles, smem, (int)tcs::kTmemCols, tcs::kThreads);
   wilson_tcs_kernel<N, NST, NB, HV><<<grid, tcs::kThreads, smem, st>>>(T, mi);
   tma_note_launch();
@@ -80,11 +77,8 @@ void launch_wilson_mma_shape(const DslashArgs& A, cudaStream_t st) {
   plan_site_order(T.A, P, N);
   const size_t smem = (size_t)mma::kWarps * 4 * mma::warp_words(P, N, S, MT, NST);
   auto* const k = &wilson_mma_kernel<P, N, S, MT, NST, L1>;
-  static std::once_flag smem_set;  // the size is the instance's own
-  if (smem > 48 * 1024)
-    std::call_once(smem_set, [&] {
-      QCU_CHECK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    });
+  static DynamicSmem limit;
+  limit.ensure(reinterpret_cast<const void*>(k), smem);
   k<<<(T.warps + mma::kWarps - 1) / mma::kWarps, 32 * mma::kWarps, smem, st>>>(T);
 }
 
@@ -129,11 +123,8 @@ void launch_wilson_tc(const DslashArgs& A, cudaStream_t st) {
   else
     memset(&mi, 0, sizeof(mi));  // not read
   const void* k = reinterpret_cast<const void*>(&wilson_tc_kernel<N, NST>);
-  static size_t smem_set = 0;
-  if (smem > 48 * 1024 && smem > smem_set) {
-    QCU_CHECK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    smem_set = smem;
-  }
+  static DynamicSmem limit;
+  limit.ensure(k, smem);
   const int grid = tc_grid(k, T.ntiles, smem);
   wilson_tc_kernel<N, NST><<<grid, 128, smem, st>>>(T, mi);
   tma_note_launch();

@@ -5,6 +5,7 @@
 
 #include <cuda.h>
 
+#include "context.h"
 #include "dslash.h"
 #include "dslash_tma.cuh"
 
@@ -67,11 +68,8 @@ void launch_wilson_tma(const DslashArgs& A, int rcta, cudaStream_t st) {
   else
     mn = mg;  // not read
   const void* k = reinterpret_cast<const void*>(&wilson_tma_kernel<P, N, R, NST>);
-  static size_t smem_set = 0;  // the attribute only grows; set outside graph capture by the first launch
-  if (smem > smem_set) {
-    QCU_CHECK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    smem_set = smem;
-  }
+  static DynamicSmem limit;
+  limit.ensure(k, smem);
   const int grid = tma_grid(k, threads, smem, T.ntiles);
   wilson_tma_kernel<P, N, R, NST><<<grid, threads, smem, st>>>(T, mi, mg, mn);
   tma_note_launch();

@@ -168,11 +168,8 @@ void launch_wilson_tmalink(const DslashArgs& A, int /*block*/, cudaStream_t st) 
     tma_encode_gauge(&mg, A.gauge, (int)sizeof(E), A.geo.vh, NN, A.geo.hx);
   const size_t smem = tmalink_smem_bytes(NN, A.geo.hx, (int)sizeof(E));
   const void* k = reinterpret_cast<const void*>(&wilson_tmalink_kernel<P, N, R, MINB, RC>);
-  static size_t smem_set = 48 * 1024;  // the attribute only grows; set outside graph capture by the first launch
-  if (smem > smem_set) {
-    QCU_CHECK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    smem_set = smem;
-  }
+  static DynamicSmem limit;
+  limit.ensure(k, smem);
   const int rows = A.geo.vh / A.geo.hx;
   const int threads = A.geo.hx * (A.nrhs / R);
   static int max_threads = 0;

@@ -6,8 +6,6 @@
 // instead of terminating the process (the reference's errorQcu / CHECK_CUDA
 // call exit(1), include/qcu_macro.cuh:16-40); QCU_ABORT_ON_ERROR=1 restores
 // that behaviour.
-#include <cudaTypedefs.h>
-
 #include <atomic>
 #include <cstdio>
 #include <cstdlib>
@@ -22,6 +20,7 @@
 #include "../../include/qcu.h"
 #include "../../include/qcu_gb300.h"
 #pragma GCC visibility pop
+#include "context.h"
 #include "dslash_tc.h"
 #include "dslash_tma.h"
 #include "serve.h"
@@ -129,64 +128,6 @@ void caller_dslash(Session& s, int prec, void* const* outs, void* const* ins, in
   if (wait) s.sync();
 }
 
-// The driver's number of a context, unique for the life of the process: a device reset gives the device's
-// primary context a new one (its handle stays the same, and its memory is gone).  0: no such context.
-class ContextId {
- public:
-  static unsigned long long current() {
-    const Fns& f = fns();
-    CUcontext c = nullptr;
-    unsigned long long id = 0;
-    if (!f.ok || f.get_current(&c) != CUDA_SUCCESS || !c || f.get_id(c, &id) != CUDA_SUCCESS) return 0;
-    return id;
-  }
-  static unsigned long long primary(int device) {
-    const Fns& f = fns();
-    CUdevice d;
-    CUcontext c;
-    unsigned flags = 0;
-    int active = 0;
-    unsigned long long id = 0;
-    if (!f.ok || f.device(&d, device) != CUDA_SUCCESS || f.state(d, &flags, &active) != CUDA_SUCCESS || !active ||
-        f.retain(&c, d) != CUDA_SUCCESS)
-      return 0;
-    if (f.get_id(c, &id) != CUDA_SUCCESS) id = 0;
-    f.release(d);
-    return id;
-  }
-
- private:
-  struct Fns {
-    PFN_cuCtxGetCurrent_v4000 get_current = nullptr;
-    PFN_cuCtxGetId_v12000 get_id = nullptr;
-    PFN_cuDeviceGet_v2000 device = nullptr;
-    PFN_cuDevicePrimaryCtxGetState_v7000 state = nullptr;
-    PFN_cuDevicePrimaryCtxRetain_v7000 retain = nullptr;
-    PFN_cuDevicePrimaryCtxRelease_v11000 release = nullptr;
-    bool ok = true;
-    template <typename F>
-    void load(F& f, const char* name, unsigned version) {
-      void* p = nullptr;
-      cudaDriverEntryPointQueryResult q;
-      ok &= cudaGetDriverEntryPointByVersion(name, &p, version, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess;
-      f = reinterpret_cast<F>(p);
-    }
-    Fns() {
-      load(get_current, "cuCtxGetCurrent", 4000);
-      load(get_id, "cuCtxGetId", 12000);
-      load(device, "cuDeviceGet", 2000);
-      load(state, "cuDevicePrimaryCtxGetState", 7000);
-      load(retain, "cuDevicePrimaryCtxRetain", 7000);
-      load(release, "cuDevicePrimaryCtxRelease", 11000);
-    }
-  };
-  static const Fns& fns() {
-    static const Fns f;
-    return f;
-  }
-};
-
 // The session of the one-call operators (dslashQcu, fullDslashQcu).  Between
 // calls on one lattice and device it keeps its stream and buffers: setting
 // them up and freeing them took 0.4 of the 0.59 ms of a 12^3x24 call.  At most kKeepBytes stay
@@ -207,8 +148,8 @@ class OneCall {
       OneCall& o;
       bool ok = false;
       ~Done() {
-        const unsigned long long now = ContextId::current();
-        o.context_ = now && now == ContextId::primary(o.device_) ? now : 0;
+        const unsigned long long now = qcu::ContextId::current();
+        o.context_ = now && now == qcu::ContextId::primary(o.device_) ? now : 0;
         if (!ok || !o.context_ || (o.s_ && o.s_->device_bytes() > kKeepBytes)) o.s_.reset();
         o.busy_.store(false);
       }
@@ -216,7 +157,7 @@ class OneCall {
     int dev = 0;
     try {
       QCU_CHECK_CUDA(cudaGetDevice(&dev));
-      bool same = s_ && dev == device_ && context_ == ContextId::current();
+      bool same = s_ && dev == device_ && context_ == qcu::ContextId::current();
       for (int i = 0; same && i < 4; i++) same = s_->latt.dim[i] == p.lattice_size[i];
       if (!same) drop();
     } catch (...) {
@@ -244,7 +185,7 @@ class OneCall {
   // true if there was a session and its memory is freed
   bool drop() {
     if (!s_) return false;
-    if (!context_ || context_ != ContextId::primary(device_)) {
+    if (!context_ || context_ != qcu::ContextId::primary(device_)) {
       (void)s_.release();
       return false;
     }
