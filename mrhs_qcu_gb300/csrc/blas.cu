@@ -52,10 +52,11 @@ __device__ __forceinline__ void st(float2* p, double2 v) { *p = Store<PREC_SINGL
 // the conversion issues there too): the norm of 24^3x48 SU(3) nrhs 12 FP32
 // took 195 us against 56 us of HBM time (75 now).  So the products of a group are added in
 // FP32 with their rounding errors kept (Knuth's TwoSum): the sum goes to FP64, the
-// errors, gathered in FP32, with every fourth group (1.25 additions a group instead
-// of 2: <x, y> with |x|^2 at 16^3x32 SU(4) nrhs 16 89 -> 59 us, <x, y> 62 -> 48).
-// Against an exact sum of the same products the error is the plain FP64 sum's
-// (3.8e-17 of the sum of magnitudes for 864 products, 3.9e-17 plain).  A group that
+// errors, added in FP32 with theirs kept in turn, with every fourth group (1.25 additions a
+// group instead of 2: <x, y> with |x|^2 at 16^3x32 SU(4) nrhs 16 89 -> 59 us, <x, y> 62 -> 48),
+// and theirs at the end.  Against an exact sum of the same products the error is the plain FP64
+// sum's, also where the products span many binades (64 products over 8 decades: 0.7e-17 of the
+// sum of magnitudes, plain 1.5e-17; without the third level 49e-17).  A group that
 // leaves FP32's range, or is not finite, is added product by product (a call: as
 // predicated instructions it would hold the FP64 pipe).
 constexpr int kGroup = 4;
@@ -67,29 +68,37 @@ static __device__ __noinline__ double add_plainly(double acc, float a, float b, 
 }
 struct GroupSum {
   float p[kGroup];
-  float rest = 0.f;  // rounding errors of the groups since the last FP64 addition of them (every fourth)
+  float rest = 0.f;   // rounding errors of the groups since the last FP64 addition of them (every fourth)
+  float rest2 = 0.f;  // rounding errors of these
   int groups = 0;
   __device__ __forceinline__ void set(int u, float v) { p[u] = v; }  // u: a constant once the loops are unrolled
+  // a + b, and its rounding error
+  static __device__ __forceinline__ float two_sum(float a, float b, float& err) {
+    const float s = __fadd_rn(a, b), c = __fsub_rn(s, a);
+    err = __fadd_rn(__fsub_rn(a, __fsub_rn(s, c)), __fsub_rn(b, c));
+    return s;
+  }
   __device__ __forceinline__ void flush(double& acc) {
-    float hi = p[0], lo = 0.f;
+    float lo, e, lo2 = 0.f, hi = two_sum(p[0], p[1], lo);
 #pragma unroll
-    for (int u = 1; u < kGroup; u++) {
-      const float s = __fadd_rn(hi, p[u]), b = __fsub_rn(s, hi);
-      lo = __fadd_rn(lo, __fadd_rn(__fsub_rn(hi, __fsub_rn(s, b)), __fsub_rn(p[u], b)));
-      hi = s;
+    for (int u = 2; u < kGroup; u++) {
+      hi = two_sum(hi, p[u], e);
+      lo = two_sum(lo, e, e);
+      lo2 = __fadd_rn(lo2, e);
     }
     if (fabsf(hi) <= 3.402823466e38f) {
       acc += to_f64(hi);
-      rest += lo;
+      rest = two_sum(rest, lo, e);
+      rest2 = __fadd_rn(rest2, __fadd_rn(lo2, e));
     } else {
       acc = add_plainly(acc, p[0], p[1], p[2], p[3]);
     }
-    if ((++groups & 3) == 0) finish(acc);
+    if ((++groups & 3) == 0) {
+      acc += to_f64(rest);
+      rest = 0.f;
+    }
   }
-  __device__ __forceinline__ void finish(double& acc) {
-    acc += to_f64(rest);
-    rest = 0.f;
-  }
+  __device__ __forceinline__ void finish(double& acc) { acc += to_f64(rest) + to_f64(rest2); }
 };
 // FP64 products accumulate as they are formed
 __device__ __forceinline__ void add_square(double& acc, double2 v) {
