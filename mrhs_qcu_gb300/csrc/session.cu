@@ -65,12 +65,19 @@ bool Autotuner::enabled() const {
   return !(e && e[0] == '0');
 }
 
+// The set of kernels that a file's choices were timed among.  Raised when a kernel is added or dropped, or a
+// shape's numbers mean another one: 1 (files without the line) had no register-fragment MMAs (tensor-core
+// variant 5 was a tcgen05 ring), FP64 multiply-adds, and scalar FP32 from SU(4) on.
+constexpr int kKernelSet = 2;
+
 void Autotuner::load_file() {
   file_loaded_ = true;
   const char* path = getenv("QCU_TUNE_CACHE");
   if (!path) return;
   std::ifstream in(path);
   std::string line;
+  int set = 0;
+  if (!std::getline(in, line) || sscanf(line.c_str(), "kernels %d", &set) != 1 || set != kKernelSet) return;
   while (std::getline(in, line)) {
     std::istringstream ls(line);
     std::string k;
@@ -89,6 +96,7 @@ void Autotuner::save_file() {
   const char* path = getenv("QCU_TUNE_CACHE");
   if (!path) return;
   std::ofstream out(path);
+  out << "kernels " << kKernelSet << "\n";
   for (auto& kv : cache_)
     out << kv.first.prec << ":" << kv.first.N << ":" << kv.first.nrhs << ":" << kv.first.vh << " " << kv.second.R << " " << kv.second.block << " " << kv.second.minb << " " << kv.second.pk
         << " " << kv.second.tma << " " << kv.second.rcta << " " << kv.second.tc << " " << kv.second.rc << " "
