@@ -515,7 +515,15 @@ void Session::hop(FieldView out, FieldView in, FieldView x, int parity, int dagg
   // built by the first hop on the loaded links, whatever its shape: a captured hop of another shape finds them
   A.gauge12 = gauge12(in.prec);
   tensor_links(A, in.prec, tunes ? -1 : c.tc);
-  if (tunes) c = tuner.tune(A, in.prec, N, stream());
+  if (tunes) {
+    DslashArgs T = A;
+    DeviceBuffer field, norm;
+    if (T.x == T.out) {  // tuning applies the hop many times: not onto what the caller's x holds
+      T.out = field.ensure(field_bytes(in.prec, in.nrhs));
+      if (T.out_norm) T.out_norm = static_cast<float*>(norm.ensure(norm_bytes(in.prec, in.nrhs)));
+    }
+    c = tuner.tune(T, in.prec, N, stream());
+  }
   launch_dslash(A, in.prec, N, c, stream());
 }
 
