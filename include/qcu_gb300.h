@@ -214,7 +214,7 @@ int qcuDslashSegments(const QcuHopSegment *segments, int count, int nColors, int
  * or the file named by QCU_TUNE_CACHE), else the fastest shape, timed now and
  * cached.  Returns the chosen RHS-per-thread, block size, register-cap variant
  * (registers per thread: 1 no cap, 2 = 128, 3 = 85, 4 = 112, 5 = 96,
- * 6 = 104), whether the packed FP32x2 arithmetic variant was chosen, and the
+ * 6 = 104, 7 = 168), whether the packed FP32x2 arithmetic variant was chosen, and the
  * ring depth of the TMA-staged kernel (0: the register kernel was chosen;
  * -v: tensor-core variant v, see qcuDslashKernels), whether the kernel
  * reads two-row SU(3) links (recon = 1), and whether its links are staged by

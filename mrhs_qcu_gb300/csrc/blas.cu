@@ -775,7 +775,7 @@ int device_sms() {
 // Grid of a reducing kernel: one even wave.  1024 threads an SM always fit (at most 64 registers a thread,
 // 32 KB of shared memory), so every SM takes the same number of blocks at once.  1024 blocks of 128 threads
 // with 32 KB each made 1.12 waves of 6 blocks, and left the second half of the time to a tenth of the
-// blocks: at 16^3x32 SU(4) nrhs 16, us, before / now: BiCGStab update 274 / 158, <x, y> with |x|^2 119 / 89,
+// blocks: at 16^3x32 SU(4) nrhs 16, us, before / now: BiCGStab update 274 / 167, <x, y> with |x|^2 119 / 89,
 // <x, y> 84 / 62.
 int reduce_grid(int64_t nchunks, int block) {
   const int64_t g = (nchunks + block - 1) / block;

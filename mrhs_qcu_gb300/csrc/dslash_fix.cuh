@@ -21,9 +21,8 @@
 // One hop, us, FP64 multiply-adds / this: SU(3) 24^3x48 nrhs 12 5763 / 1747, SU(4) 16^3x32 nrhs 16
 // 2460 / 779, SU(3) 14x10x6x18 nrhs 5 62 / 27; in the split form SU(3) 12^3x24 nrhs 1 46 / 21, SU(6)
 // 16^3x32 nrhs 16 4978 / 2486, SU(8) 8378 / 4187, SU(6) 8^3x16 nrhs 1 99 / 19.  It is bound by
-// instruction issue and latency (SU(3): 8300 instructions a warp, 216 wide multiply-adds a hop; the
-// multiplier 53% busy, the integer pipe 43%, FP64 33%, 12 or 16 warps an SM); the small sizes by the
-// latency of one warp a scheduler.
+// instruction issue and latency (SU(3): 9500 instructions a warp, 216 wide multiply-adds a hop; issue 54%, the
+// integer pipe 51%, FP64 35% busy, 15 warps an SM); the small sizes by the latency of one warp a scheduler.
 //
 // A common exponent keeps the digits of a part only down to its unit.  So a site takes the FP64 multiply-adds
 // (fp64_site) when a part of its result is made up of small products only (fix_parts_hold), when its hops lie more
